@@ -24,6 +24,12 @@ PROTOTYPES = {
     "cagnet_spmm_csr_f32": (_i32, [_vp, _vp, _vp, _i32, _i32, _i64, _vp, _i64, _vp, _i64, _i32, _f32, _vp, _vp]),
     "cagnet_spmm_noalloc_max_nnz": (_i64, []),
     "cagnet_spmm_csr_f32_noalloc": (_i32, [_vp, _vp, _vp, _i32, _i32, _i64, _vp, _i64, _vp, _i64, _i32, _f32, _vp]),
+    "cagnet_tile_count_i32": (_i32, [_vp, _vp, _i32, _vp, _vp, _i32, _i32, _vp, _vp]),
+    "cagnet_tile_fill_i32": (_i32, [_vp, _vp, _vp, _i32, _vp, _vp, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "cagnet_tile_core_workspace_bytes": (_sz, [_i32, _i32, _i32]),
+    "cagnet_tile_core_f32": (_i32, [_vp, _vp, _vp, _vp, _i32, _i32, _vp, _i32, _vp, _i32, _vp, _vp, _vp, _vp, _i64, _vp,
+                                    _i64, _i32, _vp, _sz, _vp]),
+    "cagnet_tile_core_error": (_i32, []),
     "cagnet_core_gemm_workspace_bytes": (_sz, [_i32, _i32, _i32]),
     "cagnet_core_gemm_f32": (_i32, [_vp, _i64, _vp, _i32, _vp, _i32, _vp, _i64, _vp, _i64, _i32, _vp, _sz, _vp]),
     "cagnet_core_gemm_tc_available": (_i32, []),

@@ -37,5 +37,31 @@ int set_core_chunk(int value);
 int core_chunk_int();
 int set_core_chunk_int(int value);
 
+// Programmatic dependent launch: a kernel launched through launch_pdl may be scheduled while the kernel in front of it
+// in the stream is still running (its launch latency and prologue then cost nothing), and must call pdl_wait() before
+// it touches memory: that returns when everything in front is complete and visible.  pdl_trigger() lets the kernel
+// behind it be scheduled early in turn.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl_if(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                 A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  return launch_pdl_if(true, kernel, grid, block, smem, stream, args...);
+}
 
 }  // namespace cagnet

@@ -116,6 +116,34 @@ int cagnet_spmm_csr_f32_noalloc(const int32_t* rowptr, const int32_t* col, const
                                 const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f, float beta,
                                 void* stream);
 
+/* ---- Dense tiles of a normalised block as bit matrices (256 rows x 64 columns, rows and columns taken in order of degree:
+ * rank_r / rank_c give a row's / column's place, tiles are searched among the first lim_r x lim_c).
+ *   cagnet_tile_count_i32   counts[p * ceil(lim_c / 64) + q] += nonzeros of tile (p, q) (counts zeroed by the caller)
+ *   cagnet_tile_fill_i32    tile_of: number of each chosen tile, -1 for the others.  Sets the bits of the entries that lie in
+ *                           a chosen tile and equal row_scale[r] * col_scale[c] exactly (bits zeroed by the caller, 2,048
+ *                           bytes per tile) and keep[e] = 1 for all other entries (also for the second occurrence of an
+ *                           entry listed twice)
+ *   cagnet_tile_core_f32    C[panel_rows[256 p + i], 0:f) += panel_scale[256 p + i] * sum over the panel's tiles and their
+ *                           columns c with a bit set of col_scale[c] * B[c, 0:f).  tile_kb: per tile, sorted by panel, the
+ *                           64-column block of tile_cols (-1 = no column) it covers; panel_ptr[p]: first tile of panel p;
+ *                           cta_ptr[i]: first tile of thread block i's share (every share holds at least one tile);
+ *                           join_list: (panel, first block, last block + 1, 0) of each panel that several blocks share.
+ *                           Three bf16 terms per element of B, fp32 sums in a fixed order.
+ * cagnet_tile_core_error: 1 if a multiply on the current device gave up on a wait since the library was loaded
+ * (synchronises the device).  No counterpart in the reference. */
+int cagnet_tile_count_i32(const int32_t* rowptr, const int32_t* col, int32_t n, const int32_t* rank_r,
+                          const int32_t* rank_c, int32_t lim_r, int32_t lim_c, int32_t* counts, void* stream);
+int cagnet_tile_fill_i32(const int32_t* rowptr, const int32_t* col, const float* val, int32_t n, const int32_t* rank_r,
+                         const int32_t* rank_c, int32_t lim_r, int32_t lim_c, const int32_t* tile_of,
+                         const float* row_scale, const float* col_scale, void* bits, uint8_t* keep, void* stream);
+size_t cagnet_tile_core_workspace_bytes(int32_t kbs, int32_t ctas, int32_t f);
+int cagnet_tile_core_f32(const void* bits, const int32_t* tile_kb, const int32_t* panel_ptr, const int32_t* cta_ptr,
+                         int32_t ctas, int32_t panels, const void* join_list, int32_t joins, const int32_t* tile_cols,
+                         int32_t kbs, const int32_t* panel_rows, const float* panel_scale, const float* col_scale,
+                         const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f, void* ws, size_t ws_bytes,
+                         void* stream);
+int cagnet_tile_core_error(void);
+
 /* ---- Dense core of a sparse block: C[core_rows[i], 0:f) += sum_j core[i*ld_core + j] * B[core_cols[j], 0:f)
  * for i < R, j < K.  `core` is the R x K dense fp32 sub-block (zeros where the sparse block has no entry) of
  * the hub rows `core_rows` (distinct, ascending or not) and hub columns `core_cols` that the host layer cut out
