@@ -69,11 +69,7 @@ def dense_core_info(model):
     whether it is multiplied on the tensor cores), or None when the block is all-sparse."""
     try:
         blk = model.am_pbyp.groups[0].block if hasattr(model, "am_pbyp") else model.adj_block
-        if blk.core is None:
-            return None
-        rows, cols = blk.core_shape()
-        return {"rows": rows, "cols": cols, "nnz": int(blk.nnz - blk.rest.nnz), "kind": blk.core_kind(),
-                "tensor_cores": blk.core_kind() in ("bf16-integer", "3xtf32")}
+        return blk.dense_part()
     except (AttributeError, IndexError):      # an informational field must not cost the line
         return None
 
@@ -592,7 +588,8 @@ def run_algorithm(ctx, algo, args, workload, problem, data, f, classes, info, la
         flops = sum(2.0 * r[2] * r[3] for r in wide) / max(len(wide), 1)
         core_kernel = None
         if dense_core_info(model) is not None:
-            core_kernel = {"bf16-integer": "tcgen05 kind::f16 (bf16 multiplicities x 3 bf16 terms)",
+            core_kernel = {"bit-tiles": "tcgen05 kind::f16 (bit tiles x 3 bf16 terms, A operand in tensor memory)",
+                           "bf16-integer": "tcgen05 kind::f16 (bf16 multiplicities x 3 bf16 terms)",
                            "3xtf32": "tcgen05 kind::tf32 (3xTF32)", "fp32-fma": "sgemm"}[dense_core_info(model)["kind"]]
         line = {
             "metric": METRIC, "value": ms_per_step, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -604,8 +601,8 @@ def run_algorithm(ctx, algo, args, workload, problem, data, f, classes, info, la
             "spmm_ms_per_epoch": all_ms / args.steps,
             "spmm_ms_by_width": {str(k): sum(v) / args.steps for k, v in sorted(per_width.items())},
             "roofline": {"bound": "hbm",
-                         "kernel": "spmm f=%d on rank 0 (hub-row and warp-per-row / lane-group launches on the sparse part; "
-                                   "gather+split, tcgen05 multiplies in k chunks and row-add launches on a dense core)" % f_wide,
+                         "kernel": "spmm f=%d on rank 0 (nonzero-split and join launches on the sparse part; operand, tcgen05 "
+                                   "multiply and join launches on the dense tiles)" % f_wide,
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak if peak else None,
                          "peak_source": peak_kind, "launch_ms": launch_ms, "calls_per_epoch": calls,
                          "traffic": spmm_traffic_bytes() if (world == 1 and args.workload == "cfg2" and algo == "1d") else None,

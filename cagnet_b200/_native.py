@@ -24,6 +24,11 @@ PROTOTYPES = {
     "cagnet_spmm_csr_f32": (_i32, [_vp, _vp, _vp, _i32, _i32, _i64, _vp, _i64, _vp, _i64, _i32, _f32, _vp, _vp]),
     "cagnet_spmm_noalloc_max_nnz": (_i64, []),
     "cagnet_spmm_csr_f32_noalloc": (_i32, [_vp, _vp, _vp, _i32, _i32, _i64, _vp, _i64, _vp, _i64, _i32, _f32, _vp]),
+    "cagnet_spmm_split_plan_bytes": (_sz, [_i64]),
+    "cagnet_spmm_split_plan_i32": (_i32, [_vp, _vp, _vp, _vp, _i32, _i64, _vp, _sz, _vp]),
+    "cagnet_spmm_block_workspace_bytes": (_sz, [_vp, _vp, _i64, _i32]),
+    "cagnet_spmm_block_launches": (_i32, [_vp, _i32]),
+    "cagnet_spmm_block_f32": (_i32, [_vp, _vp, _i64, _vp, _i64, _i32, _f32, _vp, _sz, _vp]),
     "cagnet_tile_count_i32": (_i32, [_vp, _vp, _i32, _vp, _vp, _i32, _i32, _vp, _vp]),
     "cagnet_tile_fill_i32": (_i32, [_vp, _vp, _vp, _i32, _vp, _vp, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp]),
     "cagnet_tile_core_workspace_bytes": (_sz, [_i32, _i32, _i32]),
@@ -57,6 +62,18 @@ PROTOTYPES = {
     "cagnet_nll_masked_f32": (_i32, [_vp, _i64, _vp, _vp, _i64, _i32, _i32, _i32, _f32, _f32, _vp, _vp, _i64, _vp,
                                      _sz, _vp]),
 }
+
+
+
+class Block(ctypes.Structure):
+    """`cagnet_block` of include/cagnet_b200.h, field for field."""
+    _fields_ = ([("n", _i32), ("m", _i32), ("nnz", _i64), ("rowptr", _vp), ("col", _vp), ("val", _vp), ("plan", _vp),
+                 ("hub_rows", _i32), ("max_row", _i32), ("split", _vp), ("rows", _vp), ("empty", _vp), ("nrows", _i32),
+                 ("nempty", _i32), ("tiles", _i32), ("panels", _i32), ("ctas", _i32), ("joins", _i32), ("tile_kbs", _i32),
+                 ("reserved", _i32), ("tile_nnz", _i64), ("tile_work", _i64)] +
+                [(name, _vp) for name in ("tile_bits", "tile_kb", "panel_ptr", "cta_ptr", "join_list", "tile_cols",
+                                          "panel_rows", "panel_scale", "col_scale", "rest")])
+
 
 _lib = None
 

@@ -105,7 +105,7 @@ class CudaBackend:
         """A received block.  `reused`: the caller keeps it across epochs, so the one-off search for a dense core
         pays; a block that lives for one multiply only gets its hub-row list."""
         blk = ops.CsrBlock(buf[:n + 1], buf[n + 1:n + 1 + nnz], buf[n + 1 + nnz:].view(torch.float32), n, m)
-        blk.build_plan(core=bool(reused))
+        blk.build_plan(core=bool(reused), lasting=bool(reused))
         return blk
 
     # ---- row-wise pieces of a log-softmax split by columns over a process row

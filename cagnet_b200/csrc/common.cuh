@@ -64,4 +64,11 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_
   return launch_pdl_if(true, kernel, grid, block, smem, stream, args...);
 }
 
+// The row kernels of spmm.cu with what the host knows about the block: hub_rows = rows listed in the plan, -1 = unknown.
+int spmm_rows_f32(const int32_t* rowptr, const int32_t* col, const float* val, int32_t n, int32_t m, int64_t nnz,
+                  const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f, float beta, const void* plan,
+                  int32_t hub_rows, void* stream);
+int spmm_forced_tile();      // "spmm_tile" when a sweep has set it: such multiplies run the row kernels
+int split_launches(const cagnet_block* b, int32_t f);
+
 }  // namespace cagnet

@@ -6,11 +6,12 @@ and adds the cached-CSR form the GCN layers use.  PyTorch is the owner of device
 here; every multiply, activation and loss is a kernel of `libcagnet_b200.so` (torch index kernels are used
 once per block, when its dense core is looked for and cut out).  CPU tensors are rejected.
 """
+import ctypes
 import os
 
 import torch
 
-from . import _native, core_select
+from . import _native, core_select, tile_plan
 
 EPI_NONE, EPI_RELU, EPI_LOG_SOFTMAX, EPI_RELU_MASK, EPI_ACCUMULATE = 0, 1, 2, 3, 4
 _INT32_MAX = 2 ** 31 - 1
@@ -148,11 +149,16 @@ def _row_major(t):
 # as the bf16 matrix of edge multiplicities between the two diagonals and multiplies it with three bf16 products
 # (csrc/core_gemm_int.cu): a quarter of the memory and a third of the tensor time of the 3xTF32 form, so the bar
 # is "density_int", the side limit "max_side_int", and products down to "min_width_int" columns use it.
+# "tiles": such a block is cut into dense TILES instead (tile_plan.py, csrc/tile_core.cu: one bit per cell, a staircase of
+# 256 x 64 tiles of at least "density_int" among the "tile_side" highest-degree rows and columns), which take over more of
+# the nonzeros at a sixteenth of the memory and pay at every width; "tile_nnz": fewest nonzeros in tiles worth a plan;
+# "tile_work": a product uses the tiles from this many gathered floats on (nonzeros in tiles x width; 0 with "min_share" 0).
 CORE = {"enabled": os.environ.get("CAGNET_DENSE_CORE", "1") != "0", "density": 0.2, "density_tc": 0.09, "step": 1024,
         "max_side": 16384, "max_bytes": 2 << 30, "min_share": 0.1, "min_width": 128, "rounds": 1,
         "tensor_cores": os.environ.get("CAGNET_CORE_TENSOR", "1") != "0",
         "integer": os.environ.get("CAGNET_CORE_INTEGER", "1") != "0", "density_int": 0.02, "max_side_int": 32768,
-        "min_width_int": 128, "min_row_nnz": 64}
+        "min_width_int": 128, "min_row_nnz": 64, "tiles": os.environ.get("CAGNET_DENSE_TILES", "1") != "0",
+        "tile_side": 1 << 18, "tile_nnz": 100000, "tile_work": 80000000}
 
 
 def core_on_tensor_cores():
@@ -187,6 +193,9 @@ def coo2csr(rows, n):
     return rowptr
 
 
+_NO_RECT = (None, None, None, None)
+
+
 class CsrBlock:
     """A static n x m sparse block on the device: int32 CSR + fp32 values + the SpMM plan (list of hub rows).
 
@@ -196,10 +205,63 @@ class CsrBlock:
     def __init__(self, rowptr, col, val, n, m, plan=None):
         self.rowptr, self.col, self.val, self.n, self.m, self.plan = rowptr, col, val, int(n), int(m), plan
         self.nnz = int(val.numel())
-        self.core = self.rest = None      # dense hub-by-hub rectangle and the CSR block of everything else
-        self.core_split = None            # the rectangle as TF32 hi + lo parts (tensor-core multiply)
-        self.core_int = None              # (bf16 multiplicities, rows, cols, row factors, column factors)
         self.row_scale = self.col_scale = None    # the diagonals a normalised block was scaled with, if known
+        self.hub_rows = self.max_row = -1         # rows in the plan's list, longest row (-1: not known on the host)
+        self.split = self.rows = self.empty = None    # nonzero-split plan, rows with and without nonzeros
+        self.tiles = self.sparse = None           # dense tiles (tile_plan.TilePlan) and the CSR block of everything else
+        self._rect = _NO_RECT                     # the rectangle form of a dense core, see extract_core
+        self._rect_config = None                  # set: the rectangle has not been looked for yet
+        self._c = None
+        self._by_width = {}
+
+    # The rectangle form of a dense core.  A block that multiplies by dense tiles computes it on request only.
+    @property
+    def core(self):
+        """(dense hub-by-hub matrix or None, row list, column list), or None without a core."""
+        return self._rectangle()[0]
+
+    @property
+    def rest(self):
+        """CSR block of everything outside the rectangle."""
+        return self._rectangle()[1]
+
+    @property
+    def core_split(self):
+        """The rectangle as TF32 hi + lo parts (tensor-core multiply)."""
+        return self._rectangle()[2]
+
+    @property
+    def core_int(self):
+        """(bf16 multiplicities, rows, cols, row factors, column factors)."""
+        return self._rectangle()[3]
+
+    def _rectangle(self):
+        if self._rect_config is not None:
+            config, self._rect_config = self._rect_config, None
+            self._cut_rectangle(config)
+        return self._rect
+
+    def native(self):
+        """The block as the C ABI's `cagnet_block` (rebuilt when a part of it is replaced)."""
+        if self._c is None:
+            c = _native.Block(n=self.n, m=self.m, nnz=self.nnz, hub_rows=self.hub_rows, max_row=self.max_row,
+                              nrows=self.n if self.rows is None else self.rows.numel(),
+                              nempty=0 if self.empty is None else self.empty.numel())
+            for name in ("rowptr", "col", "val", "plan", "split", "rows", "empty"):
+                t = getattr(self, name)
+                setattr(c, name, None if t is None else t.data_ptr())
+            if self.tiles is not None:
+                t = self.tiles
+                for name in ("tiles", "panels", "ctas", "joins", "tile_kbs"):
+                    setattr(c, name, getattr(t, name))
+                for name in ("tile_bits", "tile_kb", "panel_ptr", "cta_ptr", "join_list", "tile_cols", "panel_rows",
+                             "panel_scale"):
+                    setattr(c, name, getattr(t, name).data_ptr())
+                c.col_scale = self.col_scale.data_ptr()
+                c.tile_nnz, c.tile_work = self.nnz - self.sparse.nnz, t.work
+                c.rest = ctypes.addressof(self.sparse.native())
+            self._c = c
+        return self._c
 
     @staticmethod
     def from_coo(rows, cols, vals, n, m, validate=True, plan=True, row_scale=None, col_scale=None):
@@ -237,17 +299,80 @@ class CsrBlock:
                       5: "row index out of range"}.get(code, "?")
             raise RuntimeError("cagnet_b200: malformed sparse block: " + reason)
 
-    def build_plan(self, core=True):
-        """Hub-row list for the SpMM kernels and, with `core`, the dense-core split for wide products."""
+    def build_plan(self, core=True, lasting=True):
+        """What the multiplies of this block need: the hub-row list; for a block that is kept (`lasting`), the
+        nonzero-split form; with `core`, its dense part -- tiles, or a rectangle where tiles do not apply.  A block that
+        lives for one multiply gets the hub-row list only and costs no synchronisation."""
         nbytes = _native.lib().cagnet_spmm_plan_bytes(self.n, self.nnz)
         self.plan = torch.empty((nbytes + 15) // 16 * 16, dtype=torch.uint8, device=self.val.device)
+        self._c, self._by_width = None, {}
         with _on(self.val.device):
             _native.check(_native.lib().cagnet_spmm_plan_i32(self.rowptr.data_ptr(), self.n, self.nnz,
                                                              self.plan.data_ptr(), self.plan.numel(), _stream()),
                           "spmm_plan")
         LAUNCHES[0] += 5      # header + four length-class passes
-        if core:
-            self.extract_core()
+        if not lasting or self.n == 0:
+            return
+        if core and CORE["enabled"]:
+            integer = self.row_scale is not None and integer_core_available()
+            if not (integer and CORE["tiles"] and self.cut_tiles()):
+                self.extract_core()
+            elif self.nnz >= CORE["min_row_nnz"] * self.n:
+                self._rect_config = dict(CORE)
+        if self.nnz == 0:
+            self.hub_rows = self.max_row = 0
+            return
+        lens = self.rowptr[1:] - self.rowptr[:-1]
+        stats = torch.stack([lens.max(), (lens > 0).sum().int(), self.plan[4:8].view(torch.int32)[0]])
+        self.max_row, filled, self.hub_rows = (int(v) for v in stats.tolist())
+        if filled < self.n:
+            self.rows, self.empty = torch.nonzero(lens).flatten().int(), torch.nonzero(lens == 0).flatten().int()
+        if self.tiles is not None and (self.nnz - self.sparse.nnz) * 4 >= self.tiles.work:
+            return                     # every width from 4 columns on goes through the tiles and the rest
+        nbytes = _native.lib().cagnet_spmm_split_plan_bytes(self.nnz)
+        self.split = torch.empty(nbytes, dtype=torch.uint8, device=self.val.device)
+        with _on(self.val.device):
+            _native.check(_native.lib().cagnet_spmm_split_plan_i32(
+                self.rowptr.data_ptr(), self.col.data_ptr(), self.val.data_ptr(),
+                None if self.rows is None else self.rows.data_ptr(), filled, self.nnz, self.split.data_ptr(), nbytes,
+                _stream()), "spmm_split_plan")
+        LAUNCHES[0] += 2
+
+    def cut_tiles(self):
+        """Dense tiles of a normalised block (tile_plan.py); False when it has too few of them to matter."""
+        if self.nnz < CORE["tile_nnz"]:
+            return False
+        L, dev, n, m = _native.lib(), self.val.device, self.n, self.m
+        order_r, rank_r = tile_plan.ranks(self.rowptr[1:] - self.rowptr[:-1])
+        order_c, rank_c = tile_plan.ranks(torch.bincount(self.col, minlength=m))
+        lim_r, lim_c = min(n, CORE["tile_side"]), min(m, CORE["tile_side"])
+        counts = torch.zeros(-(-lim_r // tile_plan.ROWS), -(-lim_c // tile_plan.COLS), dtype=torch.int32, device=dev)
+        with _on(dev):
+            _native.check(L.cagnet_tile_count_i32(self.rowptr.data_ptr(), self.col.data_ptr(), n, rank_r.data_ptr(),
+                                                  rank_c.data_ptr(), lim_r, lim_c, counts.data_ptr(), _stream()), "tile_count")
+        LAUNCHES[0] += 1
+        on = tile_plan.select(counts, max(1, int(CORE["density_int"] * tile_plan.ROWS * tile_plan.COLS)))
+        if int((counts * on).sum()) < CORE["tile_nnz"]:
+            return False
+        t = tile_plan.TilePlan(on, order_r, order_c, lim_r, lim_c, self.row_scale)
+        t.work = int(CORE["tile_work"]) if CORE["min_share"] > 0 else 0
+        keep = torch.empty(self.nnz, dtype=torch.uint8, device=dev)
+        with _on(dev):
+            _native.check(L.cagnet_tile_fill_i32(self.rowptr.data_ptr(), self.col.data_ptr(), self.val.data_ptr(), n,
+                                                 rank_r.data_ptr(), rank_c.data_ptr(), lim_r, lim_c, t.tile_of.data_ptr(),
+                                                 self.row_scale.data_ptr(), self.col_scale.data_ptr(), t.tile_bits.data_ptr(),
+                                                 keep.data_ptr(), _stream()), "tile_fill")
+        LAUNCHES[0] += 1
+        kept = torch.zeros(self.nnz + 1, dtype=torch.int32, device=dev)
+        torch.cumsum(keep, 0, dtype=torch.int32, out=kept[1:])
+        if self.nnz - int(kept[-1]) < CORE["tile_nnz"]:
+            return False               # values that do not factor (scales of another block, weighted edges)
+        keep = keep.bool()
+        self.sparse = CsrBlock(kept[self.rowptr.long()], self.col[keep], self.val[keep], n, m)
+        self.sparse.build_plan(core=False)
+        t.tile_of = None
+        self.tiles = t
+        return True
 
     def extract_core(self, depth=0):
         """Cut the dense core out of a power-law block.
@@ -263,7 +388,10 @@ class CsrBlock:
         (the region is L-shaped in a symmetric matrix: hub rows x many columns, then many rows x hub columns), up
         to CORE["rounds"] rectangles.  Runs once per block, with torch index kernels on the block's device; the
         choice depends only on the block (ties broken by index)."""
-        cfg = CORE
+        self._rect_config = None
+        self._cut_rectangle(CORE, depth)
+
+    def _cut_rectangle(self, cfg, depth=0):
         if not cfg["enabled"] or self.nnz < cfg["min_row_nnz"] * self.n:
             return
         integer = self.row_scale is not None and integer_core_available()
@@ -277,6 +405,7 @@ class CsrBlock:
             return
         dense, rest_rowptr, rest_col, rest_val = core_select.split_core(self.col, self.val, self.n, choice)
         core_rows, core_cols = choice.rows.int().contiguous(), choice.cols.int().contiguous()
+        core_int = core_split = None
         if integer:
             rs, cs = self.row_scale[choice.rows].contiguous(), self.col_scale[choice.cols].contiguous()
             cnt = core_select.integer_core(dense, rs, cs)
@@ -286,27 +415,37 @@ class CsrBlock:
                 del dense, rest_rowptr, rest_col, rest_val
                 saved, self.row_scale = self.row_scale, None
                 try:
-                    return self.extract_core(depth)
+                    return self._cut_rectangle(cfg, depth)
                 finally:
                     self.row_scale = saved
-            self.core_int = (cnt.to(torch.bfloat16), core_rows, core_cols, rs, cs)
+            core_int = (cnt.to(torch.bfloat16), core_rows, core_cols, rs, cs)
             del cnt
             dense = None
         rest = CsrBlock(rest_rowptr, rest_col, rest_val, self.n, self.m)
         rest.row_scale, rest.col_scale = self.row_scale, self.col_scale
         rest.build_plan(core=False)
         if depth + 1 < int(cfg["rounds"]):
-            rest.extract_core(depth + 1)
-        self.rest = rest
-        self.core = (dense, core_rows, core_cols)
-        self.core_split = None
+            rest._cut_rectangle(cfg, depth + 1)
         if dense is not None and core_on_tensor_cores() and dense.stride(0) % 4 == 0:
             hi, lo = torch.empty_like(dense), torch.empty_like(dense)
             with _on(dense.device):
                 _native.check(_native.lib().cagnet_split_tf32_f32(dense.data_ptr(), dense.numel(), hi.data_ptr(),
                                                                   lo.data_ptr(), _stream()), "split_tf32")
             LAUNCHES[0] += 1
-            self.core_split = (hi, lo)
+            core_split = (hi, lo)
+        self._rect = ((dense, core_rows, core_cols), rest, core_split, core_int)
+
+    def dense_part(self):
+        """How much of the block is multiplied densely, without computing anything: a dict, or None when all of it is
+        sparse."""
+        if self.tiles is not None:
+            return {"kind": "bit-tiles", "tiles": self.tiles.tiles, "rows": self.tiles.panels * tile_plan.ROWS,
+                    "cols": self.tiles.tile_kbs * tile_plan.COLS, "nnz": self.nnz - self.sparse.nnz, "tensor_cores": True}
+        if self._rect_config is not None or self._rect[0] is None:
+            return None
+        rows, cols = self.core_shape()
+        return {"kind": self.core_kind(), "rows": rows, "cols": cols, "nnz": self.nnz - self.rest.nnz,
+                "tensor_cores": self.core_kind() in ("bf16-integer", "3xtf32")}
 
     def core_shape(self):
         """(rows, columns) of the dense core, or None."""
@@ -342,18 +481,28 @@ def spmm(block, B, C, beta=1.0):
     if B.device != block.val.device or C.device != block.val.device:
         raise RuntimeError("cagnet_b200: spmm operands on different devices")
     f = B.size(1)
-    min_width = CORE["min_width_int"] if block.core_int is not None else CORE["min_width"]
-    use_core = block.core is not None and f >= min_width and ldb % 4 == 0 and B.data_ptr() % 16 == 0
     cores, src = [], block
-    while use_core and src.core is not None:
-        cores.append(src)
-        src = src.rest
+    if block.tiles is None and block._rect[0] is not None:
+        min_width = CORE["min_width_int"] if block.core_int is not None else CORE["min_width"]
+        use_core = f >= min_width and ldb % 4 == 0 and B.data_ptr() % 16 == 0
+        while use_core and src.core is not None:
+            cores.append(src)
+            src = src.rest
+    L = _native.lib()
+    b_ptr = B.data_ptr()
+    key = (f, ldb & 3, b_ptr & 15)
+    sized = src._by_width.get(key)
     with _on(C.device):
-        _native.check(_native.lib().cagnet_spmm_csr_f32(
-            src.rowptr.data_ptr(), src.col.data_ptr(), src.val.data_ptr(), src.n, src.m, src.nnz,
-            B.data_ptr(), ldb, C.data_ptr(), ldc, f, float(beta),
-            None if src.plan is None else src.plan.data_ptr(), _stream()), "spmm")
-        LAUNCHES[0] += 1 if src.plan is None else 2
+        c = src.native()
+        if sized is None:
+            sized = (L.cagnet_spmm_block_workspace_bytes(ctypes.addressof(c), b_ptr, ldb, f),
+                     L.cagnet_spmm_block_launches(ctypes.addressof(c), f))
+            src._by_width[key] = sized
+        nbytes, launches = sized
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=C.device) if nbytes else None
+        _native.check(L.cagnet_spmm_block_f32(ctypes.addressof(c), b_ptr, ldb, C.data_ptr(), ldc, f, float(beta),
+                                              None if ws is None else ws.data_ptr(), nbytes, _stream()), "spmm")
+        LAUNCHES[0] += launches
         for owner in cores:
             if owner.core_int is not None:
                 _core_multiply_int(owner.core_int, B, ldb, C, ldc, f)
@@ -436,7 +585,7 @@ def spmm_gpu(A_rowindices, A_colindices, A_values, n, m, B, C, validate=None):
     block = CsrBlock(coo2csr(rows32, n), A_colindices.contiguous(), A_values.float().contiguous(), n, m)
     if SPMM_GPU_VALIDATE if validate is None else validate:
         block.validate(rows32)
-    block.build_plan(core=False)      # a per-call block: the core split only pays when it is reused
+    block.build_plan(core=False, lasting=False)      # a per-call block: what is prepared once pays only when it is reused
     Bc = B if _row_major(B) else B.contiguous()
     if _row_major(C):
         spmm(block, Bc, C, 1.0)

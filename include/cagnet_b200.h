@@ -116,6 +116,58 @@ int cagnet_spmm_csr_f32_noalloc(const int32_t* rowptr, const int32_t* col, const
                                 const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f, float beta,
                                 void* stream);
 
+/* ---- A static sparse block with everything that is prepared once for its multiplies; plain device pointers, owned by
+ * the caller, any of the optional parts may be absent (NULL / 0).
+ *   rowptr, col, val   the n x m CSR block itself
+ *   plan, hub_rows     cagnet_spmm_plan_i32's list of long rows and their number (-1: not known to the host)
+ *   max_row            nonzeros of the longest row (-1: not known to the host)
+ *   split              cagnet_spmm_split_plan_i32's pairs; rows / nrows: the rows with nonzeros (NULL = every row),
+ *                      empty / nempty: the rows without
+ *   tiles ...          dense tiles (below) that hold tile_nnz of the nonzeros, used from tile_nnz * width >= tile_work on,
+ *                      and `rest`, the block of all others */
+typedef struct cagnet_block {
+  int32_t n, m;
+  int64_t nnz;
+  const int32_t* rowptr;
+  const int32_t* col;
+  const float* val;
+  const void* plan;
+  int32_t hub_rows, max_row;
+  const void* split;
+  const int32_t* rows;
+  const int32_t* empty;
+  int32_t nrows, nempty;
+  int32_t tiles, panels, ctas, joins, tile_kbs, reserved;
+  int64_t tile_nnz, tile_work;
+  const void* tile_bits;
+  const int32_t* tile_kb;
+  const int32_t* panel_ptr;
+  const int32_t* cta_ptr;
+  const void* join_list;
+  const int32_t* tile_cols;
+  const int32_t* panel_rows;
+  const float* panel_scale;
+  const float* col_scale;
+  const struct cagnet_block* rest;
+} cagnet_block;
+
+/* The nonzero-split form of a block: (column, value) pairs with the last nonzero of every row marked, and the row at
+ * every 32nd nonzero.  `rows` lists the nrows rows that have nonzeros (NULL when all have).  plan: 16-byte aligned,
+ * cagnet_spmm_split_plan_bytes(nnz).  No counterpart in the reference. */
+size_t cagnet_spmm_split_plan_bytes(int64_t nnz);
+int cagnet_spmm_split_plan_i32(const int32_t* rowptr, const int32_t* col, const float* val, const int32_t* rows,
+                               int32_t nrows, int64_t nnz, void* plan, size_t plan_bytes, void* stream);
+
+/* C = beta*C + A*B by whichever of the block's prepared forms is the fastest at this width: dense tiles on the tensor
+ * cores plus the rest, the nonzero split, or the row kernels of cagnet_spmm_csr_f32.  Same contract as
+ * cagnet_spmm_csr_f32 (beta 0 or 1, exactly n x f elements of C written, columns [f, ld) of B's padded rows may be read).
+ * ws: cagnet_spmm_block_workspace_bytes for the same B, ldb and f, 256-byte aligned; contents need not survive between
+ * calls, two calls that may overlap on the GPU need one each.  cagnet_spmm_block_launches: kernels one call launches. */
+size_t cagnet_spmm_block_workspace_bytes(const cagnet_block* block, const float* B, int64_t ldb, int32_t f);
+int cagnet_spmm_block_launches(const cagnet_block* block, int32_t f);
+int cagnet_spmm_block_f32(const cagnet_block* block, const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f,
+                          float beta, void* ws, size_t ws_bytes, void* stream);
+
 /* ---- Dense tiles of a normalised block as bit matrices (256 rows x 64 columns, rows and columns taken in order of degree:
  * rank_r / rank_c give a row's / column's place, tiles are searched among the first lim_r x lim_c).
  *   cagnet_tile_count_i32   counts[p * ceil(lim_c / 64) + q] += nonzeros of tile (p, q) (counts zeroed by the caller)

@@ -1,0 +1,77 @@
+"""The nonzero-split multiply and the dense bit tiles at the sizes where they can go wrong: chunk and tile edges, rows
+that cross many chunks, empty rows, ragged widths, unaligned operands, several thread blocks sharing a row panel."""
+import pytest
+import torch
+
+from cagnet_b200 import _native, graphs, ops, partition as PP
+
+pytestmark = pytest.mark.gpu
+REL = 1e-5
+
+
+def _close(got, want64):
+    want64 = want64.double()
+    err = float((got.double().cpu() - want64).abs().max())
+    assert err <= REL * max(float(want64.abs().max()), 1e-30), err
+
+
+def _dense64(b):
+    return torch.sparse_coo_tensor(torch.stack([b.rows, b.cols]), b.vals.double(), (b.n_rows, b.n_cols))
+
+
+@pytest.mark.parametrize("f", [1, 5, 16, 23, 41, 64, 65, 96, 100, 129, 300])
+@pytest.mark.parametrize("lens", [[200], [1] * 70, [0, 31, 1, 0, 64, 33, 0], [65, 5000, 0, 1, 32, 32, 4000, 7], [3, 97] * 40 + [0]])
+def test_split_multiply(f, lens):
+    g = torch.Generator().manual_seed(f)
+    n, m = len(lens), 6000
+    rows = torch.repeat_interleave(torch.arange(n), torch.tensor(lens))
+    cols = torch.cat([torch.sort(torch.randperm(m, generator=g)[:k])[0] for k in lens])
+    blk = PP.Block(rows, cols, torch.randn(rows.numel(), generator=g), n, m)
+    A = ops.CsrBlock.from_coo(blk.rows, blk.cols, blk.vals, n, m)
+    A.max_row = -1                                   # as if unknown: the split form whatever the rows look like
+    assert A.split is not None
+    B, C0 = torch.randn(m, f, generator=g), torch.randn(n, f, generator=g)
+    prod = torch.sparse.mm(_dense64(blk), B.double())
+    for padded in (True, False):
+        for beta in (0.0, 1.0):
+            Bd = ops.to_padded(B.cuda()) if padded else B.cuda()
+            Cd = ops.to_padded(C0.cuda()) if padded else C0.cuda().clone()
+            ops.spmm(A, Bd, Cd, beta)
+            _close(Cd, prod + beta * C0.double())
+    wide = torch.full((n, f + 3), 7.0, device="cuda")             # a slice of a wider matrix, rows not 16-byte aligned
+    ops.spmm(A, ops.to_padded(B.cuda()), wide[:, 1:f + 1], 0.0)
+    _close(wide[:, 1:f + 1], prod)
+    assert bool((wide[:, 0] == 7.0).all()) and bool((wide[:, f + 1:] == 7.0).all())
+
+
+@pytest.mark.parametrize("n,nnz,parts", [(700, 60000, 1), (4099, 600000, 1), (9001, 1500000, 3)])
+def test_bit_tiles(n, nnz, parts):
+    if not ops.integer_core_available():
+        pytest.skip("library built without the tensor-core kernels")
+    adj = graphs.add_self_loops(graphs.rmat_graph(n, target_nnz=nnz, seed=n), n)
+    adj = torch.cat([adj, adj[:, :500]], dim=1)                    # some edges twice: those entries stay sparse
+    blk = PP.fuse_columns(PP.oned_partition(0, parts, torch.zeros(n, 1), adj, True)[1])
+    old = ops.configure_core(min_share=0.0, tile_nnz=1000, density_int=0.02)
+    try:
+        A = ops.CsrBlock.from_coo(blk.rows, blk.cols, blk.vals, blk.n_rows, n, row_scale=blk.row_scale, col_scale=blk.col_scale)
+    finally:
+        ops.configure_core(**old)
+    assert A.tiles is not None
+    bits = A.tiles.tile_bits.cpu().numpy().view("uint8")
+    assert int(sum(bin(b).count("1") for b in bits.tolist())) + A.sparse.nnz == A.nnz
+    M = _dense64(blk)
+    for f in (1, 16, 17, 41, 64, 65, 128, 200, 602):
+        g = torch.Generator().manual_seed(f)
+        B, C0 = torch.randn(n, f, generator=g), torch.randn(blk.n_rows, f, generator=g)
+        want = torch.sparse.mm(M, B.double()) + C0.double()
+        Bd = ops.to_padded(B.cuda())
+        if Bd.stride(0) > f:
+            ops.base_buffer(Bd).view(-1, Bd.stride(0))[:, f:] = float("nan")
+        C1, C2, C3 = ops.to_padded(C0.cuda()), ops.to_padded(C0.cuda()), C0.cuda().clone()
+        ops.spmm(A, Bd, C1, 1.0)
+        ops.spmm(A, Bd, C2, 1.0)
+        ops.spmm(A, B.cuda(), C3, 1.0)                             # unaligned rows where f is not a multiple of 4
+        _close(C1, want)
+        _close(C3, want)
+        assert torch.equal(C1, C2)
+    assert _native.lib().cagnet_tile_core_error() == 0
