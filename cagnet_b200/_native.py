@@ -8,8 +8,8 @@ import os
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libcagnet_b200.so")
 
-_vp, _i32, _i64, _f32, _sz, _cp = (ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_float,
-                                   ctypes.c_size_t, ctypes.c_char_p)
+_vp, _i32, _i64, _f32, _f64, _sz, _cp = (ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_float,
+                                         ctypes.c_double, ctypes.c_size_t, ctypes.c_char_p)
 
 # name -> (restype, argtypes); mirrors include/cagnet_b200.h one to one
 PROTOTYPES = {
@@ -61,6 +61,10 @@ PROTOTYPES = {
     "cagnet_nll_workspace_bytes": (_sz, [_i64]),
     "cagnet_nll_masked_f32": (_i32, [_vp, _i64, _vp, _vp, _i64, _i32, _i32, _i32, _f32, _f32, _vp, _vp, _i64, _vp,
                                      _sz, _vp]),
+    "cagnet_nll_softmax_bwd_f32": (_i32, [_vp, _i64, _vp, _vp, _i64, _i32, _i32, _i32, _f32, _vp, _i64,
+                                          ctypes.POINTER(_i32), _vp, _sz, _vp]),
+    "cagnet_adam2_f32": (_i32, [_vp, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _i64, _f64, _f64, _f64, _f64, _i64, _vp,
+                                _i32, _f32, _vp, _vp]),
 }
 
 
@@ -92,6 +96,23 @@ def lib():
             fn.restype, fn.argtypes = res, args
         _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (csrc/host.cpp), a Python extension beside the library."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError("cagnet_b200: native host module is missing or does not load (%s); build it with "
+                               "`python -m cagnet_b200.build`" % e) from e
+        _host = module
+    return _host
 
 
 def check(status, what=""):

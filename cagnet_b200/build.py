@@ -1,7 +1,7 @@
 """Build the native library in-tree: `python -m cagnet_b200.build`.
 
 Compiles every `csrc/*.cu` for sm_100a with nvcc (cross-compiles without a GPU) and links
-`cagnet_b200/libcagnet_b200.so`.  The ptxas resource report (registers, spills, shared memory per
+`cagnet_b200/libcagnet_b200.so`; `csrc/host.cpp` becomes the extension module `_host`.  The ptxas resource report (registers, spills, shared memory per
 kernel) is written next to the objects as `build/ptxas.log`.
 """
 import concurrent.futures
@@ -9,6 +9,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -56,6 +57,32 @@ def _stale(target, deps):
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def host_path():
+    return os.path.join(HERE, "_host" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def build_host(force=False):
+    """csrc/host.cpp, the native host path: a Python extension against this interpreter's PyTorch."""
+    src, out = os.path.join(CSRC, "host.cpp"), host_path()
+    header = os.path.join(os.path.dirname(HERE), "include", "cagnet_b200.h")
+    if not force and not _stale(out, [src, header]):
+        return out
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    includes = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_host",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), src, "-o", out]
+    for d in includes:
+        cmd += ["-isystem", d]
+    cmd += ["-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", LIB_PATH, "-Wl,-rpath,$ORIGIN"]
+    p = subprocess.run(cmd, capture_output=True, text=True)
+    if p.returncode != 0:
+        raise RuntimeError("g++ failed for host.cpp:\n%s\n%s" % (p.stdout, p.stderr))
+    return out
+
+
 def build(force=False, verbose=False):
     """Compile and link; returns the library path.  Re-uses objects that are newer than their sources."""
     nvcc = _nvcc()
@@ -91,10 +118,11 @@ def build(force=False, verbose=False):
         with open(os.path.join(BUILD_DIR, "ptxas.log"), "a") as fh:
             fh.write("".join(logs))
     if force or _stale(LIB_PATH, objs):
-        cmd = [nvcc, "-shared", "-o", LIB_PATH] + objs + ["-gencode", "arch=compute_100a,code=sm_100a", "-lcudart"]
+        cmd = [nvcc, "-shared", "-Xlinker", "-soname=libcagnet_b200.so", "-o", LIB_PATH] + objs + ["-gencode", "arch=compute_100a,code=sm_100a", "-lcudart"]
         p = subprocess.run(cmd, capture_output=True, text=True)
         if p.returncode != 0:
             raise RuntimeError("link failed:\n%s\n%s" % (p.stdout, p.stderr))
+    build_host(force)
     if verbose:
         print("built", LIB_PATH)
     return LIB_PATH

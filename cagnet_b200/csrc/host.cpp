@@ -1,0 +1,242 @@
+// Native host path: the calls of one multiply and of one single-process training epoch, queued from C++.
+//
+// An epoch of a small graph is a dozen kernels of 2 - 10 us; queued one by one from Python, through autograd and the
+// optimizer's own kernels, it took 750 us of host time (2.7 K vertices: 0.77 ms for 0.17 ms of kernels).  Here the same
+// sequence is one call: buffers from PyTorch's caching allocator, kernels of libcagnet_b200.so on the current stream.
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <algorithm>
+
+#include "../../include/cagnet_b200.h"
+
+namespace py = pybind11;
+
+namespace {
+
+void check(int status, const char* what) {
+  if (status != CAGNET_OK)
+    throw std::runtime_error(std::string("cagnet_b200 ") + what + " failed with status " + std::to_string(status) + ": " +
+                             cagnet_last_error_string());
+}
+
+[[noreturn]] void refuse(const std::string& text) { throw std::runtime_error("cagnet_b200: " + text); }
+
+std::string shape_text(const at::Tensor& t) {
+  std::string s = "(";
+  for (int64_t i = 0; i < t.dim(); ++i) s += (i ? ", " : "") + std::to_string(t.size(i));
+  return s + ")";
+}
+
+// Leading dimension of a row-major fp32 matrix on the device.
+int64_t ld_of(const at::Tensor& t, const char* name) {
+  if (!t.is_cuda()) refuse(std::string(name) + " must be a CUDA tensor (there is no CPU path)");
+  if (t.scalar_type() != at::kFloat || t.dim() != 2) refuse(std::string(name) + " must be a 2-D float32 tensor");
+  const int64_t rows = t.size(0), cols = t.size(1);
+  if (cols > 1 && t.stride(1) != 1) refuse(std::string(name) + " must be row-major (unit column stride)");
+  if (rows > 1) {
+    if (t.stride(0) < cols) refuse(std::string(name) + " has overlapping rows");
+    return t.stride(0);
+  }
+  return std::max<int64_t>(cols, 1);
+}
+
+int64_t pad_ld(int64_t f) { return f <= 64 ? (f + 3) / 4 * 4 : (f + 31) / 32 * 32; }
+
+// Scratch memory and matrices of an epoch: raw storage, rows padded as ops.empty_padded pads them.
+struct Buffer {
+  at::Tensor t;
+  int64_t ld = 0;
+  Buffer() = default;
+  Buffer(const at::TensorOptions& o, int64_t n, int64_t f) : t(at::empty({std::max<int64_t>(n, 1), pad_ld(f)}, o)), ld(pad_ld(f)) {}
+  float* p() const { return t.data_ptr<float>(); }
+};
+
+at::Tensor bytes_buffer(const at::TensorOptions& o, size_t bytes) {
+  return at::empty({static_cast<int64_t>((std::max<size_t>(bytes, 16) + 3) / 4)}, o);
+}
+
+int64_t multiply(const cagnet_block* b, const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f, float beta,
+                 const at::TensorOptions& o, void* stream) {
+  const size_t bytes = cagnet_spmm_block_workspace_bytes(b, B, ldb, f);
+  at::Tensor ws;
+  if (bytes) ws = bytes_buffer(o, bytes);
+  check(cagnet_spmm_block_f32(b, B, ldb, C, ldc, f, beta, bytes ? ws.data_ptr() : nullptr, bytes, stream), "spmm");
+  return cagnet_spmm_block_launches(b, f);
+}
+
+int64_t spmm(uintptr_t block, int64_t device, const at::Tensor& B, const at::Tensor& C, double beta) {
+  const auto* b = reinterpret_cast<const cagnet_block*>(block);
+  const int64_t ldb = ld_of(B, "B"), ldc = ld_of(C, "C");
+  if (B.size(0) != b->m || C.size(0) != b->n || B.size(1) != C.size(1))
+    refuse("spmm shape mismatch: A " + std::to_string(b->n) + "x" + std::to_string(b->m) + ", B " + shape_text(B) + ", C " + shape_text(C));
+  if (B.get_device() != device || C.get_device() != device) refuse("spmm operands on different devices");
+  if (B.size(1) > INT32_MAX) refuse("spmm is too wide");
+  c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+  return multiply(b, B.data_ptr<float>(), ldb, C.data_ptr<float>(), ldc, static_cast<int32_t>(B.size(1)), static_cast<float>(beta),
+                  C.options(), c10::cuda::getCurrentCUDAStream().stream());
+}
+
+struct Adam {
+  at::Tensor m1, v1, m2, v2;
+  double lr, beta1, beta2, eps;
+  int64_t step;
+};
+
+// One epoch of the two-layer model on one process: out = act2((A h) W2), h = act1((A x) W1) -- or A (h W), where
+// `min_width` and the layer's widths ask for it --, masked NLL, gradients of both weights (dist1d.GCNFunc,
+// dist1d.MaskedNLL), and Adam when its state is given.  `hook(begin, layer_block, width)` brackets every sparse product.
+py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Tensor& w1, const at::Tensor& w2,
+                const at::Tensor& y, const at::Tensor& mask, int64_t count, int64_t cls_lo, int64_t cls_hi, bool activations,
+                bool min_width, std::optional<Adam> adam, py::object hook) {
+  const auto* A = reinterpret_cast<const cagnet_block*>(fwd);
+  const auto* At = reinterpret_cast<const cagnet_block*>(bwd);
+  const int64_t ldx = ld_of(x, "x"), n = A->n;
+  ld_of(w1, "weight1");
+  ld_of(w2, "weight2");
+  const int32_t f = static_cast<int32_t>(w1.size(0)), h = static_cast<int32_t>(w1.size(1)), c = static_cast<int32_t>(w2.size(1));
+  if (x.size(1) != f || w2.size(0) != h || x.size(0) != n || A->m != n || At->n != n || At->m != n || !w1.is_contiguous() ||
+      !w2.is_contiguous())
+    refuse("epoch: shapes of the operands do not fit");
+  if (y.scalar_type() != at::kLong || !y.is_cuda() || !y.is_contiguous() || y.numel() != n || !mask.is_cuda() || mask.numel() != n ||
+      !mask.is_contiguous() || (mask.scalar_type() != at::kBool && mask.scalar_type() != at::kByte))
+    refuse("epoch: int64 labels and a bool mask on the device are needed");
+  c10::cuda::CUDAGuard guard(x.device());
+  void* s = c10::cuda::getCurrentCUDAStream().stream();
+  const auto o = x.options().requires_grad(false);
+  int64_t launches = 0;
+  auto product = [&](const cagnet_block* b, const float* B, int64_t ldb, const Buffer& C, int32_t width) {
+    if (!hook.is_none()) hook(true, b == At && b != A, width);
+    launches += multiply(b, B, ldb, C.p(), C.ld, width, 0.f, o, s);
+    if (!hook.is_none()) hook(false, b == At && b != A, width);
+  };
+  auto gemm = [&](const float* X, int64_t ld, const at::Tensor& W, bool transposed, const Buffer& Z, int32_t K, int32_t N, int epi,
+                  const float* aux, int64_t ldaux) {
+    check(cagnet_gemm_nn_f32(X, ld, W.data_ptr<float>(), W.size(1), transposed, Z.p(), Z.ld, n, K, N, epi, aux, ldaux, s), "gemm_nn");
+    ++launches;
+  };
+  // out = act(Z W) with the activation fused where the product's epilogue has it
+  auto dense_layer = [&](const float* X, int64_t ld, const at::Tensor& W, const Buffer& Z, int32_t K, int32_t N, bool last) {
+    if (!activations) return gemm(X, ld, W, false, Z, K, N, CAGNET_EPI_NONE, nullptr, 0);
+    if (!last) return gemm(X, ld, W, false, Z, K, N, CAGNET_EPI_RELU, nullptr, 0);
+    if (N <= 64) return gemm(X, ld, W, false, Z, K, N, CAGNET_EPI_LOG_SOFTMAX, nullptr, 0);
+    gemm(X, ld, W, false, Z, K, N, CAGNET_EPI_NONE, nullptr, 0);
+    check(cagnet_log_softmax_fwd_f32(Z.p(), Z.ld, Z.p(), Z.ld, n, N, s), "log_softmax");
+    ++launches;
+  };
+  auto tn = [&](const float* H, int64_t ldh, const Buffer& G, int32_t K, int32_t N) {
+    at::Tensor out = at::empty({K, N}, o);
+    const size_t bytes = cagnet_gemm_tn_workspace_bytes(n, K, N);
+    at::Tensor ws = bytes_buffer(o, bytes);
+    check(cagnet_gemm_tn_f32(H, ldh, G.p(), G.ld, out.data_ptr<float>(), N, n, K, N, 0.f, ws.data_ptr(), ws.numel() * 4, s), "gemm_tn");
+    launches += 2;
+    return out;
+  };
+  const float* X = x.data_ptr<float>();
+  const bool narrow1 = min_width && h < f, widen1 = min_width && h > f, narrow2 = min_width && c < h, widen2 = min_width && c > h;
+
+  // ---- forward
+  Buffer H(o, n, h), agg1, agg2;
+  if (narrow1) {
+    Buffer hw(o, n, h);
+    gemm(X, ldx, w1, false, hw, f, h, CAGNET_EPI_NONE, nullptr, 0);
+    product(A, hw.p(), hw.ld, H, h);
+    if (activations) {
+      check(cagnet_relu_fwd_f32(H.p(), H.ld, H.p(), H.ld, n, h, s), "relu");
+      ++launches;
+    }
+  } else {
+    Buffer z(o, n, f);
+    product(A, X, ldx, z, f);
+    dense_layer(z.p(), z.ld, w1, H, f, h, false);
+    if (widen1) agg1 = z;
+  }
+  Buffer out(o, n, c);
+  if (narrow2) {
+    Buffer hw(o, n, c);
+    gemm(H.p(), H.ld, w2, false, hw, h, c, CAGNET_EPI_NONE, nullptr, 0);
+    product(A, hw.p(), hw.ld, out, c);
+    if (activations) {
+      check(cagnet_log_softmax_fwd_f32(out.p(), out.ld, out.p(), out.ld, n, c, s), "log_softmax");
+      ++launches;
+    }
+  } else {
+    Buffer z(o, n, h);
+    product(A, H.p(), H.ld, z, h);
+    dense_layer(z.p(), z.ld, w2, out, h, c, true);
+    if (widen2) agg2 = z;
+  }
+
+  // ---- loss, and its gradient before the second activation
+  at::Tensor loss = at::empty({}, o), loss_ws = bytes_buffer(o, cagnet_nll_workspace_bytes(n));
+  Buffer dz(o, n, c);
+  int32_t parts = 0;
+  const auto* mask8 = static_cast<const uint8_t*>(mask.data_ptr());
+  if (activations) {
+    check(cagnet_nll_softmax_bwd_f32(out.p(), out.ld, y.data_ptr<int64_t>(), mask8, n, c, static_cast<int32_t>(cls_lo),
+                                     static_cast<int32_t>(cls_hi), static_cast<float>(count), dz.p(), dz.ld, &parts,
+                                     loss_ws.data_ptr(), loss_ws.numel() * 4, s), "nll_softmax_bwd");
+    ++launches;
+  } else {
+    check(cagnet_nll_masked_f32(out.p(), out.ld, y.data_ptr<int64_t>(), mask8, n, c, static_cast<int32_t>(cls_lo),
+                                static_cast<int32_t>(cls_hi), static_cast<float>(count), 1.f, loss.data_ptr<float>(), dz.p(), dz.ld,
+                                loss_ws.data_ptr(), loss_ws.numel() * 4, s), "nll_masked");
+    launches += 2;
+  }
+
+  // ---- backward: second layer
+  Buffer dh(o, n, h);         // gradient before the first activation
+  at::Tensor g1, g2;
+  const int mask_epi = activations ? CAGNET_EPI_RELU_MASK : CAGNET_EPI_NONE;
+  if (widen2) {
+    Buffer dzw(o, n, h);
+    gemm(dz.p(), dz.ld, w2, true, dzw, c, h, CAGNET_EPI_NONE, nullptr, 0);
+    product(At, dzw.p(), dzw.ld, dh, h);
+    if (activations) {
+      check(cagnet_relu_bwd_f32(H.p(), H.ld, dh.p(), dh.ld, dh.p(), dh.ld, n, h, s), "relu_bwd");
+      ++launches;
+    }
+    g2 = tn(agg2.p(), agg2.ld, dz, h, c);
+  } else {
+    Buffer ag(o, n, c);
+    product(At, dz.p(), dz.ld, ag, c);
+    gemm(ag.p(), ag.ld, w2, true, dh, c, h, mask_epi, H.p(), H.ld);
+    g2 = tn(H.p(), H.ld, ag, h, c);
+  }
+  // ---- backward: first layer
+  if (widen1) {
+    g1 = tn(agg1.p(), agg1.ld, dh, f, h);
+  } else {
+    Buffer ag(o, n, h);
+    product(At, dh.p(), dh.ld, ag, h);
+    g1 = tn(X, ldx, ag, f, h);
+  }
+  if (adam || activations) {
+    float* loss_p = activations ? loss.data_ptr<float>() : nullptr;
+    const auto* parts_p = loss_ws.data_ptr<float>();
+    if (adam) {
+      check(cagnet_adam2_f32(w1.data_ptr<float>(), adam->m1.data_ptr<float>(), adam->v1.data_ptr<float>(), g1.data_ptr<float>(), w1.numel(),
+                             w2.data_ptr<float>(), adam->m2.data_ptr<float>(), adam->v2.data_ptr<float>(), g2.data_ptr<float>(), w2.numel(),
+                             adam->lr, adam->beta1, adam->beta2, adam->eps, adam->step, parts_p, parts, static_cast<float>(count), loss_p, s),
+            "adam");
+    } else {
+      check(cagnet_adam2_f32(nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0, 0, 1, parts_p, parts,
+                             static_cast<float>(count), loss_p, s), "loss");
+    }
+    ++launches;
+  }
+  return py::make_tuple(out.t.narrow(1, 0, c).narrow(0, 0, n), loss, g1, g2, launches);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_host, m) {
+  m.def("spmm", &spmm);
+  py::class_<Adam>(m, "Adam").def(py::init([](at::Tensor m1, at::Tensor v1, at::Tensor m2, at::Tensor v2, double lr, double beta1,
+                                              double beta2, double eps, int64_t step) {
+    return Adam{m1, v1, m2, v2, lr, beta1, beta2, eps, step};
+  }));
+  m.def("epoch", &epoch);
+}

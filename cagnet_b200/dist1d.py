@@ -16,7 +16,7 @@ import torch
 import torch.distributed as dist
 import torch.nn.functional as F
 
-from . import partition
+from . import local_epoch, partition
 from .backend import ACT_LOG_SOFTMAX, ACT_NONE, ACT_RELU
 
 
@@ -456,6 +456,7 @@ class Model:
         self.rank_train_mask = data.train_mask[lo:hi].bool().to(dev)
         self.datay_rank = data.y[lo:hi].long().to(dev)
         self.train_count = int(self.rank_train_mask.sum())
+        self._local = None         # local_epoch.plan, or False where it does not apply
 
     def init_weights(self, mid_layer, capturable=False):
         """torch.manual_seed(0); rand on the CPU, then moved (gcn_distr.py:550-560).  `capturable` keeps Adam's
@@ -481,7 +482,22 @@ class Model:
         if getattr(self, "_graph", None) is not None:
             self._graph.replay()
             return self._graph_outputs
-        return self._train_eager().detach()
+        out = self._train_local()
+        return self._train_eager().detach() if out is None else out
+
+    def _train_local(self):
+        """The epoch as one native call, where it is a single process's plain epoch (local_epoch.py); None elsewhere."""
+        if self.size > 1 or self.rt.timers.enabled:
+            return None
+        if self._local is None:
+            plan = self.am_pbyp
+            back = getattr(plan, "backward_plan", None) or plan
+            self._local = len(plan.groups) == 1 and len(back.groups) == 1 and local_epoch.plan(
+                self.rt.backend, plan.groups[0].block, back.groups[0].block, 0, self.classes, self.rt.activations,
+                self.rt.order == "min_width") or False
+        if not self._local:
+            return None
+        return local_epoch.train(self._local, self, self.inputs_loc, self.datay_rank, self.rank_train_mask, self.train_count)
 
     def capture(self):
         """Record one whole epoch (both layers, loss, backward, collectives, Adam) into a CUDA graph; `train()`

@@ -21,7 +21,7 @@ import torch
 import torch.distributed as dist
 import torch.nn.functional as F
 
-from . import partition
+from . import local_epoch, partition
 from .backend import ACT_LOG_SOFTMAX, ACT_NONE, ACT_RELU
 from .dist1d import Data, act_name  # noqa: F401  (Data re-exported for callers of this module)
 from .timing import CATEGORIES_2D, Timers, all_gather_bytes, all_reduce_bytes
@@ -370,6 +370,7 @@ class Model:
                                                   degree_group=everyone, transposed=True)
             self.adj_t = AdjOperator(be, block_t, rank, q * q, g.group if g.comm else None, self.inputs_loc.device)
         self._setup_labels(data, n, classes)
+        self._local = None         # local_epoch.plan, or False where it does not apply
 
     def _setup_labels(self, data, n, classes):
         """Labels and mask as the reference's loss sees them (gcn_distr_2d.py:942-970): the slice
@@ -414,9 +415,30 @@ class Model:
         return train(self)
 
 
+def train_local(model):
+    """The epoch of a 1 x 1 (x 1) grid as one native call (local_epoch.py); None where it does not apply.  The word counters
+    go on as the schedules keep them."""
+    rt, be = model.rt, model.rt.backend
+    if model.grid.comm or model.grid.q != 1 or rt.timers.enabled:
+        return None
+    if model._local is None:
+        back = model.adj_t.adj_block if model.adj_t is not None else model.adj_block
+        model._local = local_epoch.plan(be, model.adj_block, back, model.cls_lo, model.cls_hi, rt.activations, False) or False
+    if not model._local or model.local_train_rows <= 0:
+        return None
+    outputs = local_epoch.train(model._local, model, model.inputs_loc, model.y_eff, model.mask_eff, model.train_count_global)
+    if outputs is not None:
+        h, c = model.weight2.shape
+        rt.timers.count("summa_sparse_bcast2_words", model.node_count * (model.features + h + c + h))
+    return outputs
+
+
 def train(model):
     """gcn_distr_2d.py:920-1001."""
     rt = model.rt
+    outputs = train_local(model)
+    if outputs is not None:
+        return outputs
     outputs = GCNFunc.apply(model.inputs_loc, model.weight1, model, F.relu)
     outputs = GCNFunc.apply(outputs, model.weight2, model, F.log_softmax)
     model.optimizer.zero_grad()

@@ -20,7 +20,7 @@ import torch.nn.functional as F
 from . import partition
 from .backend import ACT_LOG_SOFTMAX, ACT_NONE, ACT_RELU
 from .dist1d import Data, act_name  # noqa: F401
-from .dist2d import AdjOperator, MaskedNLL, _bcast, _offsets
+from .dist2d import AdjOperator, MaskedNLL, _bcast, _offsets, train_local
 from .timing import CATEGORIES_3D, Timers, all_gather_bytes, all_reduce_bytes
 
 
@@ -346,6 +346,7 @@ class Model:
                                                    degree_group=g.group if g.comm else None, transposed=True)
             self.adj_t = AdjOperator(be, slab_t, rank, size, g.group if g.comm else None, self.inputs_loc.device)
         self._setup_labels(data, n, classes)
+        self._local = None         # local_epoch.plan, or False where it does not apply
 
     def _setup_labels(self, data, n, classes):
         """gcn_distr_3d.py:1080-1108: slice split(., L)[i*c + k] with L this process's row count, compressed to
@@ -389,6 +390,9 @@ class Model:
 def train(model):
     """gcn_distr_3d.py:1054-1141."""
     rt = model.rt
+    outputs = train_local(model)
+    if outputs is not None:
+        return outputs
     outputs = GCNFunc.apply(model.inputs_loc, model.weight1, model, F.relu)
     outputs = GCNFunc.apply(outputs, model.weight2, model, F.log_softmax)
     model.optimizer.zero_grad()

@@ -212,7 +212,6 @@ class CsrBlock:
         self._rect = _NO_RECT                     # the rectangle form of a dense core, see extract_core
         self._rect_config = None                  # set: the rectangle has not been looked for yet
         self._c = None
-        self._by_width = {}
 
     # The rectangle form of a dense core.  A block that multiplies by dense tiles computes it on request only.
     @property
@@ -263,6 +262,10 @@ class CsrBlock:
             self._c = c
         return self._c
 
+    def address(self):
+        """Address of `native()`, valid while the block lives and is not planned again."""
+        return ctypes.addressof(self.native())
+
     @staticmethod
     def from_coo(rows, cols, vals, n, m, validate=True, plan=True, row_scale=None, col_scale=None):
         """rows/cols: integer tensors sorted by row (a coalesced COO), vals fp32; any device (moved to CUDA).
@@ -305,7 +308,7 @@ class CsrBlock:
         lives for one multiply gets the hub-row list only and costs no synchronisation."""
         nbytes = _native.lib().cagnet_spmm_plan_bytes(self.n, self.nnz)
         self.plan = torch.empty((nbytes + 15) // 16 * 16, dtype=torch.uint8, device=self.val.device)
-        self._c, self._by_width = None, {}
+        self._c = None
         with _on(self.val.device):
             _native.check(_native.lib().cagnet_spmm_plan_i32(self.rowptr.data_ptr(), self.n, self.nnz,
                                                              self.plan.data_ptr(), self.plan.numel(), _stream()),
@@ -474,35 +477,19 @@ class CsrBlock:
 
 def spmm(block, B, C, beta=1.0):
     """C = beta * C + block @ B in place (beta 0 or 1)."""
+    if block.tiles is not None or block._rect[0] is None:
+        LAUNCHES[0] += _native.host().spmm(block.address(), block.val.get_device(), B, C, beta)
+        return C
+    # a block with a rectangular dense core: what is left of it, then the core on top
     ldb, ldc = _ld(B, "B"), _ld(C, "C")
-    if B.size(0) != block.m or C.size(0) != block.n or B.size(1) != C.size(1):
-        raise RuntimeError("cagnet_b200: spmm shape mismatch: A %dx%d, B %s, C %s"
-                           % (block.n, block.m, tuple(B.shape), tuple(C.shape)))
-    if B.device != block.val.device or C.device != block.val.device:
-        raise RuntimeError("cagnet_b200: spmm operands on different devices")
     f = B.size(1)
+    min_width = CORE["min_width_int"] if block.core_int is not None else CORE["min_width"]
     cores, src = [], block
-    if block.tiles is None and block._rect[0] is not None:
-        min_width = CORE["min_width_int"] if block.core_int is not None else CORE["min_width"]
-        use_core = f >= min_width and ldb % 4 == 0 and B.data_ptr() % 16 == 0
-        while use_core and src.core is not None:
-            cores.append(src)
-            src = src.rest
-    L = _native.lib()
-    b_ptr = B.data_ptr()
-    key = (f, ldb & 3, b_ptr & 15)
-    sized = src._by_width.get(key)
+    while f >= min_width and ldb % 4 == 0 and B.data_ptr() % 16 == 0 and src.core is not None:
+        cores.append(src)
+        src = src.rest
+    LAUNCHES[0] += _native.host().spmm(src.address(), src.val.get_device(), B, C, beta)
     with _on(C.device):
-        c = src.native()
-        if sized is None:
-            sized = (L.cagnet_spmm_block_workspace_bytes(ctypes.addressof(c), b_ptr, ldb, f),
-                     L.cagnet_spmm_block_launches(ctypes.addressof(c), f))
-            src._by_width[key] = sized
-        nbytes, launches = sized
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=C.device) if nbytes else None
-        _native.check(L.cagnet_spmm_block_f32(ctypes.addressof(c), b_ptr, ldb, C.data_ptr(), ldc, f, float(beta),
-                                              None if ws is None else ws.data_ptr(), nbytes, _stream()), "spmm")
-        LAUNCHES[0] += launches
         for owner in cores:
             if owner.core_int is not None:
                 _core_multiply_int(owner.core_int, B, ldb, C, ldc, f)

@@ -314,6 +314,22 @@ int cagnet_nll_masked_f32(const float* logp, int64_t ldl, const int64_t* y, cons
                           int64_t n, int32_t N, int32_t cls_lo, int32_t cls_hi, float count, float scale,
                           float* loss_dev, float* grad, int64_t ldg, void* ws, size_t ws_bytes, void* stream);
 
+/* ---- The loss of a log-softmax model and its gradient before the log-softmax in one pass:
+ * dz[i, j] = (exp(logp[i, j]) - [j == y_i - cls_lo]) / count for rows with mask[i] and a label in [cls_lo, cls_hi), 0 for
+ * the others: log_softmax_bwd of nll_masked's gradient.  Leaves *parts (host) partial sums of logp[i, y_i] in ws
+ * (cagnet_nll_workspace_bytes), which cagnet_adam2_f32 turns into the loss.  F.nll_loss and the autograd calls at
+ * gcn_distr.py:356 and :312-322. */
+int cagnet_nll_softmax_bwd_f32(const float* logp, int64_t ldl, const int64_t* y, const uint8_t* mask, int64_t n, int32_t N,
+                               int32_t cls_lo, int32_t cls_hi, float count, float* dz, int64_t lddz, int32_t* parts,
+                               void* ws, size_t ws_bytes, void* stream);
+
+/* ---- One Adam step (torch.optim.Adam with default options; `step` counts from 1) on two parameter tensors of n1 and n2
+ * elements in one launch.  With loss != NULL also *loss = -sum(loss_parts[0 .. parts)) / count.  optimizer.step() at
+ * gcn_distr.py:364. */
+int cagnet_adam2_f32(float* p1, float* m1, float* v1, const float* g1, int64_t n1, float* p2, float* m2, float* v2,
+                     const float* g2, int64_t n2, double lr, double beta1, double beta2, double eps, int64_t step,
+                     const float* loss_parts, int32_t parts, float count, float* loss, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

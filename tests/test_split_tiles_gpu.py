@@ -75,3 +75,41 @@ def test_bit_tiles(n, nnz, parts):
         _close(C3, want)
         assert torch.equal(C1, C2)
     assert _native.lib().cagnet_tile_core_error() == 0
+
+
+@pytest.mark.parametrize("n,N,lo,hi", [(1, 1, 0, 1), (33, 7, 0, 7), (300, 41, 0, 41), (257, 256, 0, 256), (500, 20, 20, 40)])
+def test_fused_loss_and_adam(n, N, lo, hi):
+    """Loss, gradient before the log-softmax and one Adam step against fp64 autograd and torch.optim.Adam."""
+    import ctypes
+    L, g = _native.lib(), torch.Generator().manual_seed(n)
+    z = torch.randn(n, N, generator=g)
+    y = torch.randint(0, 2 * N, (n,), generator=g)
+    mask = torch.rand(n, generator=g) < 0.7
+    mask[0] = True
+    y[0] = lo
+    hit = mask & (y >= lo) & (y < hi)
+    z64 = z.double().requires_grad_(True)
+    want = -torch.log_softmax(z64, dim=1)[hit, (y - lo)[hit]].sum() / n
+    want.backward()
+    logp, dz = ops.log_softmax(ops.to_padded(z.cuda())), ops.empty_padded(n, N, "cuda")
+    ws = torch.empty(L.cagnet_nll_workspace_bytes(n), dtype=torch.uint8, device="cuda")
+    parts = ctypes.c_int32()
+    yd, md = y.cuda(), mask.cuda().view(torch.uint8)
+    _native.check(L.cagnet_nll_softmax_bwd_f32(logp.data_ptr(), logp.stride(0), yd.data_ptr(), md.data_ptr(), n, N, lo, hi, float(n),
+                                               dz.data_ptr(), dz.stride(0), ctypes.byref(parts), ws.data_ptr(), ws.numel(), None))
+    _close(dz, z64.grad)
+    w = [torch.randn(k, generator=g).cuda() for k in (n * 3, N)]
+    ref = [torch.nn.Parameter(t.clone()) for t in w]
+    opt = torch.optim.Adam(ref, lr=0.01)
+    state = [[torch.zeros_like(t), torch.zeros_like(t)] for t in w]
+    loss = torch.empty((), device="cuda")
+    for step in (1, 2, 3):
+        grads = [torch.randn(t.numel(), generator=g).cuda() for t in w]
+        for p, d in zip(ref, grads):
+            p.grad = d
+        opt.step()
+        ptr = [x for t, s, d in zip(w, state, grads) for x in (t.data_ptr(), s[0].data_ptr(), s[1].data_ptr(), d.data_ptr(), t.numel())]
+        _native.check(L.cagnet_adam2_f32(*ptr, 0.01, 0.9, 0.999, 1e-8, step, ws.data_ptr(), parts.value, float(n), loss.data_ptr(), None))
+    for t, p in zip(w, ref):
+        _close(t, p.detach().cpu())
+    assert abs(float(loss) - float(want)) <= 1e-5 * max(abs(float(want)), 1e-6)
