@@ -29,6 +29,9 @@ PROTOTYPES = {
     "cagnet_spmm_block_workspace_bytes": (_sz, [_vp, _vp, _i64, _i32]),
     "cagnet_spmm_block_launches": (_i32, [_vp, _i32]),
     "cagnet_spmm_block_f32": (_i32, [_vp, _vp, _i64, _vp, _i64, _i32, _f32, _vp, _sz, _vp]),
+    "cagnet_check_coo_i32": (_i32, [_vp, _vp, _i32, _i32, _i64, _vp, _vp]),
+    "cagnet_spmm_coo_workspace_bytes": (_sz, [_i32, _i64, _vp, _i64, _i32]),
+    "cagnet_spmm_coo_f32": (_i32, [_vp, _vp, _vp, _i32, _i32, _i64, _vp, _i64, _vp, _i64, _i32, _vp, _vp, _sz, _vp]),
     "cagnet_tile_count_i32": (_i32, [_vp, _vp, _i32, _vp, _vp, _i32, _i32, _vp, _vp]),
     "cagnet_tile_fill_i32": (_i32, [_vp, _vp, _vp, _i32, _vp, _vp, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp]),
     "cagnet_tile_core_workspace_bytes": (_sz, [_i32, _i32, _i32]),
@@ -107,6 +110,7 @@ def host():
     if _host is None:
         lib()
         try:
+            import torch  # noqa: F401  (its libraries are what the extension links against)
             from . import _host as module
         except ImportError as e:
             raise RuntimeError("cagnet_b200: native host module is missing or does not load (%s); build it with "

@@ -76,7 +76,7 @@ def build_host(force=False):
            "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), src, "-o", out]
     for d in includes:
         cmd += ["-isystem", d]
-    cmd += ["-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", LIB_PATH, "-Wl,-rpath,$ORIGIN"]
+    cmd += ["-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-L" + os.path.join(cuda, "lib64"), "-lcudart", "-ltorch_cpu", "-ltorch_python", LIB_PATH, "-Wl,-rpath,$ORIGIN"]
     p = subprocess.run(cmd, capture_output=True, text=True)
     if p.returncode != 0:
         raise RuntimeError("g++ failed for host.cpp:\n%s\n%s" % (p.stdout, p.stderr))

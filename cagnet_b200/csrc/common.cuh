@@ -37,6 +37,10 @@ int set_core_chunk(int value);
 int core_chunk_int();
 int set_core_chunk_int(int value);
 
+__device__ __forceinline__ void red_add4(float* p, float4 v) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
 // Programmatic dependent launch: a kernel launched through launch_pdl may be scheduled while the kernel in front of it
 // in the stream is still running (its launch latency and prologue then cost nothing), and must call pdl_wait() before
 // it touches memory: that returns when everything in front is complete and visible.  pdl_trigger() lets the kernel
@@ -70,5 +74,6 @@ int spmm_rows_f32(const int32_t* rowptr, const int32_t* col, const float* val, i
                   int32_t hub_rows, void* stream);
 int spmm_forced_tile();      // "spmm_tile" when a sweep has set it: such multiplies run the row kernels
 int split_launches(const cagnet_block* b, int32_t f);
+
 
 }  // namespace cagnet

@@ -6,9 +6,11 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <algorithm>
+#include <array>
 
 #include "../../include/cagnet_b200.h"
 
@@ -77,6 +79,61 @@ int64_t spmm(uintptr_t block, int64_t device, const at::Tensor& B, const at::Ten
   c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
   return multiply(b, B.data_ptr<float>(), ldb, C.data_ptr<float>(), ldc, static_cast<int32_t>(B.size(1)), static_cast<float>(beta),
                   C.options(), c10::cuda::getCurrentCUDAStream().stream());
+}
+
+// C += A.B with A as COO: the verdict of the index check is read back while the (guarded) product is already queued.
+int64_t spmm_coo(const at::Tensor& rows, const at::Tensor& cols, const at::Tensor& vals, int64_t n, int64_t m, const at::Tensor& B,
+                 const at::Tensor& C, bool validate) {
+  const int64_t ldb = ld_of(B, "B"), ldc = ld_of(C, "C"), nnz = vals.numel();
+  for (const at::Tensor* t : {&rows, &cols, &vals}) {
+    if (!t->is_cuda() || !t->is_contiguous() || t->dim() != 1 || t->numel() != nnz || t->scalar_type() != (t == &vals ? at::kFloat : at::kInt))
+      refuse("spmm_gpu needs 1-D contiguous int32 indices and float32 values of one length on the device");
+    if (t->get_device() != C.get_device()) refuse("spmm operands on different devices");
+  }
+  if (B.size(0) != m || C.size(0) != n || B.size(1) != C.size(1))
+    refuse("spmm shape mismatch: A " + std::to_string(n) + "x" + std::to_string(m) + ", B " + shape_text(B) + ", C " + shape_text(C));
+  if (B.get_device() != C.get_device()) refuse("spmm operands on different devices");
+  const int32_t f = static_cast<int32_t>(B.size(1));
+  c10::cuda::CUDAGuard guard(C.device());
+  cudaStream_t s = c10::cuda::getCurrentCUDAStream().stream();
+  const auto o = C.options().requires_grad(false);
+  // what a call waits on: one pinned word and one event per host thread and device
+  struct Verdict {
+    int32_t* word = nullptr;
+    cudaEvent_t done = nullptr;
+  };
+  static thread_local std::array<Verdict, 64> verdicts;
+  Verdict& v = verdicts[static_cast<size_t>(C.get_device()) % verdicts.size()];
+  at::Tensor status;
+  if (validate) {
+    if (!v.word) {
+      if (cudaHostAlloc(reinterpret_cast<void**>(&v.word), sizeof(int32_t), cudaHostAllocDefault) != cudaSuccess ||
+          cudaEventCreateWithFlags(&v.done, cudaEventDisableTiming) != cudaSuccess)
+        refuse("spmm_gpu: cannot allocate a pinned word");
+    }
+    status = at::empty({1}, o.dtype(at::kInt));
+    check(cagnet_check_coo_i32(rows.data_ptr<int>(), cols.data_ptr<int>(), static_cast<int32_t>(n), static_cast<int32_t>(m), nnz,
+                               status.data_ptr<int>(), s), "check_coo");
+    if (cudaMemcpyAsync(v.word, status.data_ptr<int>(), sizeof(int32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaEventRecord(v.done, s) != cudaSuccess)
+      refuse(std::string("spmm_gpu: ") + cudaGetErrorString(cudaGetLastError()));
+  }
+  const size_t bytes = cagnet_spmm_coo_workspace_bytes(static_cast<int32_t>(m), nnz, B.data_ptr<float>(), ldb, f);
+  at::Tensor ws = bytes_buffer(o, bytes);
+  check(cagnet_spmm_coo_f32(rows.data_ptr<int>(), cols.data_ptr<int>(), vals.data_ptr<float>(), static_cast<int32_t>(n),
+                            static_cast<int32_t>(m), nnz, B.data_ptr<float>(), ldb, C.data_ptr<float>(), ldc, f,
+                            validate ? status.data_ptr<int>() : nullptr, ws.data_ptr(), ws.numel() * 4, s), "spmm_gpu");
+  if (validate) {
+    cudaError_t e;
+    {
+      py::gil_scoped_release release;
+      e = cudaEventSynchronize(v.done);
+    }
+    if (e != cudaSuccess) refuse(std::string("spmm_gpu: ") + cudaGetErrorString(e));
+    static const char* const reasons[] = {"row indices not sorted", "column index out of range", "row index out of range"};
+    if (*v.word) refuse(std::string("malformed sparse block: ") + (*v.word >= 3 && *v.word <= 5 ? reasons[*v.word - 3] : "?"));
+  }
+  return 2 + (validate ? 1 : 0);
 }
 
 struct Adam {
@@ -234,6 +291,7 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
 
 PYBIND11_MODULE(_host, m) {
   m.def("spmm", &spmm);
+  m.def("spmm_coo", &spmm_coo);
   py::class_<Adam>(m, "Adam").def(py::init([](at::Tensor m1, at::Tensor v1, at::Tensor m2, at::Tensor v2, double lr, double beta1,
                                               double beta2, double eps, int64_t step) {
     return Adam{m1, v1, m2, v2, lr, beta1, beta2, eps, step};

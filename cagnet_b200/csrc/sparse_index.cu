@@ -52,6 +52,42 @@ __global__ void check_csr_kernel(const int* __restrict__ rowptr, const int* __re
   }
 }
 
+// The indices of a row-sorted COO list: 16 bytes of each array per thread and step where they are aligned (8 M entries: 20 us
+// for one entry per thread, 11 us so).
+__global__ void __launch_bounds__(256) check_coo_kernel(const int* __restrict__ rows, const int* __restrict__ cols, int n, int m,
+                                                        int64_t nnz, int vec4, int* status) {
+  pdl_trigger();
+  pdl_wait();
+  int code = 0;
+  const int64_t steps = (nnz + 3) / 4;
+  for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < steps;
+       t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t e = t * 4;
+    const int live = static_cast<int>(nnz - e < 4 ? nnz - e : 4);
+    int r[4], c[4];
+    if (vec4 && live == 4) {
+      const int4 a = __ldg(reinterpret_cast<const int4*>(rows + e)), b = __ldg(reinterpret_cast<const int4*>(cols + e));
+      r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
+      c[0] = b.x; c[1] = b.y; c[2] = b.z; c[3] = b.w;
+    } else {
+      for (int j = 0; j < live; ++j) {
+        r[j] = __ldg(rows + e + j);
+        c[j] = __ldg(cols + e + j);
+      }
+    }
+    int before = e > 0 ? __ldg(rows + e - 1) : INT_MIN;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (j >= live) break;
+      if (c[j] < 0 || c[j] >= m) code = max(code, 4);
+      if (r[j] < 0 || r[j] >= n) code = max(code, 5);
+      else if (before > r[j]) code = max(code, 3);
+      before = r[j];
+    }
+  }
+  if (code) atomicMax(status, code);
+}
+
 }  // namespace cagnet
 
 using namespace cagnet;
@@ -84,4 +120,18 @@ extern "C" int cagnet_check_csr_i32(const int32_t* rowptr, const int32_t* col, c
   check_csr_kernel<<<static_cast<unsigned>((work + 255) / 256), 256, 0, s>>>(rowptr, col, rows, n, m,
                                                                             static_cast<int>(nnz), status_dev);
   return check_launch("cagnet_check_csr_i32");
+}
+
+extern "C" int cagnet_check_coo_i32(const int32_t* rows, const int32_t* cols, int32_t n, int32_t m, int64_t nnz,
+                                    int32_t* status_dev, void* stream) {
+  if (n < 0 || m < 0 || nnz < 0 || !status_dev || (nnz > 0 && (!rows || !cols)))
+    return fail(CAGNET_E_ARG, "cagnet_check_coo_i32: bad argument");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaMemsetAsync(status_dev, 0, sizeof(int), s);
+  if (nnz == 0) return check_launch("cagnet_check_coo_i32");
+  const int64_t blocks = ((nnz + 3) / 4 + 255) / 256;
+  const int vec4 = aligned(rows, 16) && aligned(cols, 16) ? 1 : 0;
+  check_coo_kernel<<<static_cast<unsigned>(blocks < 16 * kNumSMs ? blocks : 16 * kNumSMs), 256, 0, s>>>(rows, cols, n, m, nnz, vec4,
+                                                                                                       status_dev);
+  return check_launch("cagnet_check_coo_i32");
 }

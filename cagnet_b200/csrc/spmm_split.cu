@@ -35,11 +35,17 @@ struct SplitArgs {
   float* part;             // [feature tiles][chunks][ending piece | beginning piece][tile columns]
   int64_t nnz, ldb, ldc;
   int nrows, nempty, f_eff, f, chunk, nchunks, c_vec4;
+  // a block given as row-sorted COO for one multiply (spmm_gpu), nothing prepared: instead of pairs, first, rows and empty
+  const int *coo_rows, *coo_cols;
+  const float* coo_vals;
+  const int* status;       // nonzero: the indices are malformed, nothing may be done; nullptr = not checked
 };
 
 __device__ __forceinline__ float4 ld4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 
-// C[row, this lane's columns] = acc (+ the old value); columns >= f are never written.
+// C[row, this lane's columns] = acc, or += acc: every element gets exactly one addition per multiply, so it is left to the
+// memory system (the order cannot matter) instead of a load that the whole warp waits for at every row's end.  Columns >= f
+// are never written.
 template <int LPN, int NV>
 __device__ __forceinline__ void split_store(const SplitArgs& a, int row, int column0, int nvalid, bool add,
                                             const float (&acc)[NV][4]) {
@@ -50,16 +56,17 @@ __device__ __forceinline__ void split_store(const SplitArgs& a, int row, int col
       float* p = cp + k * (LPN * 4);
       const int live = a.f - (column0 + k * (LPN * 4));
       if (live >= 4 && a.c_vec4) {
-        float4 v = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
-        if (add) {
-          const float4 o = *reinterpret_cast<const float4*>(p);
-          v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-        }
-        *reinterpret_cast<float4*>(p) = v;
+        const float4 v = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+        if (add) red_add4(p, v);
+        else *reinterpret_cast<float4*>(p) = v;
       } else {
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (j < live) p[j] = add ? p[j] + acc[k][j] : acc[k][j];
+        for (int j = 0; j < 4; ++j) {
+          if (j < live) {
+            if (add) atomicAdd(p + j, acc[k][j]);
+            else p[j] = acc[k][j];
+          }
+        }
       }
     }
   }
@@ -72,7 +79,22 @@ __device__ __forceinline__ void piece_store(float* p, const float (&acc)[NV][4])
     *reinterpret_cast<float4*>(p + w * (LPN * 4)) = make_float4(acc[w][0], acc[w][1], acc[w][2], acc[w][3]);
 }
 
-template <int LPN, int NV, int BATCH, bool ADD>
+// Row a chunk starts in, and whether it began in an earlier chunk: from the plan, or from the COO rows themselves.
+template <bool COO>
+__device__ __forceinline__ unsigned chunk_row(const SplitArgs& a, int c, bool& mid) {
+  const int64_t at = static_cast<int64_t>(c) * a.chunk;
+  if constexpr (COO) {
+    const int r = __ldg(a.coo_rows + at);
+    mid = at > 0 && __ldg(a.coo_rows + at - 1) == r;
+    return static_cast<unsigned>(r);
+  } else {
+    const unsigned fw = __ldg(a.first + at / kUnit);
+    mid = (fw & kMid) != 0;
+    return fw & ~kMid;
+  }
+}
+
+template <int LPN, int NV, int BATCH, bool ADD, bool COO>
 __global__ void __launch_bounds__(kSplitWarps * 32) spmm_split_kernel(SplitArgs a) {
   constexpr int G = 32 / LPN;
   constexpr int PL = (2 * LPN >= BATCH) ? 1 : BATCH / (2 * LPN);   // 16-byte loads (2 pairs) per lane and stage
@@ -80,8 +102,10 @@ __global__ void __launch_bounds__(kSplitWarps * 32) spmm_split_kernel(SplitArgs 
   constexpr int TILE = LPN * 4 * NV;
   static_assert(SL <= kUnit && SL % BATCH == 0, "a stage lies inside a unit");
   __shared__ __align__(16) int2 stage_s[kSplitWarps][G][SL];
+  __shared__ __align__(8) int stage_rows_s[COO ? kSplitWarps : 1][COO ? G : 1][COO ? SL : 1];
   pdl_trigger();
   pdl_wait();
+  if (COO && a.status && *a.status) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane / LPN, l = lane % LPN;
   const int chunk_id = (blockIdx.x * kSplitWarps + warp) * G + sub;
@@ -90,11 +114,11 @@ __global__ void __launch_bounds__(kSplitWarps * 32) spmm_split_kernel(SplitArgs 
   const int nvalid = column0 >= a.f_eff ? 0 : min(NV, (a.f_eff - column0 + LPN * 4 - 1) / (LPN * 4));
   const int64_t start = static_cast<int64_t>(chunk_id) * a.chunk;
   const int len = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(a.chunk), a.nnz - start)));
-  const int2* src = a.pairs + start;
+  const int2* src = COO ? nullptr : a.pairs + start;
   int2* stage = stage_s[warp][sub];
-  const unsigned fw = len > 0 ? __ldg(a.first + start / kUnit) : 0u;
-  int k = static_cast<int>(fw & ~kMid);         // position in `rows` of the row being summed
-  bool head = (fw & kMid) != 0;                 // it began in an earlier chunk
+  int* stage_rows = COO ? stage_rows_s[warp][sub] : nullptr;
+  bool head = false;                            // the row being summed began in an earlier chunk
+  int k = len > 0 ? static_cast<int>(chunk_row<COO>(a, chunk_id, head)) : 0;       // its position in `rows`
   const float* bt = a.B + column0;
   float* piece = a.part + (static_cast<int64_t>(blockIdx.y) * a.nchunks + chunk_id) * (2 * TILE) + l * 4;
 
@@ -105,10 +129,28 @@ __global__ void __launch_bounds__(kSplitWarps * 32) spmm_split_kernel(SplitArgs 
     for (int j = 0; j < 4; ++j) acc[v][j] = 0.f;
   bool open = false;      // acc holds terms of a row whose last nonzero has not been met
 
+  int2 nxt_rows[PL];
   auto load_pairs = [&](int at, int4 (&q)[PL]) {
 #pragma unroll
     for (int i = 0; i < PL; ++i) {
       const int e = at + (i * LPN + l) * 2;
+      if constexpr (COO) {
+        q[i] = make_int4(INT_MAX, 0, INT_MAX, 0);
+        if (e < len) {
+          const int64_t g = start + e;
+          const int r0 = __ldg(a.coo_rows + g), r1 = g + 1 < a.nnz ? __ldg(a.coo_rows + g + 1) : -1;
+          q[i].x = __ldg(a.coo_cols + g) | (r0 != r1 ? INT_MIN : 0);
+          q[i].y = __float_as_int(__ldg(a.coo_vals + g));
+          nxt_rows[i].x = r0;
+          if (e + 1 < len) {
+            const int r2 = g + 2 < a.nnz ? __ldg(a.coo_rows + g + 2) : -1;
+            q[i].z = __ldg(a.coo_cols + g + 1) | (r1 != r2 ? INT_MIN : 0);
+            q[i].w = __float_as_int(__ldg(a.coo_vals + g + 1));
+            nxt_rows[i].y = r1;
+          }
+        }
+        continue;
+      }
       // the array is padded to whole units: a 16-byte load that starts inside the chunk stays inside the array
       q[i] = e < len ? __ldg(reinterpret_cast<const int4*>(src + e)) : make_int4(INT_MAX, 0, INT_MAX, 0);
     }
@@ -119,7 +161,10 @@ __global__ void __launch_bounds__(kSplitWarps * 32) spmm_split_kernel(SplitArgs 
   for (int s = 0; s < steps; ++s) {
     __syncwarp();
 #pragma unroll
-    for (int i = 0; i < PL; ++i) *reinterpret_cast<int4*>(stage + (i * LPN + l) * 2) = nxt[i];
+    for (int i = 0; i < PL; ++i) {
+      *reinterpret_cast<int4*>(stage + (i * LPN + l) * 2) = nxt[i];
+      if constexpr (COO) *reinterpret_cast<int2*>(stage_rows + (i * LPN + l) * 2) = nxt_rows[i];
+    }
     __syncwarp();
     load_pairs((s + 1) * SL, nxt);
 #pragma unroll
@@ -155,7 +200,7 @@ __global__ void __launch_bounds__(kSplitWarps * 32) spmm_split_kernel(SplitArgs 
             piece_store<LPN, NV>(piece, acc);
             head = false;
           } else {
-            split_store<LPN, NV>(a, a.rows ? __ldg(a.rows + k) : k, column0, nvalid, ADD, acc);
+            split_store<LPN, NV>(a, COO ? stage_rows[b + i] : (a.rows ? __ldg(a.rows + k) : k), column0, nvalid, ADD, acc);
           }
           ++k;
 #pragma unroll
@@ -173,7 +218,7 @@ __global__ void __launch_bounds__(kSplitWarps * 32) spmm_split_kernel(SplitArgs 
 // One warp per chunk in which a row ends that began in an earlier one: the row's pieces added up in chunk order
 // (lane group g takes every G-th, the groups are folded by a fixed shuffle tree).  Blocks beyond the chunks clear the
 // rows without nonzeros when C is overwritten.
-template <int LPN, int NV, bool ADD>
+template <int LPN, int NV, bool ADD, bool COO>
 __global__ void __launch_bounds__(128) spmm_split_join_kernel(SplitArgs a, int join_blocks) {
   constexpr int G = 32 / LPN;
   constexpr int TILE = LPN * 4 * NV;
@@ -194,28 +239,30 @@ __global__ void __launch_bounds__(128) spmm_split_join_kernel(SplitArgs a, int j
     return;
   }
   const int e = blockIdx.x * 4 + (threadIdx.x >> 5);
-  const int upc = a.chunk / kUnit;
-  auto start_of = [&](int c) { return __ldg(a.first + static_cast<int64_t>(c) * upc); };
   unsigned row_k = 0;
   int lo = e;                                    // chunks lo .. e start in row row_k
   bool mine = false;
-  if (e < a.nchunks) {
-    // the row bookkeeping is constant: it may be read before the pieces are there
-    const unsigned fw = start_of(e);
-    row_k = fw & ~kMid;
-    const unsigned next = e + 1 < a.nchunks ? start_of(e + 1) & ~kMid : static_cast<unsigned>(a.nrows);
-    mine = (fw & kMid) && next != row_k;         // next == row_k: the row runs through this chunk
+  if (COO) pdl_wait();                           // the rows may be those of the kernel in front, the status is
+  if (e < a.nchunks && !(COO && a.status && *a.status)) {
+    // the plan is constant: it may be read before the pieces are there
+    bool mid, other;
+    row_k = chunk_row<COO>(a, e, mid);
+    const unsigned next = e + 1 < a.nchunks ? chunk_row<COO>(a, e + 1, other) : static_cast<unsigned>(a.nrows);
+    mine = mid && next != row_k;                 // next == row_k: the row runs through this chunk
     while (mine) {                               // first chunk that starts with this row, 32 candidates at a time
       const int c = lo - 1 - lane;
-      const bool same = c >= 0 && (start_of(c) & ~kMid) == row_k;
+      const bool same = c >= 0 && chunk_row<COO>(a, c, other) == row_k;
       const unsigned m = __ballot_sync(0xffffffffu, same);
       const int run = m == 0xffffffffu ? 32 : __ffs(~m) - 1;
       lo -= run;
       if (run < 32) break;
     }
-    if (mine && (start_of(lo) & kMid)) lo -= 1;  // it began inside the chunk before
+    if (mine) {
+      chunk_row<COO>(a, lo, mid);
+      if (mid) --lo;                             // it began inside the chunk before
+    }
   }
-  pdl_wait();
+  if (!COO) pdl_wait();
   if (!mine) return;
   const float* base = a.part + static_cast<int64_t>(blockIdx.y) * a.nchunks * (2 * TILE) + l * 4;
   float acc[NV][4];
@@ -315,7 +362,7 @@ static size_t split_bytes(int64_t nnz, int f) {
   return static_cast<size_t>(s.nchunks) * s.tiles * s.lpn * s.nv * 32;     // two pieces of 16-byte vectors
 }
 
-template <int LPN, int NV, int BATCH>
+template <bool COO, int LPN, int NV, int BATCH>
 static int launch_split(const SplitArgs& a, int tiles, float beta, cudaStream_t s) {
   constexpr int G = 32 / LPN;
   const int per_block = kSplitWarps * G;
@@ -327,12 +374,12 @@ static int launch_split(const SplitArgs& a, int tiles, float beta, cudaStream_t 
   // that split of the L1 array for its whole run (R-MAT 1 M vertices, width 602, back to back: 5.4 -> 7.5 ms).
   const bool early = a.nnz * tiles <= (1 << 21);
   cudaError_t e;
-  if (beta != 0.f) {
-    e = launch_pdl_if(early, spmm_split_kernel<LPN, NV, BATCH, true>, grid, dim3(kSplitWarps * 32), 0, s, a);
-    if (e == cudaSuccess) e = launch_pdl(spmm_split_join_kernel<LPN, NV, true>, jgrid, dim3(128), 0, s, a, join_blocks);
-  } else {
-    e = launch_pdl_if(early, spmm_split_kernel<LPN, NV, BATCH, false>, grid, dim3(kSplitWarps * 32), 0, s, a);
-    if (e == cudaSuccess) e = launch_pdl(spmm_split_join_kernel<LPN, NV, false>, jgrid, dim3(128), 0, s, a, join_blocks);
+  if (COO || beta != 0.f) {      // COO is the accumulating operator only
+    e = launch_pdl_if(early, spmm_split_kernel<LPN, NV, BATCH, true, COO>, grid, dim3(kSplitWarps * 32), 0, s, a);
+    if (e == cudaSuccess) e = launch_pdl(spmm_split_join_kernel<LPN, NV, true, COO>, jgrid, dim3(128), 0, s, a, join_blocks);
+  } else if constexpr (!COO) {
+    e = launch_pdl_if(early, spmm_split_kernel<LPN, NV, BATCH, false, COO>, grid, dim3(kSplitWarps * 32), 0, s, a);
+    if (e == cudaSuccess) e = launch_pdl(spmm_split_join_kernel<LPN, NV, false, COO>, jgrid, dim3(128), 0, s, a, join_blocks);
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -341,10 +388,20 @@ static int launch_split(const SplitArgs& a, int tiles, float beta, cudaStream_t 
   return CAGNET_OK;
 }
 
+template <bool COO>
+static int dispatch_split(const SplitArgs& a, const SplitShape& sh, float beta, cudaStream_t stream) {
+  if (sh.lpn == 4) return launch_split<COO, 4, 1, 8>(a, sh.tiles, beta, stream);
+  if (sh.lpn == 8 && sh.nv == 1) return launch_split<COO, 8, 1, 8>(a, sh.tiles, beta, stream);
+  if (sh.lpn == 8 && sh.nv == 2) return launch_split<COO, 8, 2, 4>(a, sh.tiles, beta, stream);
+  if (sh.lpn == 8) return launch_split<COO, 8, 3, 4>(a, sh.tiles, beta, stream);
+  if (sh.nv == 1) return launch_split<COO, 16, 1, 4>(a, sh.tiles, beta, stream);
+  return launch_split<COO, 16, 2, 4>(a, sh.tiles, beta, stream);
+}
+
 static int run_split(const cagnet_block* b, const float* B, int64_t ldb, float* C, int64_t ldc, int f, float beta, void* ws,
                      cudaStream_t stream) {
   const SplitShape sh = split_shape(b->nnz, f);
-  SplitArgs a;
+  SplitArgs a = {};
   const int64_t padded = (b->nnz + kUnit - 1) / kUnit * kUnit;
   a.pairs = static_cast<const int2*>(b->split);
   a.first = reinterpret_cast<const unsigned*>(a.pairs + padded);
@@ -359,14 +416,8 @@ static int run_split(const cagnet_block* b, const float* B, int64_t ldb, float* 
   a.chunk = sh.chunk;
   a.nchunks = static_cast<int>(sh.nchunks);
   a.c_vec4 = (ldc % 4 == 0 && aligned(C, 16)) ? 1 : 0;
-  if (sh.lpn == 4) return launch_split<4, 1, 8>(a, sh.tiles, beta, stream);
-  if (sh.lpn == 8 && sh.nv == 1) return launch_split<8, 1, 8>(a, sh.tiles, beta, stream);
-  if (sh.lpn == 8 && sh.nv == 2) return launch_split<8, 2, 4>(a, sh.tiles, beta, stream);
-  if (sh.lpn == 8) return launch_split<8, 3, 4>(a, sh.tiles, beta, stream);
-  if (sh.nv == 1) return launch_split<16, 1, 4>(a, sh.tiles, beta, stream);
-  return launch_split<16, 2, 4>(a, sh.tiles, beta, stream);
+  return dispatch_split<false>(a, sh, beta, stream);
 }
-
 // The row kernels stay the better choice for small blocks of short rows: one launch instead of two and no pieces (ER,
 // 13.5 K nonzeros, width 16: 3.0 us against 6.5; at 280 K nonzeros the two are level, at power-law rows the split wins
 // from the smallest block on).
@@ -386,6 +437,19 @@ static bool b_aligned(const float* B, int64_t ldb) { return ldb % 4 == 0 && alig
 static bool pad_pays(const cagnet_block* b) { return b->nnz >= 2 * static_cast<int64_t>(b->m); }
 
 static size_t round256(size_t x) { return (x + 255) / 256 * 256; }
+
+// B in rows of whole vectors: itself, or a copy at w (then w, ldb move on).
+static const float* pad_rows(const float* B, int64_t& ldb, int m, int f, char*& w, cudaStream_t s) {
+  if (b_aligned(B, ldb)) return B;
+  const int ld4 = (f + 3) / 4;
+  const int64_t total = static_cast<int64_t>(m) * ld4, blocks = (total + 255) / 256;
+  float* out = reinterpret_cast<float*>(w);
+  launch_pdl(pad_rows_kernel, dim3(static_cast<unsigned>(blocks < 16 * kNumSMs ? blocks : 16 * kNumSMs)), dim3(256), 0, s, B, ldb, m, f,
+             ld4, reinterpret_cast<float4*>(out));
+  w += round256(static_cast<size_t>(m) * ld4 * 16);
+  ldb = ld4 * 4;
+  return out;
+}
 
 int split_launches(const cagnet_block* b, int32_t f) {
   if (use_tiles(b, f)) return split_launches(b->rest, f) + 2 + (b->joins > 0);
@@ -450,17 +514,7 @@ extern "C" int cagnet_spmm_block_f32(const cagnet_block* b, const float* B, int6
     if (ldb < f || ldc < f) return fail(CAGNET_E_ALIGN, "cagnet_spmm_block_f32: leading dimension smaller than f");
     char* w = static_cast<char*>(ws);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (!b_aligned(B, ldb)) {
-      const int ld4 = (f + 3) / 4;
-      const size_t bytes = round256(static_cast<size_t>(b->m) * ld4 * 16);
-      const int64_t total = static_cast<int64_t>(b->m) * ld4;
-      const int64_t blocks = (total + 255) / 256;
-      launch_pdl(pad_rows_kernel, dim3(static_cast<unsigned>(blocks < 16 * kNumSMs ? blocks : 16 * kNumSMs)), dim3(256), 0, s, B, ldb,
-                 b->m, f, ld4, reinterpret_cast<float4*>(w));
-      B = reinterpret_cast<const float*>(w);
-      ldb = ld4 * 4;
-      w += bytes;
-    }
+    B = pad_rows(B, ldb, b->m, f, w, s);
     const int rc = run_split(src, B, ldb, C, ldc, f, beta, w, s);
     if (rc != CAGNET_OK) return rc;
     ws = w + round256(split_bytes(src->nnz, f));
@@ -469,4 +523,35 @@ extern "C" int cagnet_spmm_block_f32(const cagnet_block* b, const float* B, int6
   return cagnet_tile_core_f32(b->tile_bits, b->tile_kb, b->panel_ptr, b->cta_ptr, b->ctas, b->panels, b->join_list, b->joins,
                               b->tile_cols, b->tile_kbs, b->panel_rows, b->panel_scale, b->col_scale, B, ldb, C, ldc, f, ws,
                               cagnet_tile_core_workspace_bytes(b->tile_kbs, b->ctas, f), stream);
+}
+
+extern "C" size_t cagnet_spmm_coo_workspace_bytes(int32_t m, int64_t nnz, const float* B, int64_t ldb, int32_t f) {
+  if (nnz <= 0 || f <= 0) return 0;
+  return round256(split_bytes(nnz, f)) + (b_aligned(B, ldb) ? 0 : round256(static_cast<size_t>(m) * ((f + 3) / 4) * 16));
+}
+
+extern "C" int cagnet_spmm_coo_f32(const int32_t* rows, const int32_t* cols, const float* vals, int32_t n, int32_t m, int64_t nnz,
+                                   const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f, const int32_t* status,
+                                   void* ws, size_t ws_bytes, void* stream) {
+  if (n < 0 || m < 0 || nnz < 0 || f < 0) return fail(CAGNET_E_ARG, "cagnet_spmm_coo_f32: negative size");
+  if (n == 0 || nnz == 0 || f == 0) return CAGNET_OK;
+  if (!rows || !cols || !vals || !B || !C || !ws) return fail(CAGNET_E_ARG, "cagnet_spmm_coo_f32: null pointer");
+  if (nnz > INT_MAX) return fail(CAGNET_E_OVERFLOW, "cagnet_spmm_coo_f32: nnz %s%lld exceeds int32", "", nnz);
+  if (ldb < f || ldc < f) return fail(CAGNET_E_ALIGN, "cagnet_spmm_coo_f32: leading dimension smaller than f");
+  if (ws_bytes < cagnet_spmm_coo_workspace_bytes(m, nnz, B, ldb, f)) return fail(CAGNET_E_WORKSPACE, "cagnet_spmm_coo_f32: workspace too small");
+  char* w = static_cast<char*>(ws);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  B = pad_rows(B, ldb, m, f, w, s);
+  const SplitShape sh = split_shape(nnz, f);
+  SplitArgs a = {};
+  a.coo_rows = rows; a.coo_cols = cols; a.coo_vals = vals; a.status = status;
+  a.nrows = n;                 // no chunk starts in row n
+  a.B = B; a.C = C;
+  a.part = reinterpret_cast<float*>(w);
+  a.nnz = nnz; a.ldb = ldb; a.ldc = ldc;
+  a.f = f; a.f_eff = (f + 3) / 4 * 4;
+  a.chunk = sh.chunk;
+  a.nchunks = static_cast<int>(sh.nchunks);
+  a.c_vec4 = (ldc % 4 == 0 && aligned(C, 16)) ? 1 : 0;
+  return dispatch_split<true>(a, sh, 1.f, s);
 }

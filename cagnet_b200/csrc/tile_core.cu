@@ -262,10 +262,6 @@ __device__ __forceinline__ int tile_panel(const TileArgs& a, int u) {
   return lo;
 }
 
-__device__ __forceinline__ void red_add4(float* p, float4 v) {
-  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-}
-
 // WIDE: the three terms are accumulated into one sum by three products of N = NT; otherwise they sit side by side in
 // one product of N = 3 NT and are added when the sums are read.
 template <bool WIDE>

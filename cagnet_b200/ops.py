@@ -568,18 +568,13 @@ def spmm_gpu(A_rowindices, A_colindices, A_values, n, m, B, C, validate=None):
         raise RuntimeError("cagnet_b200: spmm_gpu expects int32 indices (call .int() as the reference does)")
     if n > _INT32_MAX or m > _INT32_MAX:
         raise RuntimeError("cagnet_b200: spmm_gpu block does not fit 32-bit indices")
-    rows32 = A_rowindices.contiguous()
-    block = CsrBlock(coo2csr(rows32, n), A_colindices.contiguous(), A_values.float().contiguous(), n, m)
-    if SPMM_GPU_VALIDATE if validate is None else validate:
-        block.validate(rows32)
-    block.build_plan(core=False, lasting=False)      # a per-call block: what is prepared once pays only when it is reused
+    rows, cols, vals = A_rowindices.contiguous(), A_colindices.contiguous(), A_values.float().contiguous()
+    check = SPMM_GPU_VALIDATE if validate is None else validate
     Bc = B if _row_major(B) else B.contiguous()
-    if _row_major(C):
-        spmm(block, Bc, C, 1.0)
-    else:  # e.g. the column-major-strided views the reference's own op leaves behind
-        tmp = C.contiguous()
-        spmm(block, Bc, tmp, 1.0)
-        C.copy_(tmp)
+    Cc = C if _row_major(C) else C.contiguous()     # e.g. the column-major-strided views the reference's own op leaves behind
+    LAUNCHES[0] += _native.host().spmm_coo(rows, cols, vals, n, m, Bc, Cc, bool(check))
+    if Cc is not C:
+        C.copy_(Cc)
 
 
 def sparse_coo_tensor_gpu(indices, values, size):

@@ -168,6 +168,17 @@ int cagnet_spmm_block_launches(const cagnet_block* block, int32_t f);
 int cagnet_spmm_block_f32(const cagnet_block* block, const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f,
                           float beta, void* ws, size_t ws_bytes, void* stream);
 
+/* C += A*B with A as row-sorted COO and nothing prepared: the nonzero split straight from the index arrays.  With `status`
+ * (device) not NULL nothing is done when *status is nonzero at the time the kernels run, so that the product can be queued
+ * behind cagnet_check_coo_i32 before its verdict is read back: 0, 3 unsorted rows, 4 column range, 5 row range.
+ * ws: cagnet_spmm_coo_workspace_bytes for the same B, ldb, f.  sparse_coo_tensor.cu:113-240. */
+int cagnet_check_coo_i32(const int32_t* rows, const int32_t* cols, int32_t n, int32_t m, int64_t nnz, int32_t* status_dev,
+                         void* stream);
+size_t cagnet_spmm_coo_workspace_bytes(int32_t m, int64_t nnz, const float* B, int64_t ldb, int32_t f);
+int cagnet_spmm_coo_f32(const int32_t* rows, const int32_t* cols, const float* vals, int32_t n, int32_t m, int64_t nnz,
+                        const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f, const int32_t* status, void* ws,
+                        size_t ws_bytes, void* stream);
+
 /* ---- Dense tiles of a normalised block as bit matrices (256 rows x 64 columns, rows and columns taken in order of degree:
  * rank_r / rank_c give a row's / column's place, tiles are searched among the first lim_r x lim_c).
  *   cagnet_tile_count_i32   counts[p * ceil(lim_c / 64) + q] += nonzeros of tile (p, q) (counts zeroed by the caller)
