@@ -75,5 +75,13 @@ int spmm_rows_f32(const int32_t* rowptr, const int32_t* col, const float* val, i
 int spmm_forced_tile();      // "spmm_tile" when a sweep has set it: such multiplies run the row kernels
 int split_launches(const cagnet_block* b, int32_t f);
 
+// X . W on the tensor cores (dense_tc.cu), where it applies
+bool gemm_nn_tc_applies(const float* X, int64_t ldx, int64_t n, int K, int N, int epilogue);
+int gemm_nn_tc(const float* X, int64_t ldx, const float* W, int64_t ldw, int transW, float* Z, int64_t ldz, int64_t n, int K, int N,
+               int epilogue, const float* aux, int64_t ldaux, cudaStream_t s);
+bool gemm_tn_tc_applies(const float* H, int64_t ldh, const float* G, int64_t ldg, int64_t n, int K, int N);
+int gemm_tn_tc_blocks(int64_t n, int K, int N);
+int gemm_tn_tc(const float* H, int64_t ldh, const float* G, int64_t ldg, int64_t n, int K, int N, float* part, cudaStream_t s);
+int gemm_tc_error();      // 1 if one of its kernels gave up on a wait
 
 }  // namespace cagnet

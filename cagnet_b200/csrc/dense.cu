@@ -12,129 +12,297 @@
 namespace cagnet {
 
 // ------------------------------------------------------------------------------------------------
-// Z[n x N] = epilogue(X[n x K] * W)       block: 128 rows x (8*TN) columns, 256 threads
-// thread (rg = tid/8, cg = tid%8) owns rows rg*4..rg*4+3 and columns cg + 8*t, t < TN.
-constexpr int kBM = 128;
-constexpr int kBK = 32;
+// Z[n x N] = epilogue(X[n x K] * W) for tall X and small W, fp32 FMAs.
+//
+// A thread owns TM rows and NP groups of 4 columns; LC lanes side by side cover one row of the tile (LC * 4 * NP columns), the
+// 32 / LC row groups of a warp share their W values through broadcasts.  Per k that is TM / 4 + NP 128-bit shared-memory reads
+// for 4 TM NP FMAs (8 x 4: three reads for 32), so the FMA pipe and HBM are what bounds it: 233K x 602 x 16 is 62 us of FMAs
+// at the peak rate over 86 us of X at the copy rate.  X tiles are fetched row by row (whole 64- or 128-byte pieces), held in
+// registers while the previous tile is multiplied, and stored k-major with rows permuted by k / 4 (xor of row bits 2-4),
+// which makes both the transposing stores and the row-vector reads conflict-free.
+template <int BK>
+__device__ __forceinline__ int x_swizzle(int k) { return (32 / (BK / 4)) * ((k >> 2) & (BK / 4 - 1)); }
 
-template <int TN>
-__global__ void __launch_bounds__(256) gemm_nn_kernel(const float* __restrict__ X, int64_t ldx,
-                                                      const float* __restrict__ W, int64_t ldw, int transW,
-                                                      float* __restrict__ Z, int64_t ldz, int64_t n, int K, int N,
-                                                      int epilogue, const float* __restrict__ aux, int64_t ldaux,
-                                                      int x_vec4) {
-  constexpr int NT = 8 * TN;
-  __shared__ float Xs[kBK][kBM + 1];
-  __shared__ float Ws[kBK][NT];
-  const int tid = threadIdx.x;
-  const int cg = tid & 7, rg = tid >> 3;
-  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * kBM;
-  const int n0 = blockIdx.y * NT;
+struct GemmArgs {
+  const float *X, *W, *aux;
+  float* Z;
+  int64_t ldx, ldw, ldz, ldaux, n;
+  int transW, K, N, epilogue, x_vec4, z_vec4;
+};
 
-  float acc[4][TN];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int t = 0; t < TN; ++t) acc[i][t] = 0.f;
+// 4 consecutive k of row gr (zeros outside the matrix)
+__device__ __forceinline__ float4 load_x4(const GemmArgs& a, int64_t gr, int k) {
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (gr < a.n && k < a.K) {
+    const float* p = a.X + gr * a.ldx + k;
+    if (a.x_vec4 && k + 3 < a.K) {
+      v = __ldg(reinterpret_cast<const float4*>(p));
+    } else {
+      v.x = __ldg(p);
+      if (k + 1 < a.K) v.y = __ldg(p + 1);
+      if (k + 2 < a.K) v.z = __ldg(p + 2);
+      if (k + 3 < a.K) v.w = __ldg(p + 3);
+    }
+  }
+  return v;
+}
+__device__ __forceinline__ float load_w(const GemmArgs& a, int k, int j) {
+  if (k >= a.K || j >= a.N) return 0.f;
+  return __ldg(a.W + (a.transW ? static_cast<int64_t>(j) * a.ldw + k : static_cast<int64_t>(k) * a.ldw + j));
+}
 
-  // The X tile of step k+1 is fetched into registers while step k is being multiplied, so the kernel waits for
-  // HBM once per tile instead of once per tile and synchronisation.
-  constexpr int WPT = (kBK * NT + 255) / 256;     // W elements per thread and step
-  const int kk = (tid & 7) * 4;
-  float xv[4][4];
-  float wv[WPT];
-
-  auto fetch = [&](int k0) {
+template <int BK, int LC, int NP, int TM>
+__device__ __forceinline__ void tile_product(const float* __restrict__ Xs, int ldxs, const float* __restrict__ Ws, int r0, int lc,
+                                             float (&acc)[TM][NP][4]) {
+  constexpr int BN = LC * 4 * NP;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int64_t gr = row0 + (tid >> 3) + 32 * i;
+  for (int k = 0; k < BK; ++k) {
+    float x[TM];
+    const float* xp = Xs + k * ldxs;
+    const int sw = x_swizzle<BK>(k);
+    if constexpr (TM >= 4) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) xv[i][j] = 0.f;
-      if (gr < n) {
-        const float* xp = X + gr * ldx + k0 + kk;
-        if (x_vec4 && k0 + kk + 3 < K) {
-          const float4 t4 = __ldg(reinterpret_cast<const float4*>(xp));
-          xv[i][0] = t4.x; xv[i][1] = t4.y; xv[i][2] = t4.z; xv[i][3] = t4.w;
-        } else {
+      for (int q = 0; q < TM / 4; ++q) {
+        const float4 t = *reinterpret_cast<const float4*>(xp + ((r0 + 4 * q) ^ sw));
+        x[4 * q] = t.x; x[4 * q + 1] = t.y; x[4 * q + 2] = t.z; x[4 * q + 3] = t.w;
+      }
+    } else {
+      const float2 t = *reinterpret_cast<const float2*>(xp + (r0 ^ sw));
+      x[0] = t.x; x[1] = t.y;
+    }
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (k0 + kk + j < K) xv[i][j] = __ldg(xp + j);
-        }
+    for (int p = 0; p < NP; ++p) {
+      const float4 w = *reinterpret_cast<const float4*>(Ws + k * BN + p * (LC * 4) + lc * 4);
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        acc[i][p][0] = fmaf(x[i], w.x, acc[i][p][0]);
+        acc[i][p][1] = fmaf(x[i], w.y, acc[i][p][1]);
+        acc[i][p][2] = fmaf(x[i], w.z, acc[i][p][2]);
+        acc[i][p][3] = fmaf(x[i], w.w, acc[i][p][3]);
       }
     }
+  }
+}
+
+// Four columns of a row through the elementwise epilogues and out.
+__device__ __forceinline__ void store_z4(const GemmArgs& a, int64_t gr, int c, float4 v) {
+  const int live = a.N - c;
+  if (live <= 0) return;
+  float* z = a.Z + gr * a.ldz + c;
+  float r[4] = {v.x, v.y, v.z, v.w};
+  if (a.epilogue == CAGNET_EPI_RELU) {
 #pragma unroll
-    for (int u = 0; u < WPT; ++u) {
-      const int idx = tid + 256 * u;
-      const int k = idx / NT, j = idx % NT;
-      float w = 0.f;
-      if (idx < kBK * NT && k0 + k < K && n0 + j < N)
-        w = transW ? __ldg(W + static_cast<int64_t>(n0 + j) * ldw + k0 + k) : __ldg(W + static_cast<int64_t>(k0 + k) * ldw + n0 + j);
-      wv[u] = w;
+    for (int j = 0; j < 4; ++j) r[j] = fmaxf(r[j], 0.f);
+  } else if (a.epilogue == CAGNET_EPI_RELU_MASK) {
+    const float* p = a.aux + gr * a.ldaux + c;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < live) r[j] = __ldg(p + j) > 0.f ? r[j] : 0.f;
+  } else if (a.epilogue == CAGNET_EPI_ACCUMULATE) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < live) r[j] += z[j];
+  }
+  if (live >= 4 && a.z_vec4) {
+    *reinterpret_cast<float4*>(z) = make_float4(r[0], r[1], r[2], r[3]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < live) z[j] = r[j];
+  }
+}
+
+// log(sum(exp)) of a row spread over LANES neighbouring lanes, COLS values each; columns from `live` on do not count.
+template <int LANES, int COLS>
+__device__ __forceinline__ float row_lse(const float (&v)[COLS], const bool (&live)[COLS]) {
+  float mx = -INFINITY;
+#pragma unroll
+  for (int j = 0; j < COLS; ++j)
+    if (live[j]) mx = fmaxf(mx, v[j]);
+#pragma unroll
+  for (int off = 1; off < LANES; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  float sum = 0.f;
+#pragma unroll
+  for (int j = 0; j < COLS; ++j) sum += live[j] ? expf(v[j] - mx) : 0.f;
+#pragma unroll
+  for (int off = 1; off < LANES; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  return mx + logf(sum);
+}
+
+template <int LC, int NP, int TM, int WARPS, int BK>
+__global__ void __launch_bounds__(WARPS * 32) gemm_nn_kernel(GemmArgs a) {
+  constexpr int BN = LC * 4 * NP, WR = 32 / LC * TM, BM = WARPS * WR, T = WARPS * 32;
+  constexpr int XV = BM * BK / 4 / T;            // float4 of X per thread and tile
+  constexpr int WV = (BK * BN + T - 1) / T;
+  static_assert(BM % 32 == 0 && BM * BK / 4 % T == 0, "tile shape");
+  __shared__ __align__(16) float Xs[BK * BM];
+  __shared__ __align__(16) float Ws[BK * BN];
+  pdl_trigger();
+  pdl_wait();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int lc = lane % LC, r0 = warp * WR + lane / LC * TM;
+  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * BM;
+  const int n0 = blockIdx.y * BN;
+
+  float acc[TM][NP][4];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][p][j] = 0.f;
+
+  float4 xv[XV];
+  float wv[WV];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < XV; ++u) {
+      const int idx = tid + T * u;
+      xv[u] = load_x4(a, row0 + idx / (BK / 4), k0 + idx % (BK / 4) * 4);
+    }
+#pragma unroll
+    for (int u = 0; u < WV; ++u) {
+      const int idx = tid + T * u;
+      wv[u] = idx < BK * BN ? load_w(a, k0 + idx / BN, n0 + idx % BN) : 0.f;
     }
   };
-
   fetch(0);
-  for (int k0 = 0; k0 < K; k0 += kBK) {
-    // X tile: 128 rows x 32 k, read row-contiguous, stored k-major; W tile: 32 k x NT columns
+  for (int k0 = 0; k0 < a.K; k0 += BK) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int u = 0; u < XV; ++u) {
+      const int idx = tid + T * u;
+      const int r = idx / (BK / 4), k = idx % (BK / 4) * 4;
+      const int at = r ^ x_swizzle<BK>(k);
+      Xs[(k + 0) * BM + at] = xv[u].x;
+      Xs[(k + 1) * BM + at] = xv[u].y;
+      Xs[(k + 2) * BM + at] = xv[u].z;
+      Xs[(k + 3) * BM + at] = xv[u].w;
+    }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) Xs[kk + j][(tid >> 3) + 32 * i] = xv[i][j];
-#pragma unroll
-    for (int u = 0; u < WPT; ++u) {
-      const int idx = tid + 256 * u;
-      if (idx < kBK * NT) Ws[idx / NT][idx % NT] = wv[u];
+    for (int u = 0; u < WV; ++u) {
+      const int idx = tid + T * u;
+      if (idx < BK * BN) Ws[idx] = wv[u];
     }
     __syncthreads();
-    if (k0 + kBK < K) fetch(k0 + kBK);
-#pragma unroll 8
-    for (int k = 0; k < kBK; ++k) {
-      float x[4], w[TN];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] = Xs[k][rg * 4 + i];
-#pragma unroll
-      for (int t = 0; t < TN; ++t) w[t] = Ws[k][cg + 8 * t];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int t = 0; t < TN; ++t) acc[i][t] = fmaf(x[i], w[t], acc[i][t]);
-    }
+    if (k0 + BK < a.K) fetch(k0 + BK);
+    tile_product<BK, LC, NP, TM>(Xs, BM, Ws, r0, lc, acc);
     __syncthreads();
   }
 
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t gr = row0 + rg * 4 + i;
-    const bool row_ok = gr < n;   // no early exit: the shuffles below need all 32 lanes
-    if (epilogue == CAGNET_EPI_LOG_SOFTMAX) {
-      float mx = -INFINITY;
+  for (int i = 0; i < TM; ++i) {
+    const int64_t gr = row0 + r0 + i;            // no early exit: the shuffles need all lanes
+    if (a.epilogue == CAGNET_EPI_LOG_SOFTMAX || a.epilogue == CAGNET_EPI_LOG_SOFTMAX_256) {
+      float v[NP * 4];
+      bool live[NP * 4];
 #pragma unroll
-      for (int t = 0; t < TN; ++t)
-        if (n0 + cg + 8 * t < N) mx = fmaxf(mx, acc[i][t]);
+      for (int p = 0; p < NP; ++p)
 #pragma unroll
-      for (int off = 1; off < 8; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-      float sum = 0.f;
+        for (int j = 0; j < 4; ++j) {
+          v[p * 4 + j] = acc[i][p][j];
+          live[p * 4 + j] = p * (LC * 4) + lc * 4 + j < a.N;
+        }
+      const float lse = row_lse<LC, NP * 4>(v, live);
 #pragma unroll
-      for (int t = 0; t < TN; ++t)
-        if (n0 + cg + 8 * t < N) sum += expf(acc[i][t] - mx);
+      for (int p = 0; p < NP; ++p)
 #pragma unroll
-      for (int off = 1; off < 8; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-      const float lse = mx + logf(sum);
-#pragma unroll
-      for (int t = 0; t < TN; ++t) acc[i][t] -= lse;
+        for (int j = 0; j < 4; ++j) acc[i][p][j] -= lse;
     }
-    if (!row_ok) continue;
+    if (gr < a.n) {
 #pragma unroll
-    for (int t = 0; t < TN; ++t) {
-      const int c = n0 + cg + 8 * t;
-      if (c < N) {
-        float v = acc[i][t];
-        if (epilogue == CAGNET_EPI_RELU) v = fmaxf(v, 0.f);
-        else if (epilogue == CAGNET_EPI_RELU_MASK) v = (__ldg(aux + gr * ldaux + c) > 0.f) ? v : 0.f;
-        else if (epilogue == CAGNET_EPI_ACCUMULATE) v += Z[gr * ldz + c];
-        Z[gr * ldz + c] = v;
-      }
+      for (int p = 0; p < NP; ++p)
+        store_z4(a, gr, n0 + p * (LC * 4) + lc * 4, make_float4(acc[i][p][0], acc[i][p][1], acc[i][p][2], acc[i][p][3]));
     }
+  }
+}
+
+// The same product for few rows and a long K: 16 rows per block, its 8 warps take K tiles in turn (own tiles, no block
+// barrier), their sums are added in warp order.  2,708 x 1,433 x 16 is 11 blocks of the kernel above, each a chain of 90
+// tiles (35 us); here 170 blocks of 6 tiles per warp (N <= 64).
+template <int LC, int TM>
+__global__ void __launch_bounds__(256) gemm_nn_splitk_kernel(GemmArgs a) {
+  constexpr int BK = LC == 4 ? 32 : 16, BN = LC * 4, ROWS = 32 / LC * TM, WARPS = 8, CPT = BN / 16;      // 48 KB of tiles
+  static_assert(ROWS == 16, "16 rows per warp");
+  __shared__ __align__(16) float Xs[WARPS][BK * 32];        // 16 rows used: the permutation moves rows inside 32
+  __shared__ __align__(16) float Ws[WARPS][BK * BN];
+  pdl_trigger();
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lc = lane % LC, r0 = lane / LC * TM;
+  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * ROWS;
+  float acc[TM][1][4];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][0][j] = 0.f;
+  constexpr int XV = ROWS * BK / 4 / 32, WV = BK * BN / 4 / 32;
+  const bool w_vec4 = !a.transW && a.N == BN && a.ldw % 4 == 0 && aligned(a.W, 16);
+  float4 xv[XV], wv[WV];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < XV; ++u) {
+      const int idx = lane + 32 * u;
+      xv[u] = load_x4(a, row0 + idx / (BK / 4), k0 + idx % (BK / 4) * 4);
+    }
+#pragma unroll
+    for (int u = 0; u < WV; ++u) {
+      const int idx = (lane + 32 * u) * 4, k = k0 + idx / BN, j = idx % BN;
+      if (w_vec4 && k < a.K) wv[u] = __ldg(reinterpret_cast<const float4*>(a.W + static_cast<int64_t>(k) * a.ldw + j));
+      else wv[u] = make_float4(load_w(a, k, j), load_w(a, k, j + 1), load_w(a, k, j + 2), load_w(a, k, j + 3));
+    }
+  };
+  int k0 = warp * BK;
+  fetch(k0);
+  for (; k0 < a.K; k0 += WARPS * BK) {
+#pragma unroll
+    for (int u = 0; u < XV; ++u) {
+      const int idx = lane + 32 * u;
+      const int r = idx / (BK / 4), k = idx % (BK / 4) * 4;
+      const int at = r ^ x_swizzle<BK>(k);
+      Xs[warp][(k + 0) * 32 + at] = xv[u].x;
+      Xs[warp][(k + 1) * 32 + at] = xv[u].y;
+      Xs[warp][(k + 2) * 32 + at] = xv[u].z;
+      Xs[warp][(k + 3) * 32 + at] = xv[u].w;
+    }
+#pragma unroll
+    for (int u = 0; u < WV; ++u) *reinterpret_cast<float4*>(&Ws[warp][(lane + 32 * u) * 4]) = wv[u];
+    __syncwarp();
+    if (k0 + WARPS * BK < a.K) fetch(k0 + WARPS * BK);
+    tile_product<BK, LC, 1, TM>(Xs[warp], 32, Ws[warp], r0, lc, acc);
+    __syncwarp();
+  }
+  // sums of the 8 warps, each in its own W tile
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+    *reinterpret_cast<float4*>(&Ws[warp][(r0 + i) * BN + lc * 4]) = make_float4(acc[i][0][0], acc[i][0][1], acc[i][0][2], acc[i][0][3]);
+  __syncthreads();
+  // 16 lanes per row, CPT columns each
+  const int r = threadIdx.x >> 4, c = (threadIdx.x & 15) * CPT;
+  float v[CPT];
+  bool live[CPT];
+#pragma unroll
+  for (int j = 0; j < CPT; ++j) {
+    v[j] = 0.f;
+    live[j] = c + j < a.N;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) v[j] += Ws[w][r * BN + c + j];
+  }
+  if (a.epilogue == CAGNET_EPI_LOG_SOFTMAX) {
+    const float lse = row_lse<16, CPT>(v, live);
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) v[j] -= lse;
+  }
+  const int64_t gr = row0 + r;
+  if (gr >= a.n) return;
+#pragma unroll
+  for (int j = 0; j < CPT; ++j) {
+    if (!live[j]) continue;
+    float* z = a.Z + gr * a.ldz + c + j;
+    float t = v[j];
+    if (a.epilogue == CAGNET_EPI_RELU) t = fmaxf(t, 0.f);
+    else if (a.epilogue == CAGNET_EPI_RELU_MASK) t = __ldg(a.aux + gr * a.ldaux + c + j) > 0.f ? t : 0.f;
+    else if (a.epilogue == CAGNET_EPI_ACCUMULATE) t += *z;
+    *z = t;
   }
 }
 
@@ -342,25 +510,29 @@ __global__ void __launch_bounds__(256, 2) gemm_tn_small_kernel(const float* __re
   }
 }
 
-// out[k, j] (+)= sum over the row chunks of their partial products.  One warp per output element: lane l adds
-// chunks l, l + 32, ... in that order, then the 32 lane sums are folded by a fixed shuffle tree -- the same order
-// on every run.  (One thread per element walking all chunks took 56 us for a 16 x 41 product cut into 561 chunks.)
+// out[k, j] (+)= sum over the row chunks of their partial products.  A block takes 32 neighbouring elements: warp w adds chunks
+// w, w + 8, ... of all 32 (whole 128-byte reads), the eight sums are added in warp order -- the same order on every run.
 __global__ void __launch_bounds__(256)
 gemm_tn_reduce_kernel(const float* __restrict__ ws, int chunks, int K, int N, float* __restrict__ out, int64_t ldo,
                       float beta, int transposed) {
-  const int idx = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;      // warp-uniform
-  const int lane = threadIdx.x & 31;
-  if (idx >= K * N) return;
+  __shared__ float red[8][32];
+  pdl_trigger();
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int idx = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int c = lane; c < chunks; c += 32) s += __ldg(ws + static_cast<int64_t>(c) * K * N + idx);
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-  if (lane == 0) {
-    // transposed: the partials are those of G^T * H (K and N as passed here); out is (H^T * G)[N x K]
-    float* o = transposed ? out + static_cast<int64_t>(idx % N) * ldo + idx / N
-                          : out + static_cast<int64_t>(idx / N) * ldo + idx % N;
-    *o = (beta != 0.f) ? s + *o : s;
+  if (idx < K * N) {
+#pragma unroll 4
+    for (int c = warp; c < chunks; c += 8) s += __ldg(ws + static_cast<int64_t>(c) * K * N + idx);
   }
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp || idx >= K * N) return;
+#pragma unroll
+  for (int w = 1; w < 8; ++w) s += red[w][lane];
+  // transposed: the partials are those of G^T * H (K and N as passed here); out is (H^T * G)[N x K]
+  float* o = transposed ? out + static_cast<int64_t>(idx % N) * ldo + idx / N : out + static_cast<int64_t>(idx / N) * ldo + idx % N;
+  *o = (beta != 0.f) ? s + *o : s;
 }
 
 struct TnShape {
@@ -388,31 +560,97 @@ static TnShape tn_shape(int64_t n, int K, int N) {
 }
 
 // ------------------------------------------------------------------------------------------------
-__global__ void relu_fwd_kernel(const float* __restrict__ z, int64_t ldz, float* __restrict__ h, int64_t ldh, int64_t n,
-                                int N) {
-  const int64_t total = n * N;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t r = i / N;
-    const int c = static_cast<int>(i - r * N);
-    h[r * ldh + c] = fmaxf(z[r * ldz + c], 0.f);
+// Element (row, group of 4 columns) of a thread's grid-stride step; 32-bit division where the count allows it.
+__device__ __forceinline__ void vec_index(int64_t i, int64_t total, int vecs, int64_t& r, int& c) {
+  r = total <= INT_MAX ? static_cast<int>(i) / vecs : i / vecs;
+  c = static_cast<int>(i - r * vecs) * 4;
+}
+__device__ __forceinline__ float4 load4_upto(const float* p, int live, int vec4) {
+  if (vec4 && live >= 4) return *reinterpret_cast<const float4*>(p);
+  float4 v = make_float4(p[0], 0.f, 0.f, 0.f);
+  if (live > 1) v.y = p[1];
+  if (live > 2) v.z = p[2];
+  if (live > 3) v.w = p[3];
+  return v;
+}
+__device__ __forceinline__ void store4_upto(float* p, float4 v, int live, int vec4) {
+  if (vec4 && live >= 4) {
+    *reinterpret_cast<float4*>(p) = v;
+  } else {
+    p[0] = v.x;
+    if (live > 1) p[1] = v.y;
+    if (live > 2) p[2] = v.z;
+    if (live > 3) p[3] = v.w;
   }
 }
 
-__global__ void relu_bwd_kernel(const float* __restrict__ h, int64_t ldh, const float* __restrict__ g, int64_t ldg,
-                                float* __restrict__ dz, int64_t lddz, int64_t n, int N) {
-  const int64_t total = n * N;
+// One 16-byte read (two for the gradient) and write per thread and step; z and h may be the same matrix.
+__global__ void __launch_bounds__(256) relu_fwd_kernel(const float* z, int64_t ldz, float* h, int64_t ldh, int64_t n, int N, int vecs,
+                                                       int vec4) {
+  pdl_trigger();
+  pdl_wait();
+  const int64_t total = n * vecs;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t r = i / N;
-    const int c = static_cast<int>(i - r * N);
-    dz[r * lddz + c] = h[r * ldh + c] > 0.f ? g[r * ldg + c] : 0.f;
+    int64_t r;
+    int c;
+    vec_index(i, total, vecs, r, c);
+    const float4 v = load4_upto(z + r * ldz + c, N - c, vec4);
+    store4_upto(h + r * ldh + c, make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f)), N - c, vec4);
   }
 }
 
-// one warp per row
-__global__ void log_softmax_fwd_kernel(const float* __restrict__ z, int64_t ldz, float* __restrict__ out, int64_t ldo,
-                                       int64_t n, int N) {
+__global__ void __launch_bounds__(256) relu_bwd_kernel(const float* __restrict__ h, int64_t ldh, const float* g, int64_t ldg, float* dz,
+                                                       int64_t lddz, int64_t n, int N, int vecs, int vec4) {
+  pdl_trigger();
+  pdl_wait();
+  const int64_t total = n * vecs;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    int64_t r;
+    int c;
+    vec_index(i, total, vecs, r, c);
+    const float4 v = load4_upto(h + r * ldh + c, N - c, vec4), q = load4_upto(g + r * ldg + c, N - c, vec4);
+    store4_upto(dz + r * lddz + c, make_float4(v.x > 0.f ? q.x : 0.f, v.y > 0.f ? q.y : 0.f, v.z > 0.f ? q.z : 0.f, v.w > 0.f ? q.w : 0.f),
+                N - c, vec4);
+  }
+}
+
+// LR lanes per row, NV groups of 4 columns per lane (column 4 lane + 4 LR v): the row is read once into registers (16-byte
+// loads), reduced by shuffles and written back; z and out may be the same matrix.  (One warp per row walking it three
+// times took 87 us for 300K x 47 and 243 us for 700K x 256.)
+template <int LR, int NV>
+__global__ void __launch_bounds__(256) log_softmax_fwd_kernel(const float* z, int64_t ldz, float* out, int64_t ldo, int64_t n, int N,
+                                                              int vec4) {
+  pdl_trigger();
+  pdl_wait();
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * (256 / LR) + threadIdx.x / LR;
+  const int l = threadIdx.x % LR;
+  const bool have = row < n;
+  float v[NV * 4];
+  bool live[NV * 4];
+#pragma unroll
+  for (int w = 0; w < NV; ++w) {
+    const int c = (l + LR * w) * 4;
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (have && c < N) t = load4_upto(z + row * ldz + c, N - c, vec4);
+    v[4 * w] = t.x; v[4 * w + 1] = t.y; v[4 * w + 2] = t.z; v[4 * w + 3] = t.w;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) live[4 * w + j] = c + j < N;
+  }
+  const float lse = row_lse<LR, NV * 4>(v, live);
+  if (!have) return;
+#pragma unroll
+  for (int w = 0; w < NV; ++w) {
+    const int c = (l + LR * w) * 4;
+    if (c < N) store4_upto(out + row * ldo + c, make_float4(v[4 * w] - lse, v[4 * w + 1] - lse, v[4 * w + 2] - lse, v[4 * w + 3] - lse), N - c, vec4);
+  }
+}
+
+// wider rows: one warp per row
+__global__ void log_softmax_fwd_wide_kernel(const float* z, int64_t ldz, float* out, int64_t ldo, int64_t n, int N) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t row = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= n) return;
   const int lane = threadIdx.x & 31;
@@ -638,34 +876,62 @@ extern "C" int cagnet_gemm_nn_f32(const float* X, int64_t ldx, const float* W, i
   if (n < 0 || K < 0 || N < 0) return fail(CAGNET_E_ARG, "cagnet_gemm_nn_f32: negative size");
   if (n == 0 || N == 0) return CAGNET_OK;
   if (!X || !W || !Z) return fail(CAGNET_E_ARG, "cagnet_gemm_nn_f32: null pointer");
-  if (epilogue < 0 || epilogue > 4) return fail(CAGNET_E_ARG, "cagnet_gemm_nn_f32: unknown epilogue");
+  if (epilogue < 0 || epilogue > 5) return fail(CAGNET_E_ARG, "cagnet_gemm_nn_f32: unknown epilogue");
   if (epilogue == CAGNET_EPI_RELU_MASK && (!aux || ldaux < N))
     return fail(CAGNET_E_ARG, "cagnet_gemm_nn_f32: the ReLU-mask epilogue needs aux (n x N)");
   if (epilogue == CAGNET_EPI_LOG_SOFTMAX && N > 64)
     return fail(CAGNET_E_ARG, "cagnet_gemm_nn_f32: fused log-softmax supports N <= 64 (got %s%lld)", "", N);
+  if (epilogue == CAGNET_EPI_LOG_SOFTMAX_256 && N > 256)
+    return fail(CAGNET_E_ARG, "cagnet_gemm_nn_f32: fused log-softmax supports N <= 256 (got %s%lld)", "", N);
   if (ldx < K || ldz < N || ldw < (transW ? K : N))
     return fail(CAGNET_E_ALIGN, "cagnet_gemm_nn_f32: leading dimension smaller than the row width");
-  if ((n + kBM - 1) / kBM > INT_MAX) return fail(CAGNET_E_OVERFLOW, "cagnet_gemm_nn_f32: too many rows");
+  if ((n + 15) / 16 > INT_MAX) return fail(CAGNET_E_OVERFLOW, "cagnet_gemm_nn_f32: too many rows");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int x_vec4 = (ldx % 4 == 0 && aligned(X, 16)) ? 1 : 0;
-  const unsigned gx = static_cast<unsigned>((n + kBM - 1) / kBM);
-  const int per = N <= 64 ? (N + 7) / 8 : 8;   // columns per thread
-#define CAGNET_GEMM_CASE(TN)                                                                                    \
-  gemm_nn_kernel<TN><<<dim3(gx, (N + 8 * TN - 1) / (8 * TN)), 256, 0, s>>>(X, ldx, W, ldw, transW, Z, ldz, n, K, N, \
-                                                                           epilogue, aux, ldaux, x_vec4)
-  if (per <= 1) CAGNET_GEMM_CASE(1);
-  else if (per <= 2) CAGNET_GEMM_CASE(2);
-  else if (per <= 3) CAGNET_GEMM_CASE(3);
-  else if (per <= 4) CAGNET_GEMM_CASE(4);
-  else if (per <= 6) CAGNET_GEMM_CASE(6);
-  else CAGNET_GEMM_CASE(8);
-#undef CAGNET_GEMM_CASE
-  return check_launch("cagnet_gemm_nn_f32");
+  if (gemm_nn_tc_applies(X, ldx, n, K, N, epilogue)) return gemm_nn_tc(X, ldx, W, ldw, transW, Z, ldz, n, K, N, epilogue, aux, ldaux, s);
+  GemmArgs a;
+  a.X = X; a.W = W; a.aux = aux; a.Z = Z;
+  a.ldx = ldx; a.ldw = ldw; a.ldz = ldz; a.ldaux = ldaux; a.n = n;
+  a.transW = transW; a.K = K; a.N = N; a.epilogue = epilogue;
+  a.x_vec4 = (ldx % 4 == 0 && aligned(X, 16)) ? 1 : 0;
+  a.z_vec4 = (ldz % 4 == 0 && aligned(Z, 16)) ? 1 : 0;
+  // Row tiles are as tall as W is narrow (8 rows per thread); below about two tiles per SM, with a K worth splitting, the
+  // warps of a block share its rows and split K instead.
+  const bool splitk = N <= 64 && K >= 64 && n < 40000 && epilogue != CAGNET_EPI_LOG_SOFTMAX_256;
+  auto rows = [&](int bm) { return dim3(static_cast<unsigned>((n + bm - 1) / bm), 1); };
+  cudaError_t e;
+  if (splitk) {
+    if (N <= 16) e = launch_pdl(gemm_nn_splitk_kernel<4, 2>, rows(16), dim3(256), 0, s, a);
+    else if (N <= 32) e = launch_pdl(gemm_nn_splitk_kernel<8, 4>, rows(16), dim3(256), 0, s, a);
+    else e = launch_pdl(gemm_nn_splitk_kernel<16, 8>, rows(16), dim3(256), 0, s, a);
+  } else if (N <= 16 && n < 20000) {
+    e = launch_pdl(gemm_nn_kernel<4, 1, 2, 4, 32>, rows(64), dim3(128), 0, s, a);
+  } else if (N <= 16 && n < 160000) {
+    e = launch_pdl(gemm_nn_kernel<4, 1, 4, 4, 32>, rows(128), dim3(128), 0, s, a);
+  } else if (N <= 16) {
+    e = launch_pdl(gemm_nn_kernel<4, 1, 8, 4, 16>, rows(256), dim3(128), 0, s, a);
+  } else if (N <= 32 && n < 80000) {
+    e = launch_pdl(gemm_nn_kernel<8, 1, 2, 4, 32>, rows(32), dim3(128), 0, s, a);
+  } else if (N <= 32) {
+    e = launch_pdl(gemm_nn_kernel<8, 1, 8, 4, 32>, rows(128), dim3(128), 0, s, a);
+  } else if (N <= 64) {
+    e = launch_pdl(gemm_nn_kernel<16, 1, 8, 8, 32>, rows(128), dim3(256), 0, s, a);
+  } else if (N <= 128) {
+    e = launch_pdl(gemm_nn_kernel<32, 1, 8, 8, 16>, rows(64), dim3(256), 0, s, a);
+  } else {
+    dim3 grid = rows(64);
+    grid.y = (N + 255) / 256;
+    e = launch_pdl(gemm_nn_kernel<32, 2, 8, 8, 16>, grid, dim3(256), 0, s, a);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(CAGNET_E_LAUNCH, "cagnet_gemm_nn_f32: CUDA launch failed: %s", cudaGetErrorString(e));
+  }
+  return CAGNET_OK;
 }
 
 extern "C" size_t cagnet_gemm_tn_workspace_bytes(int64_t n, int32_t K, int32_t N) {
   if (n < 0 || K <= 0 || N <= 0) return 0;
-  const int chunks = max(tn_shape(n, K, N).chunks, tn_shape(n, N, K).chunks);     // either operand order
+  const int chunks = max(max(tn_shape(n, K, N).chunks, tn_shape(n, N, K).chunks), kNumSMs);     // either operand order, either kernel
   return sizeof(float) * static_cast<size_t>(chunks) * K * N;
 }
 
@@ -696,13 +962,19 @@ extern "C" int cagnet_gemm_tn_f32(const float* H, int64_t ldh, const float* G, i
                 (long long)ws_bytes, (long long)cagnet_gemm_tn_workspace_bytes(n, K, N));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float* partials = static_cast<float*>(ws);
+  if (gemm_tn_tc_applies(H, ldh, G, ldg, n, K, N)) {
+    if (int rc = gemm_tn_tc(H, ldh, G, ldg, n, K, N, partials, s)) return rc;
+    launch_pdl(gemm_tn_reduce_kernel, dim3((K * N + 31) / 32), dim3(256), 0, s, partials, gemm_tn_tc_blocks(n, K, N), max(K, N), min(K, N), out,
+               ldo, beta, K < N ? 1 : 0);
+    return check_launch("cagnet_gemm_tn_f32");
+  }
   const bool rows_aligned = ldh % 4 == 0 && ldg % 4 == 0 && aligned(H, 16) && aligned(G, 16);
   if (N <= 16 && rows_aligned) {
     const TnShape sh = tn_shape(n, K, N);
     if (int rc = tn_small_opt_in()) return rc;
     gemm_tn_small_kernel<<<dim3(sh.chunks, sh.ktiles), 256, kTnSmallSmemBytes, s>>>(H, ldh, G, ldg, n, K, N,
                                                                                    sh.rows_per_chunk, partials);
-    gemm_tn_reduce_kernel<<<(K * N + 7) / 8, 256, 0, s>>>(partials, sh.chunks, K, N, out, ldo, beta, 0);
+    gemm_tn_reduce_kernel<<<(K * N + 31) / 32, 256, 0, s>>>(partials, sh.chunks, K, N, out, ldo, beta, 0);
   } else if (K <= 16 && rows_aligned) {
     // a narrow H against a wider G (the 16 x 41 weight gradient): the same kernel computes G^T * H, the reduce
     // writes it transposed
@@ -710,12 +982,12 @@ extern "C" int cagnet_gemm_tn_f32(const float* H, int64_t ldh, const float* G, i
     if (int rc = tn_small_opt_in()) return rc;
     gemm_tn_small_kernel<<<dim3(sh.chunks, sh.ktiles), 256, kTnSmallSmemBytes, s>>>(G, ldg, H, ldh, n, N, K,
                                                                                    sh.rows_per_chunk, partials);
-    gemm_tn_reduce_kernel<<<(K * N + 7) / 8, 256, 0, s>>>(partials, sh.chunks, N, K, out, ldo, beta, 1);
+    gemm_tn_reduce_kernel<<<(K * N + 31) / 32, 256, 0, s>>>(partials, sh.chunks, N, K, out, ldo, beta, 1);
   } else {
     const TnShape sh = tn_shape(n, K, N);
     gemm_tn_partial_kernel<<<dim3(sh.chunks, sh.ktiles, sh.ntiles), 256, 0, s>>>(H, ldh, G, ldg, n, K, N,
                                                                                 sh.rows_per_chunk, partials);
-    gemm_tn_reduce_kernel<<<(K * N + 7) / 8, 256, 0, s>>>(partials, sh.chunks, K, N, out, ldo, beta, 0);
+    gemm_tn_reduce_kernel<<<(K * N + 31) / 32, 256, 0, s>>>(partials, sh.chunks, K, N, out, ldo, beta, 0);
   }
   return check_launch("cagnet_gemm_tn_f32");
 }
@@ -725,7 +997,8 @@ extern "C" int cagnet_relu_fwd_f32(const float* z, int64_t ldz, float* h, int64_
   if (n < 0 || N < 0) return fail(CAGNET_E_ARG, "cagnet_relu_fwd_f32: negative size");
   if (n == 0 || N == 0) return CAGNET_OK;
   if (!z || !h || ldz < N || ldh < N) return fail(CAGNET_E_ARG, "cagnet_relu_fwd_f32: bad argument");
-  relu_fwd_kernel<<<elementwise_blocks(n * N), 256, 0, static_cast<cudaStream_t>(stream)>>>(z, ldz, h, ldh, n, N);
+  const int vecs = (N + 3) / 4, vec4 = (ldz % 4 == 0 && ldh % 4 == 0 && aligned(z, 16) && aligned(h, 16)) ? 1 : 0;
+  launch_pdl(relu_fwd_kernel, dim3(elementwise_blocks(n * vecs)), dim3(256), 0, static_cast<cudaStream_t>(stream), z, ldz, h, ldh, n, N, vecs, vec4);
   return check_launch("cagnet_relu_fwd_f32");
 }
 
@@ -734,7 +1007,10 @@ extern "C" int cagnet_relu_bwd_f32(const float* h, int64_t ldh, const float* g, 
   if (n < 0 || N < 0) return fail(CAGNET_E_ARG, "cagnet_relu_bwd_f32: negative size");
   if (n == 0 || N == 0) return CAGNET_OK;
   if (!h || !g || !dz || ldh < N || ldg < N || lddz < N) return fail(CAGNET_E_ARG, "cagnet_relu_bwd_f32: bad argument");
-  relu_bwd_kernel<<<elementwise_blocks(n * N), 256, 0, static_cast<cudaStream_t>(stream)>>>(h, ldh, g, ldg, dz, lddz, n, N);
+  const int vecs = (N + 3) / 4;
+  const int vec4 = (ldh % 4 == 0 && ldg % 4 == 0 && lddz % 4 == 0 && aligned(h, 16) && aligned(g, 16) && aligned(dz, 16)) ? 1 : 0;
+  launch_pdl(relu_bwd_kernel, dim3(elementwise_blocks(n * vecs)), dim3(256), 0, static_cast<cudaStream_t>(stream), h, ldh, g, ldg, dz, lddz, n, N,
+             vecs, vec4);
   return check_launch("cagnet_relu_bwd_f32");
 }
 
@@ -744,8 +1020,16 @@ extern "C" int cagnet_log_softmax_fwd_f32(const float* z, int64_t ldz, float* lo
   if (n == 0 || N == 0) return CAGNET_OK;
   if (!z || !logp || ldz < N || ldl < N) return fail(CAGNET_E_ARG, "cagnet_log_softmax_fwd_f32: bad argument");
   if ((n + 7) / 8 > INT_MAX) return fail(CAGNET_E_OVERFLOW, "cagnet_log_softmax_fwd_f32: too many rows");
-  log_softmax_fwd_kernel<<<static_cast<unsigned>((n + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(z, ldz, logp,
-                                                                                                          ldl, n, N);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int vec4 = (ldz % 4 == 0 && ldl % 4 == 0 && aligned(z, 16) && aligned(logp, 16)) ? 1 : 0;
+  const int vecs = (N + 3) / 4;
+  auto rows = [&](int lanes) { return dim3(static_cast<unsigned>((n + 256 / lanes - 1) / (256 / lanes))); };
+  if (vecs <= 4) launch_pdl(log_softmax_fwd_kernel<4, 1>, rows(4), dim3(256), 0, s, z, ldz, logp, ldl, n, N, vec4);
+  else if (vecs <= 8) launch_pdl(log_softmax_fwd_kernel<8, 1>, rows(8), dim3(256), 0, s, z, ldz, logp, ldl, n, N, vec4);
+  else if (vecs <= 16) launch_pdl(log_softmax_fwd_kernel<8, 2>, rows(8), dim3(256), 0, s, z, ldz, logp, ldl, n, N, vec4);
+  else if (vecs <= 32) launch_pdl(log_softmax_fwd_kernel<16, 2>, rows(16), dim3(256), 0, s, z, ldz, logp, ldl, n, N, vec4);
+  else if (vecs <= 64) launch_pdl(log_softmax_fwd_kernel<32, 2>, rows(32), dim3(256), 0, s, z, ldz, logp, ldl, n, N, vec4);
+  else launch_pdl(log_softmax_fwd_wide_kernel, rows(32), dim3(256), 0, s, z, ldz, logp, ldl, n, N);
   return check_launch("cagnet_log_softmax_fwd_f32");
 }
 

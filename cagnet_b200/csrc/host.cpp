@@ -178,7 +178,7 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
   auto dense_layer = [&](const float* X, int64_t ld, const at::Tensor& W, const Buffer& Z, int32_t K, int32_t N, bool last) {
     if (!activations) return gemm(X, ld, W, false, Z, K, N, CAGNET_EPI_NONE, nullptr, 0);
     if (!last) return gemm(X, ld, W, false, Z, K, N, CAGNET_EPI_RELU, nullptr, 0);
-    if (N <= 64) return gemm(X, ld, W, false, Z, K, N, CAGNET_EPI_LOG_SOFTMAX, nullptr, 0);
+    if (N <= 256) return gemm(X, ld, W, false, Z, K, N, N <= 64 ? CAGNET_EPI_LOG_SOFTMAX : CAGNET_EPI_LOG_SOFTMAX_256, nullptr, 0);
     gemm(X, ld, W, false, Z, K, N, CAGNET_EPI_NONE, nullptr, 0);
     check(cagnet_log_softmax_fwd_f32(Z.p(), Z.ld, Z.p(), Z.ld, n, N, s), "log_softmax");
     ++launches;

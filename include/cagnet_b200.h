@@ -36,7 +36,8 @@ enum {
   CAGNET_EPI_RELU = 1,         /* out = max(acc, 0)                         F.relu,        gcn_distr.py:287-288 */
   CAGNET_EPI_LOG_SOFTMAX = 2,  /* out = log_softmax(acc) per row (N <= 64)  F.log_softmax, gcn_distr.py:285-286 */
   CAGNET_EPI_RELU_MASK = 3,    /* out = aux > 0 ? acc : 0  (ReLU backward;  replaces autograd.grad at gcn_distr.py:312-322) */
-  CAGNET_EPI_ACCUMULATE = 4    /* out += acc               (`z_loc += torch.mm(acol, brow)`, gcn_distr_2d.py:507) */
+  CAGNET_EPI_ACCUMULATE = 4,   /* out += acc               (`z_loc += torch.mm(acol, brow)`, gcn_distr_2d.py:507) */
+  CAGNET_EPI_LOG_SOFTMAX_256 = 5  /* CAGNET_EPI_LOG_SOFTMAX for N <= 256 */
 };
 
 int cagnet_version(void);
@@ -192,7 +193,7 @@ int cagnet_spmm_coo_f32(const int32_t* rows, const int32_t* cols, const float* v
  *                           cta_ptr[i]: first tile of thread block i's share (every share holds at least one tile);
  *                           join_list: (panel, first block, last block + 1, 0) of each panel that several blocks share.
  *                           Three bf16 terms per element of B, fp32 sums in a fixed order.
- * cagnet_tile_core_error: 1 if a multiply on the current device gave up on a wait since the library was loaded
+ * cagnet_tile_core_error: 1 if a tensor-core kernel on the current device gave up on a wait since the library was loaded
  * (synchronises the device).  No counterpart in the reference. */
 int cagnet_tile_count_i32(const int32_t* rowptr, const int32_t* col, int32_t n, const int32_t* rank_r,
                           const int32_t* rank_c, int32_t lim_r, int32_t lim_c, int32_t* counts, void* stream);

@@ -113,3 +113,44 @@ def test_fused_loss_and_adam(n, N, lo, hi):
     for t, p in zip(w, ref):
         _close(t, p.detach().cpu())
     assert abs(float(loss) - float(want)) <= 1e-5 * max(abs(float(want)), 1e-6)
+
+
+@pytest.mark.parametrize("n,K,N", [(9472, 304, 16), (9601, 350, 41), (20001, 130, 100), (40003, 16, 256), (40003, 64, 80), (70000, 602, 10),
+                                   (33000, 33, 65), (19000, 64, 200), (30011, 96, 8)])
+def test_tensor_core_products(n, K, N):
+    """X.W and H^T.G at sizes that the tcgen05 kernels take, tile remainders in every direction, against fp64: as close as
+    fp32 multiply-adds come (one bf16 term would be 2e-3 off, two 1e-5), bit-reproducible, pad columns never read or written."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    X, W = torch.randn(n, K, generator=g, device="cuda"), torch.randn(K, N, generator=g, device="cuda")
+    aux, Z0 = torch.randn(n, N, generator=g, device="cuda"), torch.randn(n, N, generator=g, device="cuda")
+    Xd = ops.to_padded(X)
+    if Xd.stride(0) > K:
+        ops.base_buffer(Xd).view(-1, Xd.stride(0))[:, K:] = float("nan")
+    want = X.double() @ W.double()
+
+    def close(got, ref):
+        assert float((got.double() - ref).norm()) <= 1e-6 * float(ref.norm())
+    for trans, w in ((False, W), (True, W.t().contiguous())):
+        Z = ops.gemm_nn(Xd, w, trans)
+        close(Z, want)
+        assert torch.equal(Z, ops.gemm_nn(Xd, w, trans))
+    close(ops.gemm_nn(Xd, W, False, ops.EPI_RELU), torch.relu(want))
+    close(ops.gemm_nn(Xd, W, False, ops.EPI_RELU_MASK, aux=ops.to_padded(aux)), want * (aux > 0))
+    close(ops.gemm_nn(Xd, W, False, ops.EPI_ACCUMULATE, out=ops.to_padded(Z0)), want + Z0.double())
+    wide = torch.full((n, N + 5), 7.0, device="cuda")
+    ops.gemm_nn(Xd, W, False, ops.EPI_NONE, out=wide[:, 1:N + 1])          # rows of Z not 16-byte aligned
+    close(wide[:, 1:N + 1], want)
+    assert bool((wide[:, 0] == 7.0).all()) and bool((wide[:, N + 1:] == 7.0).all())
+    if N <= 64 or N <= 256 and K <= 64:
+        out = ops.empty_padded(n, N, "cuda")
+        epi = ops.EPI_LOG_SOFTMAX if N <= 64 else 5
+        _native.check(_native.lib().cagnet_gemm_nn_f32(Xd.data_ptr(), Xd.stride(0), W.data_ptr(), N, 0, out.data_ptr(), out.stride(0), n, K,
+                                                       N, epi, None, 0, None))
+        close(out, torch.log_softmax(want, dim=1))
+    Gd = ops.to_padded(Z0)
+    if Gd.stride(0) > N:
+        ops.base_buffer(Gd).view(-1, Gd.stride(0))[:, N:] = float("nan")
+    grad = ops.gemm_tn(Xd, Gd)
+    close(grad, X.double().t() @ Z0.double())
+    assert torch.equal(grad, ops.gemm_tn(Xd, Gd))
+    assert _native.lib().cagnet_tile_core_error() == 0
