@@ -21,7 +21,7 @@
 
 namespace cagnet {
 
-constexpr int kUnit = 32;               // granularity of the row bookkeeping, nonzeros
+constexpr int kUnit = 8;                // granularity of the row bookkeeping, nonzeros
 constexpr int kSplitWarps = 4;          // warps per block
 constexpr unsigned kMid = 0x80000000u;  // first[]: the unit starts inside a row
 
@@ -79,6 +79,12 @@ __device__ __forceinline__ void piece_store(float* p, const float (&acc)[NV][4])
     *reinterpret_cast<float4*>(p + w * (LPN * 4)) = make_float4(acc[w][0], acc[w][1], acc[w][2], acc[w][3]);
 }
 
+// Blocks of the walk kernel that an SM holds: what the registers of a variant allow (the compiler is held to it), and the
+// size of a wave in the choice of the chunk length.
+__host__ __device__ constexpr int split_blocks_per_sm(int nv, bool coo) {
+  return nv == 4 ? 4 : nv == 3 ? 5 : coo ? 6 : 7;
+}
+
 // Row a chunk starts in, and whether it began in an earlier chunk: from the plan, or from the COO rows themselves.
 template <bool COO>
 __device__ __forceinline__ unsigned chunk_row(const SplitArgs& a, int c, bool& mid) {
@@ -95,12 +101,12 @@ __device__ __forceinline__ unsigned chunk_row(const SplitArgs& a, int c, bool& m
 }
 
 template <int LPN, int NV, int BATCH, bool ADD, bool COO>
-__global__ void __launch_bounds__(kSplitWarps * 32) spmm_split_kernel(SplitArgs a) {
+__global__ void __launch_bounds__(kSplitWarps * 32, split_blocks_per_sm(NV, COO)) spmm_split_kernel(SplitArgs a) {
   constexpr int G = 32 / LPN;
   constexpr int PL = (2 * LPN >= BATCH) ? 1 : BATCH / (2 * LPN);   // 16-byte loads (2 pairs) per lane and stage
   constexpr int SL = 2 * LPN * PL;                                 // pairs per lane group and stage
   constexpr int TILE = LPN * 4 * NV;
-  static_assert(SL <= kUnit && SL % BATCH == 0, "a stage lies inside a unit");
+  static_assert(SL % kUnit == 0 && SL % BATCH == 0, "stages and chunks are whole units and batches");
   __shared__ __align__(16) int2 stage_s[kSplitWarps][G][SL];
   __shared__ __align__(8) int stage_rows_s[COO ? kSplitWarps : 1][COO ? G : 1][COO ? SL : 1];
   pdl_trigger();
@@ -331,34 +337,54 @@ struct SplitShape {
   int64_t nchunks;
 };
 
-// Lane mapping by width (vectors of 4 columns per gathered row), measured on R-MAT graphs of 0.1 - 115 M nonzeros:
-// one group per row segment as narrow as the row allows (more nonzeros in flight per warp), two or three vectors per
-// lane from 9 vectors on (fewer broadcasts per byte: width 41 0.67 -> 0.58 ms, width 128 with 16 x 2 lanes 1.18 ms against
-// 1.42 with 32 x 1) unless the matrix is so small that it cannot fill the chip (below 1 M nonzeros one vector per lane
-// gives twice the warps: width 48, 100 K nonzeros 9.2 against 10.2 us).
-// Chunk length: about 26,000 chunk walks per launch (6 resident groups per lane group slot), in [32, 512]; shorter
-// chunks start more walks than they fill, longer ones leave a ragged last wave.  Doubled where the pieces would need more
-// than half a gigabyte.
-static SplitShape split_shape(int64_t nnz, int f) {
+// Lane mapping by width (vectors of 4 columns per gathered row), measured on R-MAT graphs of 0.03 - 115 M nonzeros.
+// Narrow rows: one vector per lane, as few lanes as the row has vectors (more nonzeros in flight per warp).  From 9 vectors
+// on, 8 lanes with 2 to 4 vectors each: every lane has that many independent loads per nonzero, and a nonzero's pair, row
+// end test and broadcast are paid once for all of them (22.6 M nonzeros, width 602: 16 lanes x 2 4.7 ms, 8 x 3 4.36;
+// width 128: 16 x 2 0.87 ms, 8 x 4 0.84; width 300: 16 x 2 2.47 ms, 8 x 3 2.31).  Which of them: the one that covers
+// the width with the least padding, weighed by its time per vector (two vectors 8 % above three, four 6 %).  Two-vector
+// tiles are kept out of large multiplies (width 256: 8 x 2 2.20 ms, 8 x 4 1.73: 256-byte pieces of rows that do not stay
+// in L2) and four-vector ones out of small ones, which they cannot spread over the chip (0.6 M nonzeros, width 128:
+// 33.9 us with 2, 38.8 with 4).  The smallest take one vector per lane for the same reason (0.1 M nonzeros, width 64:
+// 11.8 us with 1, 13.7 with 2).  COO operands, whose row indices take registers and a second stage, stay with two (4 M
+// nonzeros, width 128: 158 us with 2, 230 with 4).
+//
+// Chunk length: the launch is a whole number of full waves, a wave being what the SMs hold.  All chunks take about as long,
+// so a wave that is filled to its last block ends together and one block more costs a whole wave (22.6 M nonzeros, width
+// 16: chunks of 512 end in a wave of 6 % at 216 us; chunks of 704, one wave, 174 us; of 600 on seven blocks per SM 162).
+// Chunks stay under 704 nonzeros (more waves beyond) and not under 32 (0.5 M nonzeros, width 16: 15.4 us with 16, 12.5 with
+// 32, 13.9 with 48), and are longer only where the pieces would need more than half a gigabyte.
+static SplitShape split_shape(int64_t nnz, int f, bool coo) {
+  constexpr int kLongest = 704, kShortest = 32;
   SplitShape s;
   const int v = (f + 3) / 4;
-  if (v <= 4) s.lpn = 4, s.nv = 1;
-  else if (v <= 8) s.lpn = 8, s.nv = 1;
-  else if (v <= 16 && nnz < (1 << 20)) s.lpn = 16, s.nv = 1;
-  else if (v <= 16) s.lpn = 8, s.nv = 2;
-  else if (v <= 24) s.lpn = 8, s.nv = 3;
-  else s.lpn = 16, s.nv = 2;
+  s.lpn = v <= 4 ? 4 : 8;
+  s.nv = 1;
+  if (v > 8 && nnz >= (v <= 16 ? 500000 : 150000)) {
+    const int few = coo || v <= 16 || nnz < 2000000 ? 2 : 3, many = coo ? 2 : nnz < 2000000 ? 3 : 4;
+    constexpr int weight[5] = {0, 0, 108, 100, 106};
+    for (int nv = few, best = INT_MAX; nv <= many; ++nv) {
+      const int cost = (v + 8 * nv - 1) / (8 * nv) * nv * weight[nv];
+      if (cost < best) best = cost, s.nv = nv;
+    }
+  }
   const int tile = s.lpn * s.nv;
   s.tiles = (v + tile - 1) / tile;
-  s.chunk = kUnit;
-  while (s.chunk < 512 && nnz * s.tiles > static_cast<int64_t>(s.chunk) * 37000) s.chunk *= 2;
-  while (((nnz + s.chunk - 1) / s.chunk) * s.tiles * tile * 32 > (512ll << 20)) s.chunk *= 2;
-  s.nchunks = (nnz + s.chunk - 1) / s.chunk;
+  const int unit = 2 * s.lpn, per_block = kSplitWarps * (32 / s.lpn);
+  const int64_t slots = static_cast<int64_t>(kNumSMs) * split_blocks_per_sm(s.nv, coo);        // blocks of a wave
+  int64_t waves = (nnz * s.tiles + slots * per_block * kLongest - 1) / (slots * per_block * kLongest);
+  while (waves * slots < s.tiles) ++waves;
+  const int64_t walks = waves * slots / s.tiles * per_block;                                    // chunks of a feature tile
+  int64_t chunk = (nnz + walks - 1) / walks;
+  chunk = ((chunk < kShortest ? kShortest : chunk) + unit - 1) / unit * unit;
+  while ((nnz + chunk - 1) / chunk * s.tiles * tile * 32 > (512ll << 20)) chunk *= 2;
+  s.chunk = static_cast<int>(chunk);
+  s.nchunks = (nnz + chunk - 1) / chunk;
   return s;
 }
 
-static size_t split_bytes(int64_t nnz, int f) {
-  const SplitShape s = split_shape(nnz, f);
+static size_t split_bytes(int64_t nnz, int f, bool coo) {
+  const SplitShape s = split_shape(nnz, f, coo);
   return static_cast<size_t>(s.nchunks) * s.tiles * s.lpn * s.nv * 32;     // two pieces of 16-byte vectors
 }
 
@@ -391,16 +417,17 @@ static int launch_split(const SplitArgs& a, int tiles, float beta, cudaStream_t 
 template <bool COO>
 static int dispatch_split(const SplitArgs& a, const SplitShape& sh, float beta, cudaStream_t stream) {
   if (sh.lpn == 4) return launch_split<COO, 4, 1, 8>(a, sh.tiles, beta, stream);
-  if (sh.lpn == 8 && sh.nv == 1) return launch_split<COO, 8, 1, 8>(a, sh.tiles, beta, stream);
-  if (sh.lpn == 8 && sh.nv == 2) return launch_split<COO, 8, 2, 4>(a, sh.tiles, beta, stream);
-  if (sh.lpn == 8) return launch_split<COO, 8, 3, 4>(a, sh.tiles, beta, stream);
-  if (sh.nv == 1) return launch_split<COO, 16, 1, 4>(a, sh.tiles, beta, stream);
-  return launch_split<COO, 16, 2, 4>(a, sh.tiles, beta, stream);
+  if (sh.nv == 1) return launch_split<COO, 8, 1, 8>(a, sh.tiles, beta, stream);
+  if (COO || sh.nv == 2) return launch_split<COO, 8, 2, 4>(a, sh.tiles, beta, stream);
+  if constexpr (!COO) {
+    if (sh.nv == 3) return launch_split<false, 8, 3, 4>(a, sh.tiles, beta, stream);
+    return launch_split<false, 8, 4, 4>(a, sh.tiles, beta, stream);
+  }
 }
 
 static int run_split(const cagnet_block* b, const float* B, int64_t ldb, float* C, int64_t ldc, int f, float beta, void* ws,
                      cudaStream_t stream) {
-  const SplitShape sh = split_shape(b->nnz, f);
+  const SplitShape sh = split_shape(b->nnz, f, false);
   SplitArgs a = {};
   const int64_t padded = (b->nnz + kUnit - 1) / kUnit * kUnit;
   a.pairs = static_cast<const int2*>(b->split);
@@ -489,7 +516,7 @@ extern "C" size_t cagnet_spmm_block_workspace_bytes(const cagnet_block* b, const
   const cagnet_block* src = tiles ? b->rest : b;
   size_t bytes = tiles ? round256(cagnet_tile_core_workspace_bytes(b->tile_kbs, b->ctas, f)) : 0;
   if (use_split(src) && (b_aligned(B, ldb) || pad_pays(src))) {
-    bytes += round256(split_bytes(src->nnz, f));
+    bytes += round256(split_bytes(src->nnz, f, false));
     if (!b_aligned(B, ldb)) bytes += round256(static_cast<size_t>(b->m) * ((f + 3) / 4) * 16);
   }
   return bytes;
@@ -517,7 +544,7 @@ extern "C" int cagnet_spmm_block_f32(const cagnet_block* b, const float* B, int6
     B = pad_rows(B, ldb, b->m, f, w, s);
     const int rc = run_split(src, B, ldb, C, ldc, f, beta, w, s);
     if (rc != CAGNET_OK) return rc;
-    ws = w + round256(split_bytes(src->nnz, f));
+    ws = w + round256(split_bytes(src->nnz, f, false));
   }
   if (!tiles) return check_launch("cagnet_spmm_block_f32");
   return cagnet_tile_core_f32(b->tile_bits, b->tile_kb, b->panel_ptr, b->cta_ptr, b->ctas, b->panels, b->join_list, b->joins,
@@ -527,7 +554,7 @@ extern "C" int cagnet_spmm_block_f32(const cagnet_block* b, const float* B, int6
 
 extern "C" size_t cagnet_spmm_coo_workspace_bytes(int32_t m, int64_t nnz, const float* B, int64_t ldb, int32_t f) {
   if (nnz <= 0 || f <= 0) return 0;
-  return round256(split_bytes(nnz, f)) + (b_aligned(B, ldb) ? 0 : round256(static_cast<size_t>(m) * ((f + 3) / 4) * 16));
+  return round256(split_bytes(nnz, f, true)) + (b_aligned(B, ldb) ? 0 : round256(static_cast<size_t>(m) * ((f + 3) / 4) * 16));
 }
 
 extern "C" int cagnet_spmm_coo_f32(const int32_t* rows, const int32_t* cols, const float* vals, int32_t n, int32_t m, int64_t nnz,
@@ -542,7 +569,7 @@ extern "C" int cagnet_spmm_coo_f32(const int32_t* rows, const int32_t* cols, con
   char* w = static_cast<char*>(ws);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   B = pad_rows(B, ldb, m, f, w, s);
-  const SplitShape sh = split_shape(nnz, f);
+  const SplitShape sh = split_shape(nnz, f, true);
   SplitArgs a = {};
   a.coo_rows = rows; a.coo_cols = cols; a.coo_vals = vals; a.status = status;
   a.nrows = n;                 // no chunk starts in row n

@@ -44,6 +44,29 @@ def test_split_multiply(f, lens):
     assert bool((wide[:, 0] == 7.0).all()) and bool((wide[:, f + 1:] == 7.0).all())
 
 
+@pytest.mark.parametrize("nnz", [149999, 500000, 2000001])              # sizes at which the lane mapping changes
+def test_split_multiply_lane_mappings(nnz):
+    n, m = 3001, 5003
+    g = torch.Generator(device="cuda").manual_seed(nnz)
+    keys = torch.randperm(n * m, generator=g, device="cuda")[:nnz].sort()[0]
+    rows, cols = keys // m, keys % m
+    rows[:20000] = 0                                                       # one row of many chunks
+    vals = torch.rand(nnz, generator=g, device="cuda")
+    A = ops.CsrBlock.from_coo(rows, cols, vals, n, m)
+    M = torch.sparse_coo_tensor(torch.stack([rows, cols]), vals.double(), (n, m))
+    for f in (36, 64, 68, 96, 128, 132, 256, 600):
+        B, C0 = torch.randn(m, f, generator=g, device="cuda"), torch.randn(n, f, generator=g, device="cuda")
+        want = torch.sparse.mm(M, B.double())
+        Bd, C = ops.to_padded(B), ops.to_padded(C0)
+        ops.spmm(A, Bd, C, 1.0)
+        _close(C, (want + C0.double()).cpu())
+        ops.spmm(A, Bd, C, 0.0)
+        _close(C, want.cpu())
+        out = C0.clone()
+        ops.spmm_gpu(rows.int(), cols.int(), vals, n, m, B, out)
+        _close(out, (want + C0.double()).cpu())
+
+
 @pytest.mark.parametrize("n,nnz,parts", [(700, 60000, 1), (4099, 600000, 1), (9001, 1500000, 3)])
 def test_bit_tiles(n, nnz, parts):
     if not ops.integer_core_available():
