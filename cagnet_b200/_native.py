@@ -27,7 +27,7 @@ PROTOTYPES = {
     "cagnet_spmm_split_plan_bytes": (_sz, [_i64]),
     "cagnet_spmm_split_plan_i32": (_i32, [_vp, _vp, _vp, _vp, _i32, _i64, _vp, _sz, _vp]),
     "cagnet_spmm_block_workspace_bytes": (_sz, [_vp, _vp, _i64, _i32]),
-    "cagnet_spmm_block_launches": (_i32, [_vp, _i32]),
+    "cagnet_spmm_block_launches": (_i32, [_vp, _i64, _i32]),
     "cagnet_spmm_block_f32": (_i32, [_vp, _vp, _i64, _vp, _i64, _i32, _f32, _vp, _sz, _vp]),
     "cagnet_check_coo_i32": (_i32, [_vp, _vp, _i32, _i32, _i64, _vp, _vp]),
     "cagnet_spmm_coo_workspace_bytes": (_sz, [_i32, _i64, _vp, _i64, _i32]),

@@ -73,7 +73,6 @@ int spmm_rows_f32(const int32_t* rowptr, const int32_t* col, const float* val, i
                   const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f, float beta, const void* plan,
                   int32_t hub_rows, void* stream);
 int spmm_forced_tile();      // "spmm_tile" when a sweep has set it: such multiplies run the row kernels
-int split_launches(const cagnet_block* b, int32_t f);
 
 // X . W on the tensor cores (dense_tc.cu), where it applies
 bool gemm_nn_tc_applies(const float* X, int64_t ldx, int64_t n, int K, int N, int epilogue);

@@ -66,7 +66,7 @@ int64_t multiply(const cagnet_block* b, const float* B, int64_t ldb, float* C, i
   at::Tensor ws;
   if (bytes) ws = bytes_buffer(o, bytes);
   check(cagnet_spmm_block_f32(b, B, ldb, C, ldc, f, beta, bytes ? ws.data_ptr() : nullptr, bytes, stream), "spmm");
-  return cagnet_spmm_block_launches(b, f);
+  return cagnet_spmm_block_launches(b, ldb, f);
 }
 
 int64_t spmm(uintptr_t block, int64_t device, const at::Tensor& B, const at::Tensor& C, double beta) {

@@ -345,7 +345,8 @@ struct SplitShape {
 // the width with the least padding, weighed by its time per vector (two vectors 8 % above three, four 6 %).  Two-vector
 // tiles are kept out of large multiplies (width 256: 8 x 2 2.20 ms, 8 x 4 1.73: 256-byte pieces of rows that do not stay
 // in L2) and four-vector ones out of small ones, which they cannot spread over the chip (0.6 M nonzeros, width 128:
-// 33.9 us with 2, 38.8 with 4).  The smallest take one vector per lane for the same reason (0.1 M nonzeros, width 64:
+// 33.9 us with 2, 38.8 with 4), unless their rows are even (0.75 M nonzeros in rows of 125, width 200: 45.4 us with 2, 38.9
+// with 4).  The smallest take one vector per lane for the same reason (0.1 M nonzeros, width 64:
 // 11.8 us with 1, 13.7 with 2).  COO operands, whose row indices take registers and a second stage, stay with two (4 M
 // nonzeros, width 128: 158 us with 2, 230 with 4).
 //
@@ -353,15 +354,18 @@ struct SplitShape {
 // so a wave that is filled to its last block ends together and one block more costs a whole wave (22.6 M nonzeros, width
 // 16: chunks of 512 end in a wave of 6 % at 216 us; chunks of 704, one wave, 174 us; of 600 on seven blocks per SM 162).
 // Chunks stay under 704 nonzeros (more waves beyond) and not under 32 (0.5 M nonzeros, width 16: 15.4 us with 16, 12.5 with
-// 32, 13.9 with 48), and are longer only where the pieces would need more than half a gigabyte.
-static SplitShape split_shape(int64_t nnz, int f, bool coo) {
+// 32, 13.9 with 48), and are longer only where the pieces would need more than half a gigabyte.  A B beyond L2 takes a wave
+// for every 64 MB, at most one per feature tile: waves go tile by tile, so each gathers from columns that stay in L2 (1 M
+// nonzeros in even rows, B of 200 MB, 4 tiles: one wave 224 us, four 170).
+static SplitShape split_shape(int64_t nnz, int m, int f, bool coo, bool even) {
   constexpr int kLongest = 704, kShortest = 32;
   SplitShape s;
   const int v = (f + 3) / 4;
   s.lpn = v <= 4 ? 4 : 8;
   s.nv = 1;
   if (v > 8 && nnz >= (v <= 16 ? 500000 : 150000)) {
-    const int few = coo || v <= 16 || nnz < 2000000 ? 2 : 3, many = coo ? 2 : nnz < 2000000 ? 3 : 4;
+    const bool wide = even || nnz >= 2000000;
+    const int few = coo || v <= 16 || !wide ? 2 : 3, many = coo ? 2 : wide ? 4 : 3;
     constexpr int weight[5] = {0, 0, 108, 100, 106};
     for (int nv = few, best = INT_MAX; nv <= many; ++nv) {
       const int cost = (v + 8 * nv - 1) / (8 * nv) * nv * weight[nv];
@@ -373,6 +377,8 @@ static SplitShape split_shape(int64_t nnz, int f, bool coo) {
   const int unit = 2 * s.lpn, per_block = kSplitWarps * (32 / s.lpn);
   const int64_t slots = static_cast<int64_t>(kNumSMs) * split_blocks_per_sm(s.nv, coo);        // blocks of a wave
   int64_t waves = (nnz * s.tiles + slots * per_block * kLongest - 1) / (slots * per_block * kLongest);
+  const int64_t parts = (static_cast<int64_t>(m) * f * 4 + (64 << 20) - 1) >> 26;
+  waves = max(waves, min(static_cast<int64_t>(s.tiles), parts));
   while (waves * slots < s.tiles) ++waves;
   const int64_t walks = waves * slots / s.tiles * per_block;                                    // chunks of a feature tile
   int64_t chunk = (nnz + walks - 1) / walks;
@@ -383,8 +389,7 @@ static SplitShape split_shape(int64_t nnz, int f, bool coo) {
   return s;
 }
 
-static size_t split_bytes(int64_t nnz, int f, bool coo) {
-  const SplitShape s = split_shape(nnz, f, coo);
+static size_t split_bytes(const SplitShape& s) {
   return static_cast<size_t>(s.nchunks) * s.tiles * s.lpn * s.nv * 32;     // two pieces of 16-byte vectors
 }
 
@@ -425,9 +430,14 @@ static int dispatch_split(const SplitArgs& a, const SplitShape& sh, float beta, 
   }
 }
 
+// Rows about as long as each other, as far as the host knows.
+static bool even_rows(const cagnet_block* b) { return b->max_row >= 0 && b->max_row * static_cast<int64_t>(b->n) <= 4 * b->nnz; }
+
+static SplitShape block_shape(const cagnet_block* b, int f) { return split_shape(b->nnz, b->m, f, false, even_rows(b)); }
+
 static int run_split(const cagnet_block* b, const float* B, int64_t ldb, float* C, int64_t ldc, int f, float beta, void* ws,
                      cudaStream_t stream) {
-  const SplitShape sh = split_shape(b->nnz, f, false);
+  const SplitShape sh = block_shape(b, f);
   SplitArgs a = {};
   const int64_t padded = (b->nnz + kUnit - 1) / kUnit * kUnit;
   a.pairs = static_cast<const int2*>(b->split);
@@ -445,11 +455,20 @@ static int run_split(const cagnet_block* b, const float* B, int64_t ldb, float* 
   a.c_vec4 = (ldc % 4 == 0 && aligned(C, 16)) ? 1 : 0;
   return dispatch_split<false>(a, sh, beta, stream);
 }
-// The row kernels stay the better choice for small blocks of short rows: one launch instead of two and no pieces (ER,
-// 13.5 K nonzeros, width 16: 3.0 us against 6.5; at 280 K nonzeros the two are level, at power-law rows the split wins
-// from the smallest block on).
-static bool use_split(const cagnet_block* b) {
-  return b->split && b->nnz > 0 && !(b->max_row >= 0 && b->max_row <= 64 && b->nnz <= 150000) && spmm_forced_tile() == 0;
+// The row kernels stay the better choice for small blocks of short rows, one launch instead of two and no pieces (ER, 13.5 K
+// nonzeros, width 16: 3.0 us against 6.5; at 280 K nonzeros the two are level, at widths 17 - 32 from 40 K on), and for
+// even rows of up to 16 columns until the chip is full (0.75 M nonzeros in rows of 125, width 6: 9.3 us against 12.8; 1 M
+// in rows of 20: 16.7 against 18.0; 2 M: 29.0 against 28.2).  So they are for even rows of more than 384 columns in blocks
+// that do not fill the chip many times over, if the rows are long or B's rows do not start on cache lines, which tiles of
+// columns then cut (width 500: 0.75 M nonzeros in rows of 125 82 us against 86; 2 M in rows of 20, ldb 500, 317 against 348,
+// but ldb 512 344 against 307).  At power-law rows the split wins from the smallest block on.
+static bool use_split(const cagnet_block* b, int64_t ldb, int f) {
+  if (!b->split || b->nnz <= 0 || spmm_forced_tile() != 0) return false;
+  if (b->max_row < 0 || b->max_row > 256) return true;
+  if (b->max_row <= 64 && b->nnz <= (f > 16 && f <= 32 ? 40000 : 150000)) return false;
+  if (!even_rows(b)) return true;
+  if (f > 384 && b->nnz <= 3000000) return ldb % 32 == 0 && b->nnz < 64 * static_cast<int64_t>(b->n);
+  return f > 16 || b->nnz > 1500000;
 }
 
 // Dense tiles pay when the nonzeros they take over outweigh their three launches (tile_work: about 80 M gathered floats,
@@ -478,9 +497,9 @@ static const float* pad_rows(const float* B, int64_t& ldb, int m, int f, char*& 
   return out;
 }
 
-int split_launches(const cagnet_block* b, int32_t f) {
-  if (use_tiles(b, f)) return split_launches(b->rest, f) + 2 + (b->joins > 0);
-  if (use_split(b)) return 2;
+static int split_launches(const cagnet_block* b, int64_t ldb, int32_t f) {
+  if (use_tiles(b, f)) return split_launches(b->rest, ldb, f) + 2 + (b->joins > 0);
+  if (use_split(b, ldb, f)) return 2;
   return (b->plan && b->hub_rows != 0) ? 2 : 1;
 }
 
@@ -515,14 +534,16 @@ extern "C" size_t cagnet_spmm_block_workspace_bytes(const cagnet_block* b, const
   const bool tiles = use_tiles(b, f);
   const cagnet_block* src = tiles ? b->rest : b;
   size_t bytes = tiles ? round256(cagnet_tile_core_workspace_bytes(b->tile_kbs, b->ctas, f)) : 0;
-  if (use_split(src) && (b_aligned(B, ldb) || pad_pays(src))) {
-    bytes += round256(split_bytes(src->nnz, f, false));
+  if (use_split(src, ldb, f) && (b_aligned(B, ldb) || pad_pays(src))) {
+    bytes += round256(split_bytes(block_shape(src, f)));
     if (!b_aligned(B, ldb)) bytes += round256(static_cast<size_t>(b->m) * ((f + 3) / 4) * 16);
   }
   return bytes;
 }
 
-extern "C" int cagnet_spmm_block_launches(const cagnet_block* b, int32_t f) { return b ? split_launches(b, f) : 0; }
+extern "C" int cagnet_spmm_block_launches(const cagnet_block* b, int64_t ldb, int32_t f) {
+  return b ? split_launches(b, ldb, f) : 0;
+}
 
 extern "C" int cagnet_spmm_block_f32(const cagnet_block* b, const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f,
                                      float beta, void* ws, size_t ws_bytes, void* stream) {
@@ -531,7 +552,7 @@ extern "C" int cagnet_spmm_block_f32(const cagnet_block* b, const float* B, int6
     return fail(CAGNET_E_WORKSPACE, "cagnet_spmm_block_f32: workspace too small");
   const bool tiles = use_tiles(b, f);
   const cagnet_block* src = tiles ? b->rest : b;
-  if (!use_split(src) || !(b_aligned(B, ldb) || pad_pays(src)) || f <= 0 || b->n <= 0) {
+  if (!use_split(src, ldb, f) || !(b_aligned(B, ldb) || pad_pays(src)) || f <= 0 || b->n <= 0) {
     const int rc = spmm_rows_f32(src->rowptr, src->col, src->val, src->n, src->m, src->nnz, B, ldb, C, ldc, f, beta, src->plan,
                                  src->hub_rows, stream);
     if (rc != CAGNET_OK || !tiles) return rc;
@@ -544,7 +565,7 @@ extern "C" int cagnet_spmm_block_f32(const cagnet_block* b, const float* B, int6
     B = pad_rows(B, ldb, b->m, f, w, s);
     const int rc = run_split(src, B, ldb, C, ldc, f, beta, w, s);
     if (rc != CAGNET_OK) return rc;
-    ws = w + round256(split_bytes(src->nnz, f, false));
+    ws = w + round256(split_bytes(block_shape(src, f)));
   }
   if (!tiles) return check_launch("cagnet_spmm_block_f32");
   return cagnet_tile_core_f32(b->tile_bits, b->tile_kb, b->panel_ptr, b->cta_ptr, b->ctas, b->panels, b->join_list, b->joins,
@@ -554,7 +575,7 @@ extern "C" int cagnet_spmm_block_f32(const cagnet_block* b, const float* B, int6
 
 extern "C" size_t cagnet_spmm_coo_workspace_bytes(int32_t m, int64_t nnz, const float* B, int64_t ldb, int32_t f) {
   if (nnz <= 0 || f <= 0) return 0;
-  return round256(split_bytes(nnz, f, true)) + (b_aligned(B, ldb) ? 0 : round256(static_cast<size_t>(m) * ((f + 3) / 4) * 16));
+  return round256(split_bytes(split_shape(nnz, m, f, true, false))) + (b_aligned(B, ldb) ? 0 : round256(static_cast<size_t>(m) * ((f + 3) / 4) * 16));
 }
 
 extern "C" int cagnet_spmm_coo_f32(const int32_t* rows, const int32_t* cols, const float* vals, int32_t n, int32_t m, int64_t nnz,
@@ -569,7 +590,7 @@ extern "C" int cagnet_spmm_coo_f32(const int32_t* rows, const int32_t* cols, con
   char* w = static_cast<char*>(ws);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   B = pad_rows(B, ldb, m, f, w, s);
-  const SplitShape sh = split_shape(nnz, f, true);
+  const SplitShape sh = split_shape(nnz, m, f, true, false);
   SplitArgs a = {};
   a.coo_rows = rows; a.coo_cols = cols; a.coo_vals = vals; a.status = status;
   a.nrows = n;                 // no chunk starts in row n

@@ -165,7 +165,7 @@ int cagnet_spmm_split_plan_i32(const int32_t* rowptr, const int32_t* col, const 
  * ws: cagnet_spmm_block_workspace_bytes for the same B, ldb and f, 256-byte aligned; contents need not survive between
  * calls, two calls that may overlap on the GPU need one each.  cagnet_spmm_block_launches: kernels one call launches. */
 size_t cagnet_spmm_block_workspace_bytes(const cagnet_block* block, const float* B, int64_t ldb, int32_t f);
-int cagnet_spmm_block_launches(const cagnet_block* block, int32_t f);
+int cagnet_spmm_block_launches(const cagnet_block* block, int64_t ldb, int32_t f);
 int cagnet_spmm_block_f32(const cagnet_block* block, const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f,
                           float beta, void* ws, size_t ws_bytes, void* stream);
 
