@@ -66,10 +66,15 @@ PROTOTYPES = {
                                      _sz, _vp]),
     "cagnet_nll_softmax_bwd_f32": (_i32, [_vp, _i64, _vp, _vp, _i64, _i32, _i32, _i32, _f32, _vp, _i64,
                                           ctypes.POINTER(_i32), _vp, _sz, _vp]),
-    "cagnet_adam2_f32": (_i32, [_vp, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _i64, _f64, _f64, _f64, _f64, _i64, _vp,
-                                _i32, _f32, _vp, _vp]),
+    "cagnet_gemm_tn_partials_f32": (_i32, [_vp, _i64, _vp, _i64, _i64, _i32, _i32, _vp, _sz, _vp, _vp]),
+    "cagnet_epoch_tail_f32": (_i32, [_vp] * 10 + [_f64, _f64, _f64, _f64, _i64, _vp, _i32, _f32, _vp, _vp]),
 }
 
+
+
+class TnSum(ctypes.Structure):
+    """`cagnet_tn_sum` of include/cagnet_b200.h, field for field."""
+    _fields_ = [("partials", _vp), ("chunks", _i32), ("K", _i32), ("N", _i32), ("transposed", _i32)]
 
 
 class Block(ctypes.Structure):

@@ -320,6 +320,8 @@ __global__ void __launch_bounds__(256) gemm_tn_partial_kernel(const float* __res
                                                               float* __restrict__ ws) {
   __shared__ float Hs[kTnRB][kTnKT];
   __shared__ __align__(16) float Gs[kTnRB][kTnNT];
+  pdl_trigger();
+  pdl_wait();
   const int tid = threadIdx.x;
   const int k0 = blockIdx.y * kTnKT, n0 = blockIdx.z * kTnNT;
   const int64_t r_begin = static_cast<int64_t>(blockIdx.x) * rows_per_chunk;
@@ -417,6 +419,8 @@ __global__ void __launch_bounds__(256, 2) gemm_tn_small_kernel(const float* __re
                                                                int K, int N, int64_t rows_per_chunk,
                                                                float* __restrict__ ws) {
   extern __shared__ __align__(16) float tn_smem[];
+  pdl_trigger();
+  pdl_wait();
   const int tid = threadIdx.x;
   const int kq = tid & 15, rs = tid >> 4;
   const int k0 = blockIdx.y * kTnKT;
@@ -510,26 +514,35 @@ __global__ void __launch_bounds__(256, 2) gemm_tn_small_kernel(const float* __re
   }
 }
 
-// out[k, j] (+)= sum over the row chunks of their partial products.  A block takes 32 neighbouring elements: warp w adds chunks
+// Sum over the row chunks of 32 neighbouring elements of their partial products, for the threads of a block: warp w adds chunks
 // w, w + 8, ... of all 32 (whole 128-byte reads), the eight sums are added in warp order -- the same order on every run.
+// The sum of element idx is valid in the first warp.
+__device__ __forceinline__ float tn_sum(const float* __restrict__ ws, int chunks, int total, int idx, float (&red)[8][32]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float s = 0.f;
+  if (idx < total) {
+#pragma unroll 4
+    for (int c = warp; c < chunks; c += 8) s += __ldg(ws + static_cast<int64_t>(c) * total + idx);
+  }
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) s += red[w][lane];
+  }
+  return s;
+}
+
+// out[k, j] (+)= sum of the partial products.
 __global__ void __launch_bounds__(256)
 gemm_tn_reduce_kernel(const float* __restrict__ ws, int chunks, int K, int N, float* __restrict__ out, int64_t ldo,
                       float beta, int transposed) {
   __shared__ float red[8][32];
   pdl_trigger();
   pdl_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int idx = blockIdx.x * 32 + lane;
-  float s = 0.f;
-  if (idx < K * N) {
-#pragma unroll 4
-    for (int c = warp; c < chunks; c += 8) s += __ldg(ws + static_cast<int64_t>(c) * K * N + idx);
-  }
-  red[warp][lane] = s;
-  __syncthreads();
-  if (warp || idx >= K * N) return;
-#pragma unroll
-  for (int w = 1; w < 8; ++w) s += red[w][lane];
+  const int idx = blockIdx.x * 32 + (threadIdx.x & 31);
+  const float s = tn_sum(ws, chunks, K * N, idx, red);
+  if (threadIdx.x >= 32 || idx >= K * N) return;
   // transposed: the partials are those of G^T * H (K and N as passed here); out is (H^T * G)[N x K]
   float* o = transposed ? out + static_cast<int64_t>(idx % N) * ldo + idx / N : out + static_cast<int64_t>(idx / N) * ldo + idx % N;
   *o = (beta != 0.f) ? s + *o : s;
@@ -822,42 +835,54 @@ __global__ void __launch_bounds__(256) nll_softmax_bwd_kernel(const float* __res
   }
 }
 
-// Adam on two parameter tensors in one launch (torch.optim.Adam with its default options: the same operations in the
-// same order), and the epoch's loss from its partial sums: loss = -sum / count.
-struct AdamTensor {
-  float *p, *m, *v;
-  const float* g;
-  int count;
+// The end of an epoch in one launch (4 launches of 2 - 4 us before): the two weight gradients from their partial products, Adam on
+// both weights (torch.optim.Adam with its default options: the same operations in the same order), and the loss from its
+// partial sums, loss = -sum / count.  Blocks of 32 gradient elements, then one block for the loss.
+struct EpochTailTensor {
+  const float* ws;                   // partial products, `chunks` of K x N
+  int chunks, K, N, transposed;      // transposed: of the gradient's transpose
+  float *g, *p, *m, *v;              // gradient; weight and moments (p null: no optimizer step)
 };
-__global__ void __launch_bounds__(256) adam2_kernel(AdamTensor a, AdamTensor b, float beta1, float beta2, float eps, float step_size,
-                                                    float bias2_sqrt, const float* __restrict__ partial, int parts, float count,
-                                                    float* __restrict__ loss) {
+struct EpochTailArgs {
+  EpochTailTensor t[2];
+  float beta1, beta2, eps, step_size, bias2_sqrt;
+  const float* partial;
+  int parts;
+  float count;
+  float* loss;
+};
+__global__ void __launch_bounds__(256) epoch_tail_kernel(EpochTailArgs a) {
+  __shared__ float red[8][32];
   pdl_trigger();
   pdl_wait();
-  const int total = a.count + b.count;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-    const AdamTensor& t = i < a.count ? a : b;
-    const int k = i < a.count ? i : i - a.count;
-    const float g = t.g[k];
+  const int b0 = (a.t[0].K * a.t[0].N + 31) / 32, b1 = (a.t[1].K * a.t[1].N + 31) / 32;
+  const int blk = blockIdx.x;
+  if (blk < b0 + b1) {
+    const EpochTailTensor& t = a.t[blk < b0 ? 0 : 1];
+    const int idx = (blk < b0 ? blk : blk - b0) * 32 + (threadIdx.x & 31);
+    const float g = tn_sum(t.ws, t.chunks, t.K * t.N, idx, red);
+    if (threadIdx.x >= 32 || idx >= t.K * t.N) return;
+    const int k = t.transposed ? idx % t.N * t.K + idx / t.N : idx;
+    t.g[k] = g;
+    if (!t.p) return;
     float m = t.m[k], v = t.v[k];
-    m += (1.f - beta1) * (g - m);
-    v = v * beta2 + (1.f - beta2) * g * g;
+    m += (1.f - a.beta1) * (g - m);
+    v = v * a.beta2 + (1.f - a.beta2) * g * g;
     t.m[k] = m;
     t.v[k] = v;
-    t.p[k] -= step_size * (m / (sqrtf(v) / bias2_sqrt + eps));
+    t.p[k] -= a.step_size * (m / (sqrtf(v) / a.bias2_sqrt + a.eps));
+    return;
   }
-  if (blockIdx.x == 0 && loss) {
-    __shared__ float red[256];
-    float s = 0.f;
-    for (int i = threadIdx.x; i < parts; i += 256) s += partial[i];
-    red[threadIdx.x] = s;
+  __shared__ float sums[256];
+  float s = 0.f;
+  for (int i = threadIdx.x; i < a.parts; i += 256) s += a.partial[i];
+  sums[threadIdx.x] = s;
+  __syncthreads();
+  for (int w = 128; w > 0; w >>= 1) {
+    if (threadIdx.x < w) sums[threadIdx.x] += sums[threadIdx.x + w];
     __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-      if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) *loss = -red[0] / count;
   }
+  if (threadIdx.x == 0) *a.loss = -sums[0] / a.count;
 }
 
 static int elementwise_blocks(int64_t total) {
@@ -949,47 +974,70 @@ static int tn_small_opt_in() {
   return CAGNET_OK;
 }
 
+// The partial products of H^T * G in ws, and what it takes to add them up.
+static int tn_partials(const float* H, int64_t ldh, const float* G, int64_t ldg, int64_t n, int32_t K, int32_t N, void* ws,
+                       size_t ws_bytes, cagnet_tn_sum* sum, cudaStream_t s) {
+  if (!ws || (n > 0 && (!H || !G))) return fail(CAGNET_E_ARG, "cagnet_gemm_tn_f32: null pointer");
+  if (ldh < K || ldg < N) return fail(CAGNET_E_ALIGN, "cagnet_gemm_tn_f32: leading dimension too small");
+  if (static_cast<int64_t>(K) * N > INT_MAX) return fail(CAGNET_E_OVERFLOW, "cagnet_gemm_tn_f32: K*N exceeds int32");
+  if (ws_bytes < cagnet_gemm_tn_workspace_bytes(n, K, N))
+    return fail(CAGNET_E_WORKSPACE, "cagnet_gemm_tn_f32: workspace of %s%lld bytes is too small (need %lld)", "",
+                (long long)ws_bytes, (long long)cagnet_gemm_tn_workspace_bytes(n, K, N));
+  float* partials = static_cast<float*>(ws);
+  sum->partials = partials;
+  if (gemm_tn_tc_applies(H, ldh, G, ldg, n, K, N)) {
+    sum->chunks = gemm_tn_tc_blocks(n, K, N);
+    sum->K = max(K, N); sum->N = min(K, N);
+    sum->transposed = K < N ? 1 : 0;
+    return gemm_tn_tc(H, ldh, G, ldg, n, K, N, partials, s);
+  }
+  const bool rows_aligned = ldh % 4 == 0 && ldg % 4 == 0 && aligned(H, 16) && aligned(G, 16);
+  // a narrow H against a wider G (the 16 x 41 weight gradient): the small-N kernel computes G^T * H
+  const bool small = (N <= 16 || K <= 16) && rows_aligned, swap = small && N > 16;
+  if (swap) {
+    const float* h = H; H = G; G = h;
+    const int64_t l = ldh; ldh = ldg; ldg = l;
+    const int32_t k = K; K = N; N = k;
+  }
+  const TnShape sh = tn_shape(n, K, N);
+  sum->chunks = sh.chunks;
+  sum->K = K; sum->N = N;
+  sum->transposed = swap ? 1 : 0;
+  cudaError_t e;
+  if (small) {
+    if (int rc = tn_small_opt_in()) return rc;
+    e = launch_pdl(gemm_tn_small_kernel, dim3(sh.chunks, sh.ktiles), dim3(256), kTnSmallSmemBytes, s, H, ldh, G, ldg, n, K, N,
+                   sh.rows_per_chunk, partials);
+  } else {
+    e = launch_pdl(gemm_tn_partial_kernel, dim3(sh.chunks, sh.ktiles, sh.ntiles), dim3(256), 0, s, H, ldh, G, ldg, n, K, N,
+                   sh.rows_per_chunk, partials);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(CAGNET_E_LAUNCH, "cagnet_gemm_tn_f32: CUDA launch failed: %s", cudaGetErrorString(e));
+  }
+  return CAGNET_OK;
+}
+
 extern "C" int cagnet_gemm_tn_f32(const float* H, int64_t ldh, const float* G, int64_t ldg, float* out, int64_t ldo,
                                   int64_t n, int32_t K, int32_t N, float beta, void* ws, size_t ws_bytes, void* stream) {
   if (n < 0 || K < 0 || N < 0) return fail(CAGNET_E_ARG, "cagnet_gemm_tn_f32: negative size");
   if (K == 0 || N == 0) return CAGNET_OK;
   if (beta != 0.f && beta != 1.f) return fail(CAGNET_E_ARG, "cagnet_gemm_tn_f32: beta must be 0 or 1");
-  if (!out || !ws || (n > 0 && (!H || !G))) return fail(CAGNET_E_ARG, "cagnet_gemm_tn_f32: null pointer");
-  if (ldh < K || ldg < N || ldo < N) return fail(CAGNET_E_ALIGN, "cagnet_gemm_tn_f32: leading dimension too small");
-  if (static_cast<int64_t>(K) * N > INT_MAX) return fail(CAGNET_E_OVERFLOW, "cagnet_gemm_tn_f32: K*N exceeds int32");
-  if (ws_bytes < cagnet_gemm_tn_workspace_bytes(n, K, N))
-    return fail(CAGNET_E_WORKSPACE, "cagnet_gemm_tn_f32: workspace of %s%lld bytes is too small (need %lld)", "",
-                (long long)ws_bytes, (long long)cagnet_gemm_tn_workspace_bytes(n, K, N));
+  if (!out) return fail(CAGNET_E_ARG, "cagnet_gemm_tn_f32: null pointer");
+  if (ldo < N) return fail(CAGNET_E_ALIGN, "cagnet_gemm_tn_f32: leading dimension too small");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  float* partials = static_cast<float*>(ws);
-  if (gemm_tn_tc_applies(H, ldh, G, ldg, n, K, N)) {
-    if (int rc = gemm_tn_tc(H, ldh, G, ldg, n, K, N, partials, s)) return rc;
-    launch_pdl(gemm_tn_reduce_kernel, dim3((K * N + 31) / 32), dim3(256), 0, s, partials, gemm_tn_tc_blocks(n, K, N), max(K, N), min(K, N), out,
-               ldo, beta, K < N ? 1 : 0);
-    return check_launch("cagnet_gemm_tn_f32");
-  }
-  const bool rows_aligned = ldh % 4 == 0 && ldg % 4 == 0 && aligned(H, 16) && aligned(G, 16);
-  if (N <= 16 && rows_aligned) {
-    const TnShape sh = tn_shape(n, K, N);
-    if (int rc = tn_small_opt_in()) return rc;
-    gemm_tn_small_kernel<<<dim3(sh.chunks, sh.ktiles), 256, kTnSmallSmemBytes, s>>>(H, ldh, G, ldg, n, K, N,
-                                                                                   sh.rows_per_chunk, partials);
-    gemm_tn_reduce_kernel<<<(K * N + 31) / 32, 256, 0, s>>>(partials, sh.chunks, K, N, out, ldo, beta, 0);
-  } else if (K <= 16 && rows_aligned) {
-    // a narrow H against a wider G (the 16 x 41 weight gradient): the same kernel computes G^T * H, the reduce
-    // writes it transposed
-    const TnShape sh = tn_shape(n, N, K);
-    if (int rc = tn_small_opt_in()) return rc;
-    gemm_tn_small_kernel<<<dim3(sh.chunks, sh.ktiles), 256, kTnSmallSmemBytes, s>>>(G, ldg, H, ldh, n, N, K,
-                                                                                   sh.rows_per_chunk, partials);
-    gemm_tn_reduce_kernel<<<(K * N + 31) / 32, 256, 0, s>>>(partials, sh.chunks, N, K, out, ldo, beta, 1);
-  } else {
-    const TnShape sh = tn_shape(n, K, N);
-    gemm_tn_partial_kernel<<<dim3(sh.chunks, sh.ktiles, sh.ntiles), 256, 0, s>>>(H, ldh, G, ldg, n, K, N,
-                                                                                sh.rows_per_chunk, partials);
-    gemm_tn_reduce_kernel<<<(K * N + 31) / 32, 256, 0, s>>>(partials, sh.chunks, K, N, out, ldo, beta, 0);
-  }
+  cagnet_tn_sum sum;
+  if (int rc = tn_partials(H, ldh, G, ldg, n, K, N, ws, ws_bytes, &sum, s)) return rc;
+  launch_pdl(gemm_tn_reduce_kernel, dim3((K * N + 31) / 32), dim3(256), 0, s, sum.partials, sum.chunks, sum.K, sum.N, out, ldo, beta,
+             sum.transposed);
   return check_launch("cagnet_gemm_tn_f32");
+}
+
+extern "C" int cagnet_gemm_tn_partials_f32(const float* H, int64_t ldh, const float* G, int64_t ldg, int64_t n, int32_t K, int32_t N,
+                                           void* ws, size_t ws_bytes, cagnet_tn_sum* sum, void* stream) {
+  if (n < 0 || K <= 0 || N <= 0 || !sum) return fail(CAGNET_E_ARG, "cagnet_gemm_tn_partials_f32: bad argument");
+  return tn_partials(H, ldh, G, ldg, n, K, N, ws, ws_bytes, sum, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int cagnet_relu_fwd_f32(const float* z, int64_t ldz, float* h, int64_t ldh, int64_t n, int32_t N,
@@ -1125,18 +1173,20 @@ extern "C" int cagnet_nll_softmax_bwd_f32(const float* logp, int64_t ldl, const 
   return check_launch("cagnet_nll_softmax_bwd_f32");
 }
 
-extern "C" int cagnet_adam2_f32(float* p1, float* m1, float* v1, const float* g1, int64_t n1, float* p2, float* m2, float* v2,
-                                const float* g2, int64_t n2, double lr, double beta1, double beta2, double eps, int64_t step,
-                                const float* loss_parts, int32_t parts, float count, float* loss, void* stream) {
-  if (n1 < 0 || n2 < 0 || step < 1 || parts < 0) return fail(CAGNET_E_ARG, "cagnet_adam2_f32: bad size");
-  if ((n1 > 0 && (!p1 || !m1 || !v1 || !g1)) || (n2 > 0 && (!p2 || !m2 || !v2 || !g2)) || (loss && (!loss_parts || !(count > 0.f))))
-    return fail(CAGNET_E_ARG, "cagnet_adam2_f32: bad argument");
-  if (n1 + n2 > INT_MAX) return fail(CAGNET_E_OVERFLOW, "cagnet_adam2_f32: too many parameters");
-  if (n1 + n2 == 0 && !loss) return CAGNET_OK;
+extern "C" int cagnet_epoch_tail_f32(const cagnet_tn_sum* s1, float* g1, float* p1, float* m1, float* v1, const cagnet_tn_sum* s2,
+                                     float* g2, float* p2, float* m2, float* v2, double lr, double beta1, double beta2, double eps,
+                                     int64_t step, const float* loss_parts, int32_t parts, float count, float* loss, void* stream) {
+  if (!s1 || !s2 || !g1 || !g2 || step < 1 || parts < 0 || (loss && (!loss_parts || !(count > 0.f))) ||
+      (p1 && (!m1 || !v1)) || (p2 && (!m2 || !v2)))
+    return fail(CAGNET_E_ARG, "cagnet_epoch_tail_f32: bad argument");
   const double bias1 = 1.0 - pow(beta1, static_cast<double>(step)), bias2 = 1.0 - pow(beta2, static_cast<double>(step));
-  const AdamTensor a{p1, m1, v1, g1, static_cast<int>(n1)}, b{p2, m2, v2, g2, static_cast<int>(n2)};
-  launch_pdl(adam2_kernel, dim3(elementwise_blocks(n1 + n2)), dim3(256), 0, static_cast<cudaStream_t>(stream), a, b,
-             static_cast<float>(beta1), static_cast<float>(beta2), static_cast<float>(eps), static_cast<float>(lr / bias1),
-             static_cast<float>(sqrt(bias2)), loss_parts, parts, count, loss);
-  return check_launch("cagnet_adam2_f32");
+  EpochTailArgs a;
+  a.t[0] = EpochTailTensor{s1->partials, s1->chunks, s1->K, s1->N, s1->transposed, g1, p1, m1, v1};
+  a.t[1] = EpochTailTensor{s2->partials, s2->chunks, s2->K, s2->N, s2->transposed, g2, p2, m2, v2};
+  a.beta1 = static_cast<float>(beta1); a.beta2 = static_cast<float>(beta2); a.eps = static_cast<float>(eps);
+  a.step_size = static_cast<float>(lr / bias1); a.bias2_sqrt = static_cast<float>(sqrt(bias2));
+  a.partial = loss_parts; a.parts = parts; a.count = count; a.loss = loss;
+  const int64_t blocks = (static_cast<int64_t>(s1->K) * s1->N + 31) / 32 + (static_cast<int64_t>(s2->K) * s2->N + 31) / 32 + (loss ? 1 : 0);
+  launch_pdl(epoch_tail_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream), a);
+  return check_launch("cagnet_epoch_tail_f32");
 }

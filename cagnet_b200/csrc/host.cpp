@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <array>
+#include <vector>
 
 #include "../../include/cagnet_b200.h"
 
@@ -47,25 +48,60 @@ int64_t ld_of(const at::Tensor& t, const char* name) {
 
 int64_t pad_ld(int64_t f) { return f <= 64 ? (f + 3) / 4 * 4 : (f + 31) / 32 * 32; }
 
-// Scratch memory and matrices of an epoch: raw storage, rows padded as ops.empty_padded pads them.
-struct Buffer {
-  at::Tensor t;
-  int64_t ld = 0;
-  Buffer() = default;
-  Buffer(const at::TensorOptions& o, int64_t n, int64_t f) : t(at::empty({std::max<int64_t>(n, 1), pad_ld(f)}, o)), ld(pad_ld(f)) {}
-  float* p() const { return t.data_ptr<float>(); }
-};
-
 at::Tensor bytes_buffer(const at::TensorOptions& o, size_t bytes) {
   return at::empty({static_cast<int64_t>((std::max<size_t>(bytes, 16) + 3) / 4)}, o);
 }
 
-int64_t multiply(const cagnet_block* b, const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f, float beta,
-                 const at::TensorOptions& o, void* stream) {
+// Scratch memory of one call: from one allocation of `room` bytes as long as that lasts, which saves a small epoch's host
+// some 20 trips to the allocator, from allocations of their own beyond.  Everything goes back when the call returns.
+class Scratch {
+ public:
+  Scratch(const at::TensorOptions& o, size_t room) : options_(o), left_(room) {
+    if (room) next_ = static_cast<char*>(keep(room));
+  }
+  void* bytes(size_t n, at::Tensor* owner = nullptr) {
+    n = (std::max<size_t>(n, 16) + 511) / 512 * 512;
+    if (n <= left_) {
+      char* p = next_;
+      next_ += n;
+      left_ -= n;
+      return p;
+    }
+    if (!owner) return keep(n);
+    *owner = bytes_buffer(options_, n);        // released with its matrix
+    return owner->data_ptr();
+  }
+
+ private:
+  void* keep(size_t n) {
+    kept_.push_back(bytes_buffer(options_, n));
+    return kept_.back().data_ptr();
+  }
+  at::TensorOptions options_;
+  std::vector<at::Tensor> kept_;
+  char* next_ = nullptr;
+  size_t left_;
+};
+
+// A scratch matrix, rows padded as ops.empty_padded pads them.
+struct Buffer {
+  at::Tensor owner;
+  float* data = nullptr;
+  int64_t ld = 0;
+  Buffer() = default;
+  Buffer(Scratch& s, int64_t n, int64_t f) : ld(pad_ld(f)) {
+    data = static_cast<float*>(s.bytes(static_cast<size_t>(std::max<int64_t>(n, 1)) * ld * 4, &owner));
+  }
+  explicit Buffer(const at::Tensor& t) : owner(t), data(t.data_ptr<float>()), ld(t.stride(0)) {}
+  float* p() const { return data; }
+};
+
+int64_t multiply(const cagnet_block* b, const float* B, int64_t ldb, float* C, int64_t ldc, int32_t f, float beta, Scratch& scratch,
+                 void* stream) {
   const size_t bytes = cagnet_spmm_block_workspace_bytes(b, B, ldb, f);
-  at::Tensor ws;
-  if (bytes) ws = bytes_buffer(o, bytes);
-  check(cagnet_spmm_block_f32(b, B, ldb, C, ldc, f, beta, bytes ? ws.data_ptr() : nullptr, bytes, stream), "spmm");
+  at::Tensor owner;
+  void* ws = bytes ? scratch.bytes(bytes, &owner) : nullptr;
+  check(cagnet_spmm_block_f32(b, B, ldb, C, ldc, f, beta, ws, bytes, stream), "spmm");
   return cagnet_spmm_block_launches(b, ldb, f);
 }
 
@@ -77,8 +113,9 @@ int64_t spmm(uintptr_t block, int64_t device, const at::Tensor& B, const at::Ten
   if (B.get_device() != device || C.get_device() != device) refuse("spmm operands on different devices");
   if (B.size(1) > INT32_MAX) refuse("spmm is too wide");
   c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+  Scratch scratch(C.options().requires_grad(false), 0);
   return multiply(b, B.data_ptr<float>(), ldb, C.data_ptr<float>(), ldc, static_cast<int32_t>(B.size(1)), static_cast<float>(beta),
-                  C.options(), c10::cuda::getCurrentCUDAStream().stream());
+                  scratch, c10::cuda::getCurrentCUDAStream().stream());
 }
 
 // C += A.B with A as COO: the verdict of the index check is read back while the (guarded) product is already queued.
@@ -136,10 +173,10 @@ int64_t spmm_coo(const at::Tensor& rows, const at::Tensor& cols, const at::Tenso
   return 2 + (validate ? 1 : 0);
 }
 
+// State of torch.optim.Adam over both weights; the step counts are the optimizer's own (fp32 on the host) and are advanced.
 struct Adam {
-  at::Tensor m1, v1, m2, v2;
+  at::Tensor m1, v1, step1, m2, v2, step2;
   double lr, beta1, beta2, eps;
-  int64_t step;
 };
 
 // One epoch of the two-layer model on one process: out = act2((A h) W2), h = act1((A x) W1) -- or A (h W), where
@@ -164,9 +201,12 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
   void* s = c10::cuda::getCurrentCUDAStream().stream();
   const auto o = x.options().requires_grad(false);
   int64_t launches = 0;
+  // One allocation for what a small epoch needs: its matrices (eight at most) and about as much again for workspaces.
+  const int64_t floats = n * (pad_ld(f) + 4 * pad_ld(h) + 3 * pad_ld(c));
+  Scratch scratch(o, floats <= (2 << 20) ? static_cast<size_t>(floats) * 8 + (4 << 20) : 0);
   auto product = [&](const cagnet_block* b, const float* B, int64_t ldb, const Buffer& C, int32_t width) {
     if (!hook.is_none()) hook(true, b == At && b != A, width);
-    launches += multiply(b, B, ldb, C.p(), C.ld, width, 0.f, o, s);
+    launches += multiply(b, B, ldb, C.p(), C.ld, width, 0.f, scratch, s);
     if (!hook.is_none()) hook(false, b == At && b != A, width);
   };
   auto gemm = [&](const float* X, int64_t ld, const at::Tensor& W, bool transposed, const Buffer& Z, int32_t K, int32_t N, int epi,
@@ -183,21 +223,18 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
     check(cagnet_log_softmax_fwd_f32(Z.p(), Z.ld, Z.p(), Z.ld, n, N, s), "log_softmax");
     ++launches;
   };
-  auto tn = [&](const float* H, int64_t ldh, const Buffer& G, int32_t K, int32_t N) {
-    at::Tensor out = at::empty({K, N}, o);
+  auto tn = [&](const float* H, int64_t ldh, const Buffer& G, int32_t K, int32_t N, cagnet_tn_sum& sum) {
     const size_t bytes = cagnet_gemm_tn_workspace_bytes(n, K, N);
-    at::Tensor ws = bytes_buffer(o, bytes);
-    check(cagnet_gemm_tn_f32(H, ldh, G.p(), G.ld, out.data_ptr<float>(), N, n, K, N, 0.f, ws.data_ptr(), ws.numel() * 4, s), "gemm_tn");
-    launches += 2;
-    return out;
+    check(cagnet_gemm_tn_partials_f32(H, ldh, G.p(), G.ld, n, K, N, scratch.bytes(bytes), bytes, &sum, s), "gemm_tn");
+    ++launches;
   };
   const float* X = x.data_ptr<float>();
   const bool narrow1 = min_width && h < f, widen1 = min_width && h > f, narrow2 = min_width && c < h, widen2 = min_width && c > h;
 
   // ---- forward
-  Buffer H(o, n, h), agg1, agg2;
+  Buffer H(scratch, n, h), agg1, agg2;
   if (narrow1) {
-    Buffer hw(o, n, h);
+    Buffer hw(scratch, n, h);
     gemm(X, ldx, w1, false, hw, f, h, CAGNET_EPI_NONE, nullptr, 0);
     product(A, hw.p(), hw.ld, H, h);
     if (activations) {
@@ -205,14 +242,15 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
       ++launches;
     }
   } else {
-    Buffer z(o, n, f);
+    Buffer z(scratch, n, f);
     product(A, X, ldx, z, f);
     dense_layer(z.p(), z.ld, w1, H, f, h, false);
     if (widen1) agg1 = z;
   }
-  Buffer out(o, n, c);
+  const at::Tensor out_t = at::empty({std::max<int64_t>(n, 1), pad_ld(c)}, o);
+  const Buffer out(out_t);
   if (narrow2) {
-    Buffer hw(o, n, c);
+    Buffer hw(scratch, n, c);
     gemm(H.p(), H.ld, w2, false, hw, h, c, CAGNET_EPI_NONE, nullptr, 0);
     product(A, hw.p(), hw.ld, out, c);
     if (activations) {
@@ -220,71 +258,77 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
       ++launches;
     }
   } else {
-    Buffer z(o, n, h);
+    Buffer z(scratch, n, h);
     product(A, H.p(), H.ld, z, h);
     dense_layer(z.p(), z.ld, w2, out, h, c, true);
     if (widen2) agg2 = z;
   }
 
   // ---- loss, and its gradient before the second activation
-  at::Tensor loss = at::empty({}, o), loss_ws = bytes_buffer(o, cagnet_nll_workspace_bytes(n));
-  Buffer dz(o, n, c);
+  at::Tensor loss = at::empty({}, o);
+  const size_t loss_bytes = cagnet_nll_workspace_bytes(n);
+  float* loss_ws = static_cast<float*>(scratch.bytes(loss_bytes));
+  Buffer dz(scratch, n, c);
   int32_t parts = 0;
   const auto* mask8 = static_cast<const uint8_t*>(mask.data_ptr());
   if (activations) {
     check(cagnet_nll_softmax_bwd_f32(out.p(), out.ld, y.data_ptr<int64_t>(), mask8, n, c, static_cast<int32_t>(cls_lo),
                                      static_cast<int32_t>(cls_hi), static_cast<float>(count), dz.p(), dz.ld, &parts,
-                                     loss_ws.data_ptr(), loss_ws.numel() * 4, s), "nll_softmax_bwd");
+                                     loss_ws, loss_bytes, s), "nll_softmax_bwd");
     ++launches;
   } else {
     check(cagnet_nll_masked_f32(out.p(), out.ld, y.data_ptr<int64_t>(), mask8, n, c, static_cast<int32_t>(cls_lo),
                                 static_cast<int32_t>(cls_hi), static_cast<float>(count), 1.f, loss.data_ptr<float>(), dz.p(), dz.ld,
-                                loss_ws.data_ptr(), loss_ws.numel() * 4, s), "nll_masked");
+                                loss_ws, loss_bytes, s), "nll_masked");
     launches += 2;
   }
 
   // ---- backward: second layer
-  Buffer dh(o, n, h);         // gradient before the first activation
-  at::Tensor g1, g2;
+  Buffer dh(scratch, n, h);         // gradient before the first activation
+  cagnet_tn_sum sum1, sum2;
   const int mask_epi = activations ? CAGNET_EPI_RELU_MASK : CAGNET_EPI_NONE;
   if (widen2) {
-    Buffer dzw(o, n, h);
+    Buffer dzw(scratch, n, h);
     gemm(dz.p(), dz.ld, w2, true, dzw, c, h, CAGNET_EPI_NONE, nullptr, 0);
     product(At, dzw.p(), dzw.ld, dh, h);
     if (activations) {
       check(cagnet_relu_bwd_f32(H.p(), H.ld, dh.p(), dh.ld, dh.p(), dh.ld, n, h, s), "relu_bwd");
       ++launches;
     }
-    g2 = tn(agg2.p(), agg2.ld, dz, h, c);
+    tn(agg2.p(), agg2.ld, dz, h, c, sum2);
   } else {
-    Buffer ag(o, n, c);
+    Buffer ag(scratch, n, c);
     product(At, dz.p(), dz.ld, ag, c);
     gemm(ag.p(), ag.ld, w2, true, dh, c, h, mask_epi, H.p(), H.ld);
-    g2 = tn(H.p(), H.ld, ag, h, c);
+    tn(H.p(), H.ld, ag, h, c, sum2);
   }
   // ---- backward: first layer
   if (widen1) {
-    g1 = tn(agg1.p(), agg1.ld, dh, f, h);
+    tn(agg1.p(), agg1.ld, dh, f, h, sum1);
   } else {
-    Buffer ag(o, n, h);
+    Buffer ag(scratch, n, h);
     product(At, dh.p(), dh.ld, ag, h);
-    g1 = tn(X, ldx, ag, f, h);
+    tn(X, ldx, ag, f, h, sum1);
   }
-  if (adam || activations) {
-    float* loss_p = activations ? loss.data_ptr<float>() : nullptr;
-    const auto* parts_p = loss_ws.data_ptr<float>();
-    if (adam) {
-      check(cagnet_adam2_f32(w1.data_ptr<float>(), adam->m1.data_ptr<float>(), adam->v1.data_ptr<float>(), g1.data_ptr<float>(), w1.numel(),
-                             w2.data_ptr<float>(), adam->m2.data_ptr<float>(), adam->v2.data_ptr<float>(), g2.data_ptr<float>(), w2.numel(),
-                             adam->lr, adam->beta1, adam->beta2, adam->eps, adam->step, parts_p, parts, static_cast<float>(count), loss_p, s),
-            "adam");
-    } else {
-      check(cagnet_adam2_f32(nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0, 0, 1, parts_p, parts,
-                             static_cast<float>(count), loss_p, s), "loss");
-    }
-    ++launches;
+  // ---- gradients from their partial sums, Adam, loss
+  at::Tensor g1 = at::empty({f, h}, o), g2 = at::empty({h, c}, o);
+  std::array<float*, 6> a = {};
+  int64_t step = 1;
+  if (adam) {
+    float *t1 = adam->step1.data_ptr<float>(), *t2 = adam->step2.data_ptr<float>();
+    step = static_cast<int64_t>(*t1) + 1;
+    a = {w1.data_ptr<float>(), adam->m1.data_ptr<float>(), adam->v1.data_ptr<float>(),
+         w2.data_ptr<float>(), adam->m2.data_ptr<float>(), adam->v2.data_ptr<float>()};
+    *t1 += 1.f;
+    *t2 += 1.f;
+    adam->step1.unsafeGetTensorImpl()->bump_version();
+    adam->step2.unsafeGetTensorImpl()->bump_version();
   }
-  return py::make_tuple(out.t.narrow(1, 0, c).narrow(0, 0, n), loss, g1, g2, launches);
+  check(cagnet_epoch_tail_f32(&sum1, g1.data_ptr<float>(), a[0], a[1], a[2], &sum2, g2.data_ptr<float>(), a[3], a[4], a[5],
+                              adam ? adam->lr : 0., adam ? adam->beta1 : 0., adam ? adam->beta2 : 0., adam ? adam->eps : 0., step,
+                              loss_ws, parts, static_cast<float>(count), activations ? loss.data_ptr<float>() : nullptr, s), "epoch_tail");
+  ++launches;
+  return py::make_tuple(out_t.narrow(1, 0, c).narrow(0, 0, n), loss, g1, g2, launches);
 }
 
 }  // namespace
@@ -292,9 +336,9 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
 PYBIND11_MODULE(_host, m) {
   m.def("spmm", &spmm);
   m.def("spmm_coo", &spmm_coo);
-  py::class_<Adam>(m, "Adam").def(py::init([](at::Tensor m1, at::Tensor v1, at::Tensor m2, at::Tensor v2, double lr, double beta1,
-                                              double beta2, double eps, int64_t step) {
-    return Adam{m1, v1, m2, v2, lr, beta1, beta2, eps, step};
+  py::class_<Adam>(m, "Adam").def(py::init([](at::Tensor m1, at::Tensor v1, at::Tensor step1, at::Tensor m2, at::Tensor v2,
+                                              at::Tensor step2, double lr, double beta1, double beta2, double eps) {
+    return Adam{m1, v1, step1, m2, v2, step2, lr, beta1, beta2, eps};
   }));
   m.def("epoch", &epoch);
 }

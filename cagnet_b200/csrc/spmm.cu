@@ -119,6 +119,11 @@ __device__ __forceinline__ void store_row(float* __restrict__ cp, int column0, i
 __device__ __forceinline__ void pdl_release_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 // True for the appended block: its first thread waits for the hub kernel, all its threads then leave.
 __device__ __forceinline__ bool pdl_waiter_block(int waiter) {
+  if (waiter < 0) {           // no hub kernel: an ordinary dependent of the kernel in front (common.cuh)
+    pdl_trigger();
+    pdl_wait();
+    return false;
+  }
   if (!waiter || blockIdx.x != gridDim.x - 1) return false;
   if (blockIdx.y == 0 && threadIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
   return true;
@@ -592,8 +597,10 @@ static int launch_spmm_impl(const int* rowptr, const int* col, const float* val,
   cfg.attrs = attr;
   // Measured on one box, serialised against overlapped: 4 M-vertex R-MAT graph width 128 7.99 -> 6.95 ms, width 602
   // 37.4 -> 36.8 ms; 233K-vertex graph width 602 with its dense core 10.14 -> 9.52 ms; width 16 0.78 -> 0.76 ms.
-  cfg.numAttrs = (plan && g_tuning.spmm_overlap) ? 1 : 0;
-  const int waiter = static_cast<int>(cfg.numAttrs);      // one block more, which only waits for the hub kernel
+  // Without a hub kernel the launch latency of a small multiply hides under the kernel in front (epoch of 16 K vertices:
+  // 2 - 5 us between kernels); large ones start on idle SMs for the reason given at the nonzero-split launch.
+  cfg.numAttrs = (plan ? g_tuning.spmm_overlap : nnz * tiles <= (1 << 21)) ? 1 : 0;
+  const int waiter = plan ? static_cast<int>(cfg.numAttrs) : -static_cast<int>(cfg.numAttrs);   // 1: one block that only waits
   cudaError_t e;
   bool grouped = false;
   if constexpr (LPN < 32) grouped = g_tuning.spmm_group_avg > 0 && nnz <= static_cast<int64_t>(g_tuning.spmm_group_avg) * n;
@@ -601,13 +608,13 @@ static int launch_spmm_impl(const int* rowptr, const int* col, const float* val,
     if (grouped) {
       const int pool = group_pool_rows(n);
       const int pools = (n + pool - 1) / pool;
-      cfg.gridDim = dim3((pools + rows_per_block - 1) / rows_per_block + waiter, tiles);
+      cfg.gridDim = dim3((pools + rows_per_block - 1) / rows_per_block + max(waiter, 0), tiles);
       e = cudaLaunchKernelEx(&cfg, spmm_group_rows_kernel<VEC, LPN, NV, DEEP>, rowptr, col, val, n, B, ldb, C, ldc, f_eff, f,
                              beta, plan, min_threshold, g_tuning.spmm_group_max, pool, waiter);
     }
   }
   if (!grouped) {
-    cfg.gridDim = dim3((n + rows_per_block - 1) / rows_per_block + waiter, tiles);
+    cfg.gridDim = dim3((n + rows_per_block - 1) / rows_per_block + max(waiter, 0), tiles);
     e = cudaLaunchKernelEx(&cfg, spmm_warp_rows_kernel<VEC, LPN, NV, DEEP>, rowptr, col, val, n, B, ldb, C, ldc, f_eff, f, beta,
                            plan, min_threshold, waiter);
   }

@@ -24,7 +24,7 @@ def _weight_ok(w, device):
 
 
 def _adam_state(optimizer, w1, w2):
-    """(exp_avg, exp_avg_sq) of both weights, step count and options of a default torch.optim.Adam over [w1, w2], created
+    """States (exp_avg, exp_avg_sq, step) of both weights and the options of a default torch.optim.Adam over [w1, w2], created
     as its first step would create them; None for any other optimizer."""
     if type(optimizer) is not torch.optim.Adam or len(optimizer.param_groups) != 1:
         return None
@@ -42,13 +42,13 @@ def _adam_state(optimizer, w1, w2):
             s["step"] = torch.tensor(0.0, dtype=torch.float32)
             s["exp_avg"] = torch.zeros_like(w, memory_format=torch.preserve_format)
             s["exp_avg_sq"] = torch.zeros_like(w, memory_format=torch.preserve_format)
-        if not (s["exp_avg"].is_contiguous() and s["exp_avg_sq"].is_contiguous()) or s["step"].is_cuda:
+        if not (s["exp_avg"].is_contiguous() and s["exp_avg_sq"].is_contiguous()) or s["step"].is_cuda or \
+                s["step"].dtype != torch.float32:
             return None
         states.append(s)
-    step = float(states[0]["step"])
-    if float(states[1]["step"]) != step:
+    if float(states[0]["step"]) != float(states[1]["step"]):
         return None
-    return states, int(step) + 1, g
+    return states, g
 
 
 def plan(backend, fwd, bwd, cls_lo, cls_hi, activations, min_width):
@@ -71,9 +71,9 @@ def train(p, model, x, y, mask, count):
     host = _native.host()
     adam, hook = None, None
     if state is not None:
-        (s1, s2), step, g = state
-        adam = host.Adam(s1["exp_avg"], s1["exp_avg_sq"], s2["exp_avg"], s2["exp_avg_sq"], g["lr"], g["betas"][0],
-                         g["betas"][1], g["eps"], step)
+        (s1, s2), g = state
+        adam = host.Adam(s1["exp_avg"], s1["exp_avg_sq"], s1["step"], s2["exp_avg"], s2["exp_avg_sq"], s2["step"], g["lr"],
+                         g["betas"][0], g["betas"][1], g["eps"])
     if p.backend.spmm_events is not None:
         hook = _event_hook(p)
     out, loss, g1, g2, launches = host.epoch(p.fwd.address(), p.bwd.address(), x, w1.detach(), w2.detach(), y.contiguous(),
@@ -81,8 +81,6 @@ def train(p, model, x, y, mask, count):
     ops.LAUNCHES[0] += launches
     w1.grad, w2.grad = g1, g2
     if state is not None:
-        s1["step"] += 1
-        s2["step"] += 1
         model.optimizer._opt_called = True        # what lr schedulers look at
         torch.autograd.graph.increment_version((w1, w2))
     else:

@@ -288,6 +288,15 @@ int cagnet_gemm_tn_f32(const float* H, int64_t ldh, const float* G, int64_t ldg,
                        float* out, int64_t ldo, int64_t n, int32_t K, int32_t N, float beta,
                        void* ws, size_t ws_bytes, void* stream);
 
+/* The same product left as partial sums in ws (which has to live until they are added up), described by *sum: `chunks` of
+ * K x N floats, of the transpose where `transposed` is set. */
+typedef struct {
+  float* partials;
+  int32_t chunks, K, N, transposed;
+} cagnet_tn_sum;
+int cagnet_gemm_tn_partials_f32(const float* H, int64_t ldh, const float* G, int64_t ldg, int64_t n, int32_t K, int32_t N,
+                                void* ws, size_t ws_bytes, cagnet_tn_sum* sum, void* stream);
+
 /* ---- Elementwise / row-wise pieces, for callers that do not use the fused epilogues. */
 int cagnet_relu_fwd_f32(const float* z, int64_t ldz, float* h, int64_t ldh, int64_t n, int32_t N, void* stream);
 /* dz = h > 0 ? g : 0 */
@@ -329,18 +338,19 @@ int cagnet_nll_masked_f32(const float* logp, int64_t ldl, const int64_t* y, cons
 /* ---- The loss of a log-softmax model and its gradient before the log-softmax in one pass:
  * dz[i, j] = (exp(logp[i, j]) - [j == y_i - cls_lo]) / count for rows with mask[i] and a label in [cls_lo, cls_hi), 0 for
  * the others: log_softmax_bwd of nll_masked's gradient.  Leaves *parts (host) partial sums of logp[i, y_i] in ws
- * (cagnet_nll_workspace_bytes), which cagnet_adam2_f32 turns into the loss.  F.nll_loss and the autograd calls at
+ * (cagnet_nll_workspace_bytes), which cagnet_epoch_tail_f32 turns into the loss.  F.nll_loss and the autograd calls at
  * gcn_distr.py:356 and :312-322. */
 int cagnet_nll_softmax_bwd_f32(const float* logp, int64_t ldl, const int64_t* y, const uint8_t* mask, int64_t n, int32_t N,
                                int32_t cls_lo, int32_t cls_hi, float count, float* dz, int64_t lddz, int32_t* parts,
                                void* ws, size_t ws_bytes, void* stream);
 
-/* ---- One Adam step (torch.optim.Adam with default options; `step` counts from 1) on two parameter tensors of n1 and n2
- * elements in one launch.  With loss != NULL also *loss = -sum(loss_parts[0 .. parts)) / count.  optimizer.step() at
- * gcn_distr.py:364. */
-int cagnet_adam2_f32(float* p1, float* m1, float* v1, const float* g1, int64_t n1, float* p2, float* m2, float* v2,
-                     const float* g2, int64_t n2, double lr, double beta1, double beta2, double eps, int64_t step,
-                     const float* loss_parts, int32_t parts, float count, float* loss, void* stream);
+/* ---- The end of an epoch in one launch: both weight gradients g1, g2 (contiguous) from the partial products that
+ * cagnet_gemm_tn_partials_f32 left, one Adam step (torch.optim.Adam with default options; `step` counts from 1) on the
+ * weights p1, p2 unless they are NULL, and with loss != NULL *loss = -sum(loss_parts[0 .. parts)) / count.
+ * loss.backward()'s last products and optimizer.step() at gcn_distr.py:356-364. */
+int cagnet_epoch_tail_f32(const cagnet_tn_sum* s1, float* g1, float* p1, float* m1, float* v1, const cagnet_tn_sum* s2,
+                          float* g2, float* p2, float* m2, float* v2, double lr, double beta1, double beta2, double eps,
+                          int64_t step, const float* loss_parts, int32_t parts, float count, float* loss, void* stream);
 
 #ifdef __cplusplus
 }

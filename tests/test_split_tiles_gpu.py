@@ -121,18 +121,22 @@ def test_fused_loss_and_adam(n, N, lo, hi):
     _native.check(L.cagnet_nll_softmax_bwd_f32(logp.data_ptr(), logp.stride(0), yd.data_ptr(), md.data_ptr(), n, N, lo, hi, float(n),
                                                dz.data_ptr(), dz.stride(0), ctypes.byref(parts), ws.data_ptr(), ws.numel(), None))
     _close(dz, z64.grad)
-    w = [torch.randn(k, generator=g).cuda() for k in (n * 3, N)]
+    w = [torch.randn(*k, generator=g).cuda() for k in ((n, 3), (5, N))]
     ref = [torch.nn.Parameter(t.clone()) for t in w]
     opt = torch.optim.Adam(ref, lr=0.01)
     state = [[torch.zeros_like(t), torch.zeros_like(t)] for t in w]
     loss = torch.empty((), device="cuda")
     for step in (1, 2, 3):
-        grads = [torch.randn(t.numel(), generator=g).cuda() for t in w]
+        partials = [torch.randn(11, 3, n, generator=g).cuda(), torch.randn(3, 5, N, generator=g).cuda()]      # the first transposed
+        sums = [_native.TnSum(d.data_ptr(), d.size(0), d.size(1), d.size(2), k) for d, k in zip(partials, (1, 0))]
+        grads = [torch.full_like(t, float("nan")) for t in w]
+        ptr = [x for t, s, d, q in zip(w, state, grads, sums) for x in (ctypes.addressof(q), d.data_ptr(), t.data_ptr(), s[0].data_ptr(), s[1].data_ptr())]
+        _native.check(L.cagnet_epoch_tail_f32(*ptr, 0.01, 0.9, 0.999, 1e-8, step, ws.data_ptr(), parts.value, float(n), loss.data_ptr(), None))
+        _close(grads[0], partials[0].double().sum(0).t().cpu())
+        _close(grads[1], partials[1].double().sum(0).cpu())
         for p, d in zip(ref, grads):
-            p.grad = d
+            p.grad = d.clone()
         opt.step()
-        ptr = [x for t, s, d in zip(w, state, grads) for x in (t.data_ptr(), s[0].data_ptr(), s[1].data_ptr(), d.data_ptr(), t.numel())]
-        _native.check(L.cagnet_adam2_f32(*ptr, 0.01, 0.9, 0.999, 1e-8, step, ws.data_ptr(), parts.value, float(n), loss.data_ptr(), None))
     for t, p in zip(w, ref):
         _close(t, p.detach().cpu())
     assert abs(float(loss) - float(want)) <= 1e-5 * max(abs(float(want)), 1e-6)
