@@ -78,6 +78,19 @@ int spmm_forced_tile();      // "spmm_tile" when a sweep has set it: such multip
 bool gemm_nn_tc_applies(const float* X, int64_t ldx, int64_t n, int K, int N, int epilogue);
 int gemm_nn_tc(const float* X, int64_t ldx, const float* W, int64_t ldw, int transW, float* Z, int64_t ldz, int64_t n, int K, int N,
                int epilogue, const float* aux, int64_t ldaux, cudaStream_t s);
+// The masked NLL of log-softmax rows and its gradient before the log-softmax, written with them by the product's epilogue.
+struct TcLoss {
+  const int64_t* y;
+  const uint8_t* mask;
+  float* dz;
+  float* parts;              // partial sums of the labels' log-probabilities, kTcLossParts at most
+  int64_t lddz;
+  int cls_lo, cls_hi;
+  float inv_count;
+};
+constexpr int kTcLossParts = kNumSMs * 16;
+int gemm_nn_tc_nll(const float* X, int64_t ldx, const float* W, int64_t ldw, float* Z, int64_t ldz, int64_t n, int K, int N, const TcLoss& loss,
+                   int32_t* parts, cudaStream_t s);
 bool gemm_tn_tc_applies(const float* H, int64_t ldh, const float* G, int64_t ldg, int64_t n, int K, int N);
 int gemm_tn_tc_blocks(int64_t n, int K, int N);
 int gemm_tn_tc(const float* H, int64_t ldh, const float* G, int64_t ldg, int64_t n, int K, int N, float* part, cudaStream_t s);

@@ -8,12 +8,14 @@
 //   warp 0        TMA boxes of 128 rows x 32 columns of X into a ring of stages (128-byte swizzle; rows and columns outside
 //                 the matrix arrive as zeros)
 //   warps 12 - 27 four groups take the boxes in turn: a thread reads its row's 128 bytes, splits them and stores the three
-//                 terms to TENSOR memory, where the multiply takes its A operand from
+//                 terms to TENSOR memory, where the multiply takes its A operand from (K <= 64: warps 20 - 27, two groups)
 //   warp 1        tcgen05.mma kind::f16, M = 128, against W's terms, which stay in shared memory (K-major, 128-byte swizzle) for
 //                 the block's whole run
-//   warps 4 - 11  sums out of tensor memory (a thread holds a whole row: log-softmax needs no exchange), epilogue, whole
-//                 row segments to Z through a shared-memory exchange
-// Blocks are persistent over row tiles.
+//   warps 4 - 11  sums out of tensor memory (K <= 64: warps 4 - 19), epilogue, whole row segments to Z through a shared-memory
+//                 exchange; the sums are given back to warp 1 as soon as they are read, before they are stored
+// Blocks are persistent over row tiles.  With K <= 64 a tile has two boxes at most and the time is the epilogue's, which is
+// why it gets twice the warps there (300K x 47 x 64 with the ReLU mask: 138 us with 8 storing warps that asked for the mask
+// after the sums were there and kept the sums until everything was stored).
 #include <cuda.h>
 #include <limits.h>
 #include <math.h>
@@ -29,10 +31,18 @@ constexpr int kXStageBytes = 128 * 128;           // 128 rows x 32 floats
 constexpr int kTcThreads = 896;
 constexpr int kTcMaxStages = 8;
 constexpr int kTcSmem = 226 * 1024;
-constexpr int kTcExchange = 8 * 32 * 36 * 4;      // storing warps: 32 rows x 32 columns each, rows padded to 36 floats
 constexpr int kTcMaxW = 124 * 1024;               // W's terms
-constexpr int kTcBuffers = 4;                     // operand buffers of 3 terms x 16 tensor-memory columns
+constexpr int kTcMaxBuffers = 4;                  // operand buffers of 3 terms x 16 tensor-memory columns
 constexpr int kTcBufferCols = 48;
+constexpr int kTcLightK = 64;
+constexpr int kTcSlots = 4;                       // row tiles whose sums are kept at a time, at most
+
+// Storing warps of a block, and columns that one takes at a time (an exchange of 32 rows, padded by 4 floats).
+__host__ __device__ constexpr int tc_storing_warps(int sets) { return sets == 0 ? 16 : 8; }
+__host__ __device__ constexpr bool tc_reads_old(int epilogue) { return epilogue == CAGNET_EPI_RELU_MASK || epilogue == CAGNET_EPI_ACCUMULATE; }
+__host__ __device__ constexpr int tc_piece(bool old) { return old ? 16 : 32; }        // (32 columns of old values in flight spill: 620 bytes)
+__host__ __device__ constexpr int tc_exchange_bytes(int sets, bool old) { return tc_storing_warps(sets) * 32 * (tc_piece(old) + 4) * 4; }
+constexpr int kEpiNll = 6;                        // log-softmax, its masked NLL and the gradient before the log-softmax
 
 struct TcArgs {
   const float* W;
@@ -40,6 +50,7 @@ struct TcArgs {
   float* Z;
   int64_t ldw, ldz, ldaux, n;
   int transW, K, N, NP, z_vec4, aux_vec4, stages, tiles;
+  TcLoss loss;
 };
 
 __device__ int g_gemm_error;
@@ -71,47 +82,56 @@ __device__ __forceinline__ void load_sums(unsigned at, int NP, float (&v)[16]) {
   }
 }
 
-// Barrier of the 64 threads that share `id`, and whether `ok` holds for all of them.
-__device__ __forceinline__ bool pair_and(bool ok, int id) {
+// Barrier of the `threads` threads that share `id`, and whether `ok` holds for all of them.
+__device__ __forceinline__ bool group_and(bool ok, int id, int threads) {
   unsigned r;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 p, %1, 0;\n\t"
-      "barrier.cta.red.and.pred q, %2, 64, p;\n\t"
+      "barrier.cta.red.and.pred q, %2, %3, p;\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(r)
-      : "r"(ok ? 1u : 0u), "r"(id)
+      : "r"(ok ? 1u : 0u), "r"(id), "r"(threads)
       : "memory");
   return r != 0;
 }
 
 // SETS > 0: the terms of W side by side, three sums of NP columns (x1 w1 | x1 w2 + x2 w1 | x1 w3 + x2 w2 + x3 w1) that three
-// products of N = 3 NP, 2 NP, NP per k step fill; SETS = 0 (NP > 80, K <= 64): all six products into one sum.  An addition in
-// tensor memory drops what does not fit (1.7e-8 of the sum on average, always towards zero), so the number of additions per
-// sum is kept at the size of fp32 rounding: K > 320 alternates between two sets of sums, N > 80 with K > 64 is cut into parts.
+// products of N = 3 NP, 2 NP, NP per k step fill; SETS = 0 (K <= 64): all products into one sum, which leaves room for more
+// row tiles in tensor memory and a third of it to read.  An addition in tensor memory drops what does not fit (1.7e-8 of
+// the sum on average, always towards zero), so the number of additions to a full-sized sum is kept at the size of fp32
+// rounding: SETS = 0 adds the five small products of all k first, K > 320 alternates between two sets of sums.
 template <int SETS, int EPI>
 __global__ void __launch_bounds__(kTcThreads, 1) gemm_nn_tc_kernel(const __grid_constant__ CUtensorMap map, TcArgs a) {
+  constexpr bool LIGHT = SETS == 0;
+  constexpr int STORING = tc_storing_warps(SETS), EXPAND = 4 + STORING, GROUPS = (kTcThreads / 32 - EXPAND) / 4;
   extern __shared__ __align__(1024) char smem_raw[];
-  __shared__ __align__(8) unsigned long long bars[2 * kTcMaxStages + 2 * kTcBuffers + 5];
+  __shared__ __align__(8) unsigned long long bars[2 * kTcMaxStages + 2 * kTcMaxBuffers + 2 * kTcSlots + 1];
   __shared__ unsigned tmem_base_s;
   __shared__ int dead_s;
   char* smem = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = a.stages, NP = a.NP;
+  const int BUF = LIGHT && S < kTcMaxBuffers ? 2 : kTcMaxBuffers;       // a power of two, not above S (see the expanding warps)
   const int kblocks = (a.K + 63) / 64, ksteps = (a.K + 31) / 32;
   const int wtile = 3 * NP * 128;                 // W's terms for 64 k
   char* wsm = smem + S * kXStageBytes;
   float* xch_all = reinterpret_cast<float*>(wsm + kblocks * wtile);
   const int sums = SETS > 0 ? 3 * NP * SETS : NP;   // tensor-memory columns of a row tile's sums
-  const int AS = 2 * sums <= 512 - kTcBuffers * kTcBufferCols ? 2 : 1;
+  // Row tiles whose sums fit at a time.  LIGHT: as many tiles are stored side by side, by PARTS warps per 32 rows each, as one
+  // tile's epilogue is a chain of waits (233K x 16 x 41, log-softmax: 38 us with one tile at a time); else all warps take every
+  // tile.
+  const int room = 512 - BUF * kTcBufferCols;
+  const int AS = LIGHT && kTcSlots * sums <= room ? kTcSlots : 2 * sums <= room ? 2 : 1;
+  const int PARTS = LIGHT ? STORING / 4 / AS : STORING / 4;
   const unsigned bar0 = smem_u32(bars);
   auto full = [&](int s) { return bar0 + 8 * s; };
   auto empty = [&](int s) { return bar0 + 8 * (kTcMaxStages + s); };
   auto a_full = [&](int b) { return bar0 + 8 * (2 * kTcMaxStages + b); };
-  auto a_empty = [&](int b) { return bar0 + 8 * (2 * kTcMaxStages + kTcBuffers + b); };
-  auto acc_full = [&](int c) { return bar0 + 8 * (2 * kTcMaxStages + 2 * kTcBuffers + c); };
-  auto acc_empty = [&](int c) { return bar0 + 8 * (2 * kTcMaxStages + 2 * kTcBuffers + 2 + c); };
-  const unsigned drain = bar0 + 8 * (2 * kTcMaxStages + 2 * kTcBuffers + 4);
+  auto a_empty = [&](int b) { return bar0 + 8 * (2 * kTcMaxStages + BUF + b); };
+  auto acc_full = [&](int c) { return bar0 + 8 * (2 * kTcMaxStages + 2 * BUF + c); };
+  auto acc_empty = [&](int c) { return bar0 + 8 * (2 * kTcMaxStages + 2 * BUF + kTcSlots + c); };
+  const unsigned drain = bar0 + 8 * (2 * kTcMaxStages + 2 * BUF + 2 * kTcSlots);
   volatile int* dead = &dead_s;
 
   if (threadIdx.x == 0) {
@@ -119,13 +139,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_nn_tc_kernel(const __grid_
       mbar_init(full(s), 1);
       mbar_init(empty(s), 4);        // one arrival per warp of the group that read the stage
     }
-    for (int b = 0; b < kTcBuffers; ++b) {
+    for (int b = 0; b < BUF; ++b) {
       mbar_init(a_full(b), 4);
       mbar_init(a_empty(b), 1);
     }
-    for (int c = 0; c < 2; ++c) {
+    for (int c = 0; c < AS; ++c) {
       mbar_init(acc_full(c), 1);
-      mbar_init(acc_empty(c), 8);
+      mbar_init(acc_empty(c), 4 * PARTS);
     }
     mbar_init(drain, 1);
     dead_s = 0;
@@ -161,7 +181,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_nn_tc_kernel(const __grid_
   __syncthreads();
   tc_fence_after();
   const unsigned tmem = tmem_base_s;
-  const unsigned a_col = 512 - kTcBuffers * kTcBufferCols;
+  const unsigned a_col = 512 - BUF * kTcBufferCols;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -191,63 +211,102 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_nn_tc_kernel(const __grid_
       const unsigned term = static_cast<unsigned>(NP * 128) >> 4;
       int b = 0, c = 0;
       unsigned aph = 0, cph = 0;
-      bool ok = blockIdx.x >= a.tiles || mbar_wait(a_full(0), 0, dead);
-      for (int t = blockIdx.x; t < a.tiles && ok; t += gridDim.x) {
-        ok = mbar_wait(acc_empty(c), cph ^ 1, dead);
-        for (int k = 0; k < ksteps && ok; ++k) {
-          const int set = SETS == 2 ? k & 1 : 0;
-          const unsigned d = tmem + c * sums + set * 3 * NP;
-          const unsigned long long w = smem_desc(smem_u32(wsm + (k >> 1) * wtile) + (k & 1) * 64);
-          const unsigned at = tmem + a_col + b * kTcBufferCols;
-          const int nb = b + 1 == kTcBuffers ? 0 : b + 1;
-          const unsigned naph = nb ? aph : aph ^ 1;
+      if constexpr (LIGHT) {
+        bool ok = true;
+        for (int t = blockIdx.x; t < a.tiles && ok; t += gridDim.x) {
+          const unsigned d = tmem + c * sums;
+          const int b1 = (b + 1) & (BUF - 1);
+          const unsigned aph1 = b1 ? aph : aph ^ 1;
+          auto multiply = [&](int k, int buffer, bool large) {
+            const unsigned long long w = smem_desc(smem_u32(wsm) + k * 64);
+            const unsigned at = tmem + a_col + buffer * kTcBufferCols;
+            for (int ks = 0; ks < 2 && k * 32 + ks * 16 < a.K; ++ks) {
+              const unsigned x1 = at + ks * 8, x2 = x1 + 16, x3 = x1 + 32;
+              const unsigned long long w1 = w + ks * 2, w2 = w1 + term, w3 = w2 + term;
+              if (large) {
+                tc_mma_ts(d, x1, w1, i1, 1u);
+              } else {
+                tc_mma_ts(d, x3, w1, i1, k + ks > 0 ? 1u : 0u);
+                tc_mma_ts(d, x2, w2, i1, 1u);
+                tc_mma_ts(d, x1, w3, i1, 1u);
+                tc_mma_ts(d, x2, w1, i1, 1u);
+                tc_mma_ts(d, x1, w2, i1, 1u);
+              }
+            }
+          };
+          ok = mbar_wait(acc_empty(c), cph ^ 1, dead) && mbar_wait(a_full(b), aph, dead);
+          if (!ok) break;
           tc_fence_after();
+          multiply(0, b, false);
+          if (ksteps == 2) {
+            ok = mbar_wait(a_full(b1), aph1, dead);
+            if (!ok) break;
+            tc_fence_after();
+            multiply(1, b1, false);
+          }
+          multiply(0, b, true);
+          tc_commit(a_empty(b));
+          b = b1;
+          aph = aph1;
+          if (ksteps == 2) {
+            multiply(1, b, true);
+            tc_commit(a_empty(b));
+            b = (b + 1) & (BUF - 1);
+            aph = b ? aph : aph ^ 1;
+          }
+          tc_commit(acc_full(c));
+          if (++c == AS) { c = 0; cph ^= 1; }
+        }
+      } else {
+        bool ok = blockIdx.x >= a.tiles || mbar_wait(a_full(0), 0, dead);
+        for (int t = blockIdx.x; t < a.tiles && ok; t += gridDim.x) {
+          ok = mbar_wait(acc_empty(c), cph ^ 1, dead);
+          for (int k = 0; k < ksteps && ok; ++k) {
+            const int set = SETS == 2 ? k & 1 : 0;
+            const unsigned d = tmem + c * sums + set * 3 * NP;
+            const unsigned long long w = smem_desc(smem_u32(wsm + (k >> 1) * wtile) + (k & 1) * 64);
+            const unsigned at = tmem + a_col + b * kTcBufferCols;
+            const int nb = b + 1 == BUF ? 0 : b + 1;
+            const unsigned naph = nb ? aph : aph ^ 1;
+            tc_fence_after();
 #pragma unroll
-          for (int ks = 0; ks < 2; ++ks) {
-            if (ks == 1 && k * 32 + 16 >= a.K) break;          // nothing but zeros
-            const unsigned first = k >= max(SETS, 1) || ks > 0 ? 1u : 0u;
-            if constexpr (SETS > 0) {
+            for (int ks = 0; ks < 2; ++ks) {
+              if (ks == 1 && k * 32 + 16 >= a.K) break;          // nothing but zeros
+              const unsigned first = k >= max(SETS, 1) || ks > 0 ? 1u : 0u;
               tc_mma_ts(d, at + ks * 8, w + ks * 2, i3, first);
               tc_mma_ts(d + NP, at + 16 + ks * 8, w + ks * 2, i2, 1u);
               tc_mma_ts(d + 2 * NP, at + 32 + ks * 8, w + ks * 2, i1, 1u);
-            } else {
-              // small products first
-              tc_mma_ts(d, at + 32 + ks * 8, w + ks * 2, i1, first);
-              tc_mma_ts(d, at + 16 + ks * 8, w + term + ks * 2, i1, 1u);
-              tc_mma_ts(d, at + ks * 8, w + 2 * term + ks * 2, i1, 1u);
-              tc_mma_ts(d, at + 16 + ks * 8, w + ks * 2, i1, 1u);
-              tc_mma_ts(d, at + ks * 8, w + term + ks * 2, i1, 1u);
-              tc_mma_ts(d, at + ks * 8, w + ks * 2, i1, 1u);
+              // the wait for the next box stands between the two halves of this one, whose products run meanwhile
+              if (ks == 0 && (k + 1 < ksteps || t + static_cast<int>(gridDim.x) < a.tiles)) ok = mbar_wait(a_full(nb), naph, dead);
             }
-            // the wait for the next box stands between the two halves of this one, whose products run meanwhile
-            if (ks == 0 && (k + 1 < ksteps || t + static_cast<int>(gridDim.x) < a.tiles)) ok = mbar_wait(a_full(nb), naph, dead);
+            tc_commit(a_empty(b));
+            b = nb;
+            aph = naph;
           }
-          tc_commit(a_empty(b));
-          b = nb;
-          aph = naph;
+          if (ok) tc_commit(acc_full(c));
+          if (++c == AS) { c = 0; cph ^= 1; }
         }
-        if (ok) tc_commit(acc_full(c));
-        if (++c == AS) { c = 0; cph ^= 1; }
       }
       if (*dead) {        // products in flight still use the tensor memory
         tc_commit(drain);
         for (int i = 0; i < kWaitLimit && !mbar_try(drain, 0); ++i) {}
       }
     }
-  } else if (warp >= 12) {
-    const int grp = (warp - 12) >> 2;
+  } else if (warp >= EXPAND) {
+    const int grp = (warp - EXPAND) >> 2;
     const int quad = (warp & 3) * 32, row = quad + lane;
-    const unsigned dst = tmem + (static_cast<unsigned>(quad) << 16) + a_col + grp * kTcBufferCols;
+    const unsigned dst0 = tmem + (static_cast<unsigned>(quad) << 16) + a_col;
     const int mine = (a.tiles - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
     const int count = max(0, mine) * ksteps;
     int s = grp % S;
     unsigned ph = static_cast<unsigned>(grp / S) & 1, bph = 1;
-    for (int i = grp; i < count; i += kTcBuffers) {
-      // a stage's phase is known by its parity alone: its previous box (i - S, S >= 4) must have been multiplied first
-      if (!mbar_wait(a_empty(grp), bph, dead)) break;
-      bph ^= 1;
+    int b = grp;
+    for (int i = grp; i < count; i += GROUPS) {
+      // a stage's phase is known by its parity alone: its previous box (i - S, S >= BUF) must have been multiplied first
+      if (!mbar_wait(a_empty(b), bph, dead)) break;
       if (!mbar_wait(full(s), ph, dead)) break;
       tc_fence_after();
+      const unsigned dst = dst0 + b * kTcBufferCols;
       const char* src = smem + s * kXStageBytes + row * 128;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -266,48 +325,61 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_nn_tc_kernel(const __grid_
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(a_full(grp));
-      s += kTcBuffers;
+      if (lane == 0) mbar_arrive(a_full(b));
+      s += GROUPS;
       while (s >= S) { s -= S; ph ^= 1; }
+      b += GROUPS;
+      if (b >= BUF) { b -= BUF; bph ^= 1; }
     }
   } else if (warp >= 4) {
-    // two warps per 32 rows take the 32-column pieces in turn
-    const int half = (warp - 4) >> 2, quad = (warp & 3) * 32;
+    // PARTS warps per 32 rows take their column pieces in turn
+    constexpr bool OLD = tc_reads_old(EPI);
+    constexpr int PIECE = tc_piece(OLD);
+    constexpr bool SOFTMAX = EPI == CAGNET_EPI_LOG_SOFTMAX || EPI == kEpiNll;
+    const int slot = LIGHT ? ((warp - 4) >> 2) / PARTS : 0, part = ((warp - 4) >> 2) - slot * PARTS, quad = (warp & 3) * 32;
+    const int group_id = 1 + slot * 4 + (warp & 3), every = static_cast<int>(gridDim.x) * (LIGHT ? AS : 1);
     const unsigned lane_base = static_cast<unsigned>(quad) << 16;
-    float* xch = xch_all + (warp - 4) * (32 * 36);
+    float* xch = xch_all + (warp - 4) * (32 * (PIECE + 4));
     const int width = min(NP, a.N - n0);
     const bool vec = a.z_vec4 != 0;
-    int c = 0;
+    int c = slot;
     unsigned cph = 0;
-    for (int t = blockIdx.x; t < a.tiles; t += gridDim.x) {
+    [[maybe_unused]] float picked = 0.f;            // log-probabilities of the labels that this thread wrote
+    for (int t = blockIdx.x + slot * gridDim.x; t < a.tiles; t += every) {
       const int64_t row0 = static_cast<int64_t>(t) * 128 + quad;
       const int rows = static_cast<int>(min(static_cast<int64_t>(32), a.n - row0));       // may be <= 0
-      // one piece of COLS columns: LR lanes per row, 32 / LR rows per step
-      auto piece = [&](auto cols_tag, int j0, unsigned acc, float lse) {
-        constexpr int COLS = decltype(cols_tag)::value, LR = COLS / 4, RS = 32 / LR, STRIDE = COLS + 4;
-        const int jj = j0 + (lane % LR) * 4, r0 = lane / LR;
-        const int live = width - jj;
-        float* z = a.Z + (row0 + r0) * a.ldz + n0 + jj;
-        [[maybe_unused]] float4 old[EPI == CAGNET_EPI_RELU_MASK || EPI == CAGNET_EPI_ACCUMULATE ? LR : 1];
-        if constexpr (EPI == CAGNET_EPI_RELU_MASK || EPI == CAGNET_EPI_ACCUMULATE) {
-          // asked for before the sums are read
-          const float* m = EPI == CAGNET_EPI_RELU_MASK ? a.aux + (row0 + r0) * a.ldaux + n0 + jj : z;
-          const int64_t step = (EPI == CAGNET_EPI_RELU_MASK ? a.ldaux : a.ldz) * RS;
+      // a piece of COLS columns: LR lanes per row, 32 / LR rows per step
+      [[maybe_unused]] float4 old[OLD ? PIECE / 4 : 1];
+      [[maybe_unused]] auto ask = [&](auto cols_tag, int j0) {
+        constexpr int LR = decltype(cols_tag)::value / 4, RS = 32 / LR;
+        const int jj = j0 + (lane % LR) * 4, r0 = lane / LR, live = width - jj;
+        const float* m = EPI == CAGNET_EPI_RELU_MASK ? a.aux + (row0 + r0) * a.ldaux + n0 + jj : a.Z + (row0 + r0) * a.ldz + n0 + jj;
+        const int64_t step = (EPI == CAGNET_EPI_RELU_MASK ? a.ldaux : a.ldz) * RS;
 #pragma unroll
-          for (int i = 0; i < LR; ++i) {
-            old[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (live > 0 && r0 + i * RS < rows) {
-              if (live >= 4 && a.aux_vec4) {
-                old[i] = __ldcg(reinterpret_cast<const float4*>(m + i * step));
-              } else {
-                old[i].x = __ldcg(m + i * step);
-                if (live > 1) old[i].y = __ldcg(m + i * step + 1);
-                if (live > 2) old[i].z = __ldcg(m + i * step + 2);
-                if (live > 3) old[i].w = __ldcg(m + i * step + 3);
-              }
+        for (int i = 0; i < LR; ++i) {
+          old[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (live > 0 && r0 + i * RS < rows) {
+            if (live >= 4 && a.aux_vec4) {
+              old[i] = __ldcg(reinterpret_cast<const float4*>(m + i * step));
+            } else {
+              old[i].x = __ldcg(m + i * step);
+              if (live > 1) old[i].y = __ldcg(m + i * step + 1);
+              if (live > 2) old[i].z = __ldcg(m + i * step + 2);
+              if (live > 3) old[i].w = __ldcg(m + i * step + 3);
             }
           }
         }
+      };
+      [[maybe_unused]] int label = -1;              // of row row0 + lane, where the loss has it
+      if constexpr (EPI == kEpiNll) {
+        if (lane < rows && a.loss.mask[row0 + lane]) {
+          const int64_t l = a.loss.y[row0 + lane];
+          if (l >= a.loss.cls_lo && l < a.loss.cls_hi) label = static_cast<int>(l - a.loss.cls_lo);
+        }
+      }
+      auto piece = [&](auto cols_tag, int j0, unsigned acc, float lse) {
+        constexpr int COLS = decltype(cols_tag)::value, LR = COLS / 4, RS = 32 / LR, STRIDE = COLS + 4;
+        const int jj = j0 + (lane % LR) * 4, r0 = lane / LR, live = width - jj;
 #pragma unroll
         for (int h = 0; h < COLS / 16; ++h) {
           float v[16];
@@ -316,42 +388,66 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_nn_tc_kernel(const __grid_
           for (int i = 0; i < 16; i += 4)
             *reinterpret_cast<float4*>(xch + lane * STRIDE + 16 * h + i) = make_float4(v[i] - lse, v[i + 1] - lse, v[i + 2] - lse, v[i + 3] - lse);
         }
+        tc_fence_before();
         __syncwarp();
+        if (lane == 0 && j0 + PIECE * PARTS >= NP) mbar_arrive(acc_empty(c));        // the last that this warp reads of this tile
 #pragma unroll
         for (int i = 0; i < LR; ++i) {
-          float4 v = *reinterpret_cast<const float4*>(xch + (r0 + i * RS) * STRIDE + (lane % LR) * 4);
+          const int r = r0 + i * RS;
+          float4 v = *reinterpret_cast<const float4*>(xch + r * STRIDE + (lane % LR) * 4);
+          [[maybe_unused]] float4 g;
           if constexpr (EPI == CAGNET_EPI_RELU) {
             v = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
           } else if constexpr (EPI == CAGNET_EPI_RELU_MASK) {
             v = make_float4(old[i].x > 0.f ? v.x : 0.f, old[i].y > 0.f ? v.y : 0.f, old[i].z > 0.f ? v.z : 0.f, old[i].w > 0.f ? v.w : 0.f);
           } else if constexpr (EPI == CAGNET_EPI_ACCUMULATE) {
             v = make_float4(v.x + old[i].x, v.y + old[i].y, v.z + old[i].z, v.w + old[i].w);
-          }
-          if (r0 + i * RS < rows && live > 0) {
-            float* p = z + i * RS * a.ldz;
-            if (live >= 4 && vec) {
-              *reinterpret_cast<float4*>(p) = v;
-            } else {
-              p[0] = v.x;
-              if (live > 1) p[1] = v.y;
-              if (live > 2) p[2] = v.z;
-              if (live > 3) p[3] = v.w;
+          } else if constexpr (EPI == kEpiNll) {
+            const int at = __shfl_sync(0xffffffffu, label, r), d = at - jj;
+            g = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (at >= 0) {
+              const float w = a.loss.inv_count;
+              g = make_float4((d == 0 ? -w : 0.f) + expf(v.x) * w, (d == 1 ? -w : 0.f) + expf(v.y) * w, (d == 2 ? -w : 0.f) + expf(v.z) * w,
+                              (d == 3 ? -w : 0.f) + expf(v.w) * w);
+              if (d >= 0 && d < 4) picked += d == 0 ? v.x : d == 1 ? v.y : d == 2 ? v.z : v.w;
             }
+          }
+          if (r < rows && live > 0) {
+            auto store = [&](float* p, const float4& x) {
+              if (live >= 4 && vec) {
+                *reinterpret_cast<float4*>(p) = x;
+              } else {
+                p[0] = x.x;
+                if (live > 1) p[1] = x.y;
+                if (live > 2) p[2] = x.z;
+                if (live > 3) p[3] = x.w;
+              }
+            };
+            store(a.Z + (row0 + r) * a.ldz + n0 + jj, v);
+            if constexpr (EPI == kEpiNll) store(a.loss.dz + (row0 + r) * a.loss.lddz + jj, g);
           }
         }
         __syncwarp();
       };
+      // with a piece of PIECE columns or, at the end of an NP that is no multiple of it, of 16
+      auto sized = [&](int j0, auto&& what) {
+        if (PIECE == 16 || NP - j0 < PIECE) what(std::integral_constant<int, 16>{});
+        else what(std::integral_constant<int, PIECE>{});
+      };
+      if constexpr (OLD) {                          // asked for before the sums are waited for
+        if (PIECE * part < NP) sized(PIECE * part, [&](auto tag) { ask(tag, PIECE * part); });
+      }
       bool ready = mbar_wait(acc_full(c), cph, dead);
-      if constexpr (EPI == CAGNET_EPI_LOG_SOFTMAX) ready = pair_and(ready, 1 + (warp & 3));     // the two leave together
+      if (SOFTMAX && PARTS > 1) ready = group_and(ready, group_id, 32 * PARTS);        // they leave together
       if (!ready) break;
       tc_fence_after();
       const unsigned acc = tmem + lane_base + c * sums;
       float lse = 0.f;
-      if constexpr (EPI == CAGNET_EPI_LOG_SOFTMAX) {
-        // this thread's row, 16 columns at a time; the two warps of a row take every other 16 and exchange what they found.
+      if constexpr (SOFTMAX) {
+        // this thread's row, 16 columns at a time; the warps of a row take them in turn and exchange what they found.
         // (Columns that do not exist count as -infinity: a branch per column would keep the exponentials from overlapping.)
         float mx = -INFINITY, sum = 0.f;
-        for (int j = 16 * half; j < width; j += 32) {
+        for (int j = 16 * part; j < width; j += 16 * PARTS) {
           float v[16];
           load_sums<SETS>(acc + j, NP, v);
           float m = mx;
@@ -366,27 +462,35 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_nn_tc_kernel(const __grid_
           sum = (mx == -INFINITY ? 0.f : sum * expf(mx - m)) + ((e[0] + e[1]) + (e[2] + e[3]));
           mx = m;
         }
-        float2* mine = reinterpret_cast<float2*>(xch) + lane;
-        const float2* other = reinterpret_cast<const float2*>(xch_all + ((warp - 4) ^ 4) * (32 * 36)) + lane;
-        *mine = make_float2(mx, sum);
-        pair_and(true, 1 + (warp & 3));
-        const float2 t2 = *other;
-        pair_and(true, 1 + (warp & 3));
-        const float m2 = fmaxf(mx, t2.x);
-        // the first half's sum first, in both warps
-        const float s_own = mx == -INFINITY ? 0.f : sum * expf(mx - m2), s_other = t2.x == -INFINITY ? 0.f : t2.y * expf(t2.x - m2);
-        sum = half ? s_other + s_own : s_own + s_other;
-        mx = m2;
+        if (PARTS > 1) {
+          reinterpret_cast<float2*>(xch)[lane] = make_float2(mx, sum);
+          group_and(true, group_id, 32 * PARTS);
+          const float* others = xch_all + (slot * PARTS * 4 + (warp & 3)) * (32 * (PIECE + 4));
+          auto of = [&](int p) { return reinterpret_cast<const float2*>(others + 4 * p * (32 * (PIECE + 4)))[lane]; };
+          for (int p = 0; p < PARTS; ++p) mx = fmaxf(mx, of(p).x);
+          sum = 0.f;                                // in the same order in every warp
+          for (int p = 0; p < PARTS; ++p) sum += of(p).x == -INFINITY ? 0.f : of(p).y * expf(of(p).x - mx);
+          group_and(true, group_id, 32 * PARTS);
+        }
         lse = mx + logf(sum);
       }
-      for (int j0 = 32 * half; j0 < NP; j0 += 64) {
-        if (NP - j0 >= 32) piece(std::integral_constant<int, 32>{}, j0, acc, lse);
-        else piece(std::integral_constant<int, 16>{}, j0, acc, lse);
+      for (int j0 = PIECE * part; j0 < NP; j0 += PIECE * PARTS) {
+        if constexpr (OLD) {
+          if (j0 != PIECE * part) sized(j0, [&](auto tag) { ask(tag, j0); });
+        }
+        sized(j0, [&](auto tag) { piece(tag, j0, acc, lse); });
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty(c));
-      if (++c == AS) { c = 0; cph ^= 1; }
+      if (PIECE * part >= NP) {                     // no piece of its own
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty(c));
+      }
+      if (LIGHT || ++c == AS) { c = slot; cph ^= 1; }
+    }
+    if constexpr (EPI == kEpiNll) {
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) picked += __shfl_xor_sync(0xffffffffu, picked, off);
+      if (lane == 0) a.loss.parts[blockIdx.x * STORING + warp - 4] = picked;
     }
   }
   __syncwarp();
@@ -421,7 +525,7 @@ struct TnTcArgs {
 __global__ void __launch_bounds__(kTnThreads, 1) gemm_tn_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                                                                    TnTcArgs a) {
   extern __shared__ __align__(1024) char smem_raw[];
-  __shared__ __align__(8) unsigned long long bars[2 * kTnMaxSlots + 2 * kTcBuffers + 11];
+  __shared__ __align__(8) unsigned long long bars[2 * kTnMaxSlots + 2 * kTcMaxBuffers + 11];
   __shared__ unsigned tmem_base_s;
   __shared__ int dead_s;
   char* smem = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -439,8 +543,8 @@ __global__ void __launch_bounds__(kTnThreads, 1) gemm_tn_tc_kernel(const __grid_
   auto full = [&](int s) { return bar0 + 8 * s; };
   auto empty = [&](int s) { return bar0 + 8 * (kTnMaxSlots + s); };
   auto a_full = [&](int b) { return bar0 + 8 * (2 * kTnMaxSlots + b); };
-  auto a_empty = [&](int b) { return bar0 + 8 * (2 * kTnMaxSlots + kTcBuffers + b); };
-  const unsigned rest0 = bar0 + 8 * (2 * kTnMaxSlots + 2 * kTcBuffers);
+  auto a_empty = [&](int b) { return bar0 + 8 * (2 * kTnMaxSlots + kTcMaxBuffers + b); };
+  const unsigned rest0 = bar0 + 8 * (2 * kTnMaxSlots + 2 * kTcMaxBuffers);
   auto g_full = [&](int b) { return rest0 + 8 * b; };
   auto g_empty = [&](int b) { return rest0 + 8 * (2 + b); };
   auto b_full = [&](int b) { return rest0 + 8 * (4 + b); };
@@ -453,7 +557,7 @@ __global__ void __launch_bounds__(kTnThreads, 1) gemm_tn_tc_kernel(const __grid_
       mbar_init(full(s), 1);
       mbar_init(empty(s), 8);        // four warps for each half of the step
     }
-    for (int b = 0; b < kTcBuffers; ++b) {
+    for (int b = 0; b < kTcMaxBuffers; ++b) {
       mbar_init(a_full(b), 4);
       mbar_init(a_empty(b), 1);
     }
@@ -478,7 +582,7 @@ __global__ void __launch_bounds__(kTnThreads, 1) gemm_tn_tc_kernel(const __grid_
   __syncthreads();
   tc_fence_after();
   const unsigned tmem = tmem_base_s;
-  const unsigned a_col = 512 - kTcBuffers * kTcBufferCols;
+  const unsigned a_col = 512 - kTcMaxBuffers * kTcBufferCols;
   pdl_trigger();
   pdl_wait();
   const int s0 = static_cast<int>(a.steps * blockIdx.x / gridDim.x), s1 = static_cast<int>(a.steps * (blockIdx.x + 1) / gridDim.x);
@@ -537,7 +641,7 @@ __global__ void __launch_bounds__(kTnThreads, 1) gemm_tn_tc_kernel(const __grid_
             tc_mma_ts(d + 2 * NP, at + 32 + ks * 8, w + ks * 2, i1, 1u);
           }
           tc_commit(a_empty(b));
-          if (++b == kTcBuffers) { b = 0; aph ^= 1; }
+          if (++b == kTcMaxBuffers) { b = 0; aph ^= 1; }
         }
         if (ok) tc_commit(b_empty(i & 1));
         if (ok && (run + 1 == kTnRun || i + 1 == count)) tc_commit(acc_full);
@@ -552,7 +656,7 @@ __global__ void __launch_bounds__(kTnThreads, 1) gemm_tn_tc_kernel(const __grid_
     const unsigned dst = tmem + (static_cast<unsigned>(quad * 32) << 16) + a_col + grp * kTcBufferCols;
     const int units = count * 2 * MT;
     unsigned bph = 1;
-    for (int u = grp; u < units; u += kTcBuffers) {
+    for (int u = grp; u < units; u += kTcMaxBuffers) {
       const int q = u >> 1, s = q % S;
       // (a slot's phase is known by its parity alone: the slots before it must have been multiplied, S >= 2)
       if (!mbar_wait(a_empty(grp), bph, dead)) break;
@@ -677,7 +781,7 @@ static bool encode_rows(CUtensorMap* map, const float* X, int64_t n, int K, int6
 static int tc_columns(int K, int N, int epilogue) {
   const int fit = kTcMaxW / ((K + 63) / 64 * 3 * 128) / 16 * 16;
   int np = (N + 15) / 16 * 16;
-  if (epilogue == CAGNET_EPI_LOG_SOFTMAX || epilogue == CAGNET_EPI_LOG_SOFTMAX_256)
+  if (epilogue == CAGNET_EPI_LOG_SOFTMAX || epilogue == CAGNET_EPI_LOG_SOFTMAX_256 || epilogue == kEpiNll)
     return (np <= 80 || (np <= 256 && K <= 64)) && np <= fit && (K <= 320 || np <= 48) ? np : 0;
   const int most = min(fit, K > 320 ? 48 : (K > 64 ? 80 : 160));
   // at most 160 columns, so that two sets of sums fit and one tile's stores run under the next one's products
@@ -714,12 +818,13 @@ static cudaError_t launch_tc_epilogue(int epilogue, dim3 grid, size_t smem, cuda
     case CAGNET_EPI_RELU: return launch_tc<SETS, CAGNET_EPI_RELU>(grid, smem, s, map, a);
     case CAGNET_EPI_RELU_MASK: return launch_tc<SETS, CAGNET_EPI_RELU_MASK>(grid, smem, s, map, a);
     case CAGNET_EPI_ACCUMULATE: return launch_tc<SETS, CAGNET_EPI_ACCUMULATE>(grid, smem, s, map, a);
+    case kEpiNll: return launch_tc<SETS, kEpiNll>(grid, smem, s, map, a);
     default: return launch_tc<SETS, CAGNET_EPI_LOG_SOFTMAX>(grid, smem, s, map, a);
   }
 }
 
-int gemm_nn_tc(const float* X, int64_t ldx, const float* W, int64_t ldw, int transW, float* Z, int64_t ldz, int64_t n, int K, int N,
-               int epilogue, const float* aux, int64_t ldaux, cudaStream_t s) {
+static int run_nn_tc(const float* X, int64_t ldx, const float* W, int64_t ldw, int transW, float* Z, int64_t ldz, int64_t n, int K, int N,
+                     int epilogue, const float* aux, int64_t ldaux, const TcLoss* loss, int32_t* parts, cudaStream_t s) {
   CUtensorMap map;
   if (!encode_rows(&map, X, n, K, ldx, 128, true)) return fail(CAGNET_E_LAUNCH, "cagnet_gemm_nn_f32: cannot describe X to the copy engine");
   TcArgs a;
@@ -727,21 +832,34 @@ int gemm_nn_tc(const float* X, int64_t ldx, const float* W, int64_t ldw, int tra
   a.ldw = ldw; a.ldz = ldz; a.ldaux = ldaux; a.n = n;
   a.transW = transW; a.K = K; a.N = N;
   a.NP = tc_columns(K, N, epilogue);
-  a.z_vec4 = (ldz % 4 == 0 && aligned(Z, 16)) ? 1 : 0;
+  a.loss = loss ? *loss : TcLoss{};
+  a.z_vec4 = (ldz % 4 == 0 && aligned(Z, 16) && (!loss || (loss->lddz % 4 == 0 && aligned(loss->dz, 16)))) ? 1 : 0;
   a.aux_vec4 = epilogue == CAGNET_EPI_RELU_MASK ? ldaux % 4 == 0 && aligned(aux, 16) : a.z_vec4;
   a.tiles = static_cast<int>((n + 127) / 128);
   const int wbytes = (K + 63) / 64 * 3 * a.NP * 128;
-  a.stages = min(kTcMaxStages, (kTcSmem - 1024 - kTcExchange - wbytes) / kXStageBytes);
-  const size_t smem = 1024 + static_cast<size_t>(a.stages) * kXStageBytes + wbytes + kTcExchange;
+  const int sets = K <= kTcLightK ? 0 : K > 320 ? 2 : 1, exchange = tc_exchange_bytes(sets, tc_reads_old(epilogue));
+  a.stages = min(kTcMaxStages, (kTcSmem - 1024 - exchange - wbytes) / kXStageBytes);
+  const size_t smem = 1024 + static_cast<size_t>(a.stages) * kXStageBytes + wbytes + exchange;
   const dim3 grid(a.tiles < kNumSMs ? a.tiles : kNumSMs, (N + a.NP - 1) / a.NP);
-  const cudaError_t e = a.NP > 80 ? launch_tc_epilogue<0>(epilogue, grid, smem, s, map, a)
-                        : K > 320 ? launch_tc_epilogue<2>(epilogue, grid, smem, s, map, a)
-                                  : launch_tc_epilogue<1>(epilogue, grid, smem, s, map, a);
+  if (parts) *parts = static_cast<int32_t>(grid.x) * tc_storing_warps(sets);
+  const cudaError_t e = sets == 0   ? launch_tc_epilogue<0>(epilogue, grid, smem, s, map, a)
+                        : sets == 2 ? launch_tc_epilogue<2>(epilogue, grid, smem, s, map, a)
+                                    : launch_tc_epilogue<1>(epilogue, grid, smem, s, map, a);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(CAGNET_E_LAUNCH, "cagnet_gemm_nn_f32: CUDA launch failed: %s", cudaGetErrorString(e));
   }
   return CAGNET_OK;
+}
+
+int gemm_nn_tc(const float* X, int64_t ldx, const float* W, int64_t ldw, int transW, float* Z, int64_t ldz, int64_t n, int K, int N,
+               int epilogue, const float* aux, int64_t ldaux, cudaStream_t s) {
+  return run_nn_tc(X, ldx, W, ldw, transW, Z, ldz, n, K, N, epilogue, aux, ldaux, nullptr, nullptr, s);
+}
+
+int gemm_nn_tc_nll(const float* X, int64_t ldx, const float* W, int64_t ldw, float* Z, int64_t ldz, int64_t n, int K, int N, const TcLoss& loss,
+                   int32_t* parts, cudaStream_t s) {
+  return run_nn_tc(X, ldx, W, ldw, 0, Z, ldz, n, K, N, kEpiNll, nullptr, 0, &loss, parts, s);
 }
 
 // Shape of A^T . B on this kernel: NP columns of B per block (three sums each), MT column tiles of A per block.

@@ -214,11 +214,11 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
     check(cagnet_gemm_nn_f32(X, ld, W.data_ptr<float>(), W.size(1), transposed, Z.p(), Z.ld, n, K, N, epi, aux, ldaux, s), "gemm_nn");
     ++launches;
   };
-  // out = act(Z W) with the activation fused where the product's epilogue has it
+  // out = act(Z W) with the activation fused where the product's epilogue has it; log-softmax of up to 256 columns comes with the
+  // loss (below)
   auto dense_layer = [&](const float* X, int64_t ld, const at::Tensor& W, const Buffer& Z, int32_t K, int32_t N, bool last) {
     if (!activations) return gemm(X, ld, W, false, Z, K, N, CAGNET_EPI_NONE, nullptr, 0);
     if (!last) return gemm(X, ld, W, false, Z, K, N, CAGNET_EPI_RELU, nullptr, 0);
-    if (N <= 256) return gemm(X, ld, W, false, Z, K, N, N <= 64 ? CAGNET_EPI_LOG_SOFTMAX : CAGNET_EPI_LOG_SOFTMAX_256, nullptr, 0);
     gemm(X, ld, W, false, Z, K, N, CAGNET_EPI_NONE, nullptr, 0);
     check(cagnet_log_softmax_fwd_f32(Z.p(), Z.ld, Z.p(), Z.ld, n, N, s), "log_softmax");
     ++launches;
@@ -247,6 +247,13 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
     dense_layer(z.p(), z.ld, w1, H, f, h, false);
     if (widen1) agg1 = z;
   }
+  at::Tensor loss = at::empty({}, o);
+  const size_t loss_bytes = cagnet_nll_workspace_bytes(n);
+  float* loss_ws = static_cast<float*>(scratch.bytes(loss_bytes));
+  Buffer dz(scratch, n, c);
+  int32_t parts = 0;
+  const auto* mask8 = static_cast<const uint8_t*>(mask.data_ptr());
+  bool loss_done = false;
   const at::Tensor out_t = at::empty({std::max<int64_t>(n, 1), pad_ld(c)}, o);
   const Buffer out(out_t);
   if (narrow2) {
@@ -260,23 +267,26 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
   } else {
     Buffer z(scratch, n, h);
     product(A, H.p(), H.ld, z, h);
-    dense_layer(z.p(), z.ld, w2, out, h, c, true);
+    if (activations && c <= 256) {                  // with the loss and its gradient
+      int32_t kernels = 0;
+      check(cagnet_gemm_nll_f32(z.p(), z.ld, w2.data_ptr<float>(), c, n, h, c, y.data_ptr<int64_t>(), mask8, static_cast<int32_t>(cls_lo),
+                                static_cast<int32_t>(cls_hi), static_cast<float>(count), out.p(), out.ld, dz.p(), dz.ld, &parts, &kernels,
+                                loss_ws, loss_bytes, s), "gemm_nll");
+      launches += kernels;
+      loss_done = true;
+    } else {
+      dense_layer(z.p(), z.ld, w2, out, h, c, true);
+    }
     if (widen2) agg2 = z;
   }
 
   // ---- loss, and its gradient before the second activation
-  at::Tensor loss = at::empty({}, o);
-  const size_t loss_bytes = cagnet_nll_workspace_bytes(n);
-  float* loss_ws = static_cast<float*>(scratch.bytes(loss_bytes));
-  Buffer dz(scratch, n, c);
-  int32_t parts = 0;
-  const auto* mask8 = static_cast<const uint8_t*>(mask.data_ptr());
-  if (activations) {
+  if (activations && !loss_done) {
     check(cagnet_nll_softmax_bwd_f32(out.p(), out.ld, y.data_ptr<int64_t>(), mask8, n, c, static_cast<int32_t>(cls_lo),
                                      static_cast<int32_t>(cls_hi), static_cast<float>(count), dz.p(), dz.ld, &parts,
                                      loss_ws, loss_bytes, s), "nll_softmax_bwd");
     ++launches;
-  } else {
+  } else if (!activations) {
     check(cagnet_nll_masked_f32(out.p(), out.ld, y.data_ptr<int64_t>(), mask8, n, c, static_cast<int32_t>(cls_lo),
                                 static_cast<int32_t>(cls_hi), static_cast<float>(count), 1.f, loss.data_ptr<float>(), dz.p(), dz.ld,
                                 loss_ws, loss_bytes, s), "nll_masked");

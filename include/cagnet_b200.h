@@ -344,6 +344,11 @@ int cagnet_nll_softmax_bwd_f32(const float* logp, int64_t ldl, const int64_t* y,
                                int32_t cls_lo, int32_t cls_hi, float count, float* dz, int64_t lddz, int32_t* parts,
                                void* ws, size_t ws_bytes, void* stream);
 
+/* ---- logp = log_softmax(X . W) (N <= 256) followed by cagnet_nll_softmax_bwd_f32 on it; *launches (host): kernels launched. */
+int cagnet_gemm_nll_f32(const float* X, int64_t ldx, const float* W, int64_t ldw, int64_t n, int32_t K, int32_t N, const int64_t* y,
+                        const uint8_t* mask, int32_t cls_lo, int32_t cls_hi, float count, float* logp, int64_t ldl, float* dz,
+                        int64_t lddz, int32_t* parts, int32_t* launches, void* ws, size_t ws_bytes, void* stream);
+
 /* ---- The end of an epoch in one launch: both weight gradients g1, g2 (contiguous) from the partial products that
  * cagnet_gemm_tn_partials_f32 left, one Adam step (torch.optim.Adam with default options; `step` counts from 1) on the
  * weights p1, p2 unless they are NULL, and with loss != NULL *loss = -sum(loss_parts[0 .. parts)) / count.

@@ -181,3 +181,30 @@ def test_tensor_core_products(n, K, N):
     close(grad, X.double().t() @ Z0.double())
     assert torch.equal(grad, ops.gemm_tn(Xd, Gd))
     assert _native.lib().cagnet_tile_core_error() == 0
+
+
+@pytest.mark.parametrize("n,K,N,lo", [(70, 12, 7, 0), (60001, 16, 41, 0), (60001, 40, 64, 3), (40003, 100, 30, 0), (40003, 16, 97, 0), (40003, 64, 256, 5)])
+def test_product_with_loss(n, K, N, lo):
+    """log_softmax(X.W), its masked NLL and the gradient before the log-softmax from one call, against fp64."""
+    import ctypes
+    L, g, hi = _native.lib(), torch.Generator(device="cuda").manual_seed(n + N), lo + N - 1
+    X, W = torch.randn(n, K, generator=g, device="cuda"), torch.randn(K, N, generator=g, device="cuda")
+    y = torch.randint(0, hi + 3, (n,), generator=g, device="cuda")
+    mask = torch.rand(n, generator=g, device="cuda") < 0.6
+    want = torch.log_softmax(X.double() @ W.double(), dim=1)
+    hit = mask & (y >= lo) & (y < hi)
+    grad = want.exp()
+    grad[hit, (y - lo)[hit]] -= 1
+    grad = torch.where(hit[:, None], grad / n, torch.zeros_like(grad))
+    ws, parts, launches = torch.zeros(L.cagnet_nll_workspace_bytes(n) // 4, device="cuda"), ctypes.c_int32(), ctypes.c_int32()
+    for make in (ops.empty_padded, lambda n, N, d: torch.full((n, N + 1), 7.0, device=d)[:, 1:]):         # rows on 16 bytes, and not
+        logp, dz = make(n, N, "cuda"), make(n, N, "cuda")
+        Xd = ops.to_padded(X)
+        _native.check(L.cagnet_gemm_nll_f32(Xd.data_ptr(), Xd.stride(0), W.data_ptr(), N, n, K, N, y.data_ptr(), mask.data_ptr(), lo, hi,
+                                            float(n), logp.data_ptr(), logp.stride(0), dz.data_ptr(), dz.stride(0), ctypes.byref(parts),
+                                            ctypes.byref(launches), ws.data_ptr(), ws.numel() * 4, None))
+        assert float((logp.double() - want).norm()) <= 1e-6 * float(want.norm())
+        assert float((dz.double() - grad).norm()) <= 1e-6 * float(grad.norm())
+        total = want[hit, (y - lo)[hit]].sum()
+        assert abs(float(ws[:parts.value].double().sum() - total)) <= 1e-6 * abs(float(total))
+    assert launches.value == (1 if n > 1000 else 2) and L.cagnet_tile_core_error() == 0
