@@ -260,7 +260,13 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
     Buffer hw(scratch, n, c);
     gemm(H.p(), H.ld, w2, false, hw, h, c, CAGNET_EPI_NONE, nullptr, 0);
     product(A, hw.p(), hw.ld, out, c);
-    if (activations) {
+    if (activations && c <= 256) {
+      check(cagnet_log_softmax_nll_f32(out.p(), out.ld, n, c, y.data_ptr<int64_t>(), mask8, static_cast<int32_t>(cls_lo),
+                                       static_cast<int32_t>(cls_hi), static_cast<float>(count), out.p(), out.ld, dz.p(), dz.ld, &parts,
+                                       loss_ws, loss_bytes, s), "log_softmax_nll");
+      ++launches;
+      loss_done = true;
+    } else if (activations) {
       check(cagnet_log_softmax_fwd_f32(out.p(), out.ld, out.p(), out.ld, n, c, s), "log_softmax");
       ++launches;
     }

@@ -353,14 +353,14 @@ struct SplitShape {
 // Chunk length: the launch is a whole number of full waves, a wave being what the SMs hold.  All chunks take about as long,
 // so a wave that is filled to its last block ends together and one block more costs a whole wave (22.6 M nonzeros, width
 // 16: chunks of 512 end in a wave of 6 % at 216 us; chunks of 704, one wave, 174 us; of 600 on seven blocks per SM 162).
-// Chunks stay under 704 nonzeros (more waves beyond) and not under 32 (0.5 M nonzeros, width 16: 15.4 us with 16, 12.5 with
+// Chunks stay under 704 nonzeros, 1,024 for narrow rows (more waves beyond: 23.6 M nonzeros, width 16: one wave 144 us, two 170) and not under 32 (0.5 M nonzeros, width 16: 15.4 us with 16, 12.5 with
 // 32, 13.9 with 48), and are longer only where the pieces would need more than half a gigabyte.  A B beyond L2 takes a wave
 // for every 64 MB, at most one per feature tile: waves go tile by tile, so each gathers from columns that stay in L2 (1 M
 // nonzeros in even rows, B of 200 MB, 4 tiles: one wave 224 us, four 170).
 static SplitShape split_shape(int64_t nnz, int m, int f, bool coo, bool even) {
-  constexpr int kLongest = 704, kShortest = 32;
   SplitShape s;
   const int v = (f + 3) / 4;
+  const int longest = v <= 8 ? 1024 : 704, shortest = 32;
   s.lpn = v <= 4 ? 4 : 8;
   s.nv = 1;
   if (v > 8 && nnz >= (v <= 16 ? 500000 : 150000)) {
@@ -376,13 +376,13 @@ static SplitShape split_shape(int64_t nnz, int m, int f, bool coo, bool even) {
   s.tiles = (v + tile - 1) / tile;
   const int unit = 2 * s.lpn, per_block = kSplitWarps * (32 / s.lpn);
   const int64_t slots = static_cast<int64_t>(kNumSMs) * split_blocks_per_sm(s.nv, coo);        // blocks of a wave
-  int64_t waves = (nnz * s.tiles + slots * per_block * kLongest - 1) / (slots * per_block * kLongest);
+  int64_t waves = (nnz * s.tiles + slots * per_block * longest - 1) / (slots * per_block * longest);
   const int64_t parts = (static_cast<int64_t>(m) * f * 4 + (64 << 20) - 1) >> 26;
   waves = max(waves, min(static_cast<int64_t>(s.tiles), parts));
   while (waves * slots < s.tiles) ++waves;
   const int64_t walks = waves * slots / s.tiles * per_block;                                    // chunks of a feature tile
   int64_t chunk = (nnz + walks - 1) / walks;
-  chunk = ((chunk < kShortest ? kShortest : chunk) + unit - 1) / unit * unit;
+  chunk = ((chunk < shortest ? shortest : chunk) + unit - 1) / unit * unit;
   while ((nnz + chunk - 1) / chunk * s.tiles * tile * 32 > (512ll << 20)) chunk *= 2;
   s.chunk = static_cast<int>(chunk);
   s.nchunks = (nnz + chunk - 1) / chunk;

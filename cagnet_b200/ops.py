@@ -152,11 +152,13 @@ def _row_major(t):
 # "tiles": such a block is cut into dense TILES instead (tile_plan.py, csrc/tile_core.cu: one bit per cell, a staircase of
 # 256 x 64 tiles of at least "density_int" among the "tile_side" highest-degree rows and columns), which take over more of
 # the nonzeros at a sixteenth of the memory and pay at every width; "tile_nnz": fewest nonzeros in tiles worth a plan;
+# (2.5 %: a 64-column tile product and a gathered nonzero break even near 360 nonzeros = 2.2 %, the largest gain is at 233K
+# vertices, width 602: 6.51 ms at 2 %, 6.28 at 2.5, 6.67 at 3);
 # "tile_work": a product uses the tiles from this many gathered floats on (nonzeros in tiles x width; 0 with "min_share" 0).
 CORE = {"enabled": os.environ.get("CAGNET_DENSE_CORE", "1") != "0", "density": 0.2, "density_tc": 0.09, "step": 1024,
         "max_side": 16384, "max_bytes": 2 << 30, "min_share": 0.1, "min_width": 128, "rounds": 1,
         "tensor_cores": os.environ.get("CAGNET_CORE_TENSOR", "1") != "0",
-        "integer": os.environ.get("CAGNET_CORE_INTEGER", "1") != "0", "density_int": 0.02, "max_side_int": 32768,
+        "integer": os.environ.get("CAGNET_CORE_INTEGER", "1") != "0", "density_int": 0.025, "max_side_int": 32768,
         "min_width_int": 128, "min_row_nnz": 64, "tiles": os.environ.get("CAGNET_DENSE_TILES", "1") != "0",
         "tile_side": 1 << 18, "tile_nnz": 100000, "tile_work": 80000000}
 

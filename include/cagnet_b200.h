@@ -344,6 +344,11 @@ int cagnet_nll_softmax_bwd_f32(const float* logp, int64_t ldl, const int64_t* y,
                                int32_t cls_lo, int32_t cls_hi, float count, float* dz, int64_t lddz, int32_t* parts,
                                void* ws, size_t ws_bytes, void* stream);
 
+/* ---- logp = log_softmax(z) (N <= 256; logp may be z) followed by cagnet_nll_softmax_bwd_f32 on it, in one pass. */
+int cagnet_log_softmax_nll_f32(const float* z, int64_t ldz, int64_t n, int32_t N, const int64_t* y, const uint8_t* mask, int32_t cls_lo,
+                               int32_t cls_hi, float count, float* logp, int64_t ldl, float* dz, int64_t lddz, int32_t* parts, void* ws,
+                               size_t ws_bytes, void* stream);
+
 /* ---- logp = log_softmax(X . W) (N <= 256) followed by cagnet_nll_softmax_bwd_f32 on it; *launches (host): kernels launched. */
 int cagnet_gemm_nll_f32(const float* X, int64_t ldx, const float* W, int64_t ldw, int64_t n, int32_t K, int32_t N, const int64_t* y,
                         const uint8_t* mask, int32_t cls_lo, int32_t cls_hi, float count, float* logp, int64_t ldl, float* dz,

@@ -207,4 +207,12 @@ def test_product_with_loss(n, K, N, lo):
         assert float((dz.double() - grad).norm()) <= 1e-6 * float(grad.norm())
         total = want[hit, (y - lo)[hit]].sum()
         assert abs(float(ws[:parts.value].double().sum() - total)) <= 1e-6 * abs(float(total))
+        z = make(n, N, "cuda").copy_(X @ W)                                   # the same from the logits, in place
+        dz.fill_(9.0)
+        _native.check(L.cagnet_log_softmax_nll_f32(z.data_ptr(), z.stride(0), n, N, y.data_ptr(), mask.data_ptr(), lo, hi, float(n),
+                                                   z.data_ptr(), z.stride(0), dz.data_ptr(), dz.stride(0), ctypes.byref(parts),
+                                                   ws.data_ptr(), ws.numel() * 4, None))
+        assert float((z.double() - want).norm()) <= 1e-6 * float(want.norm())
+        assert float((dz.double() - grad).norm()) <= 1e-6 * float(grad.norm())
+        assert abs(float(ws[:parts.value].double().sum() - total)) <= 1e-6 * abs(float(total))
     assert launches.value == (1 if n > 1000 else 2) and L.cagnet_tile_core_error() == 0
