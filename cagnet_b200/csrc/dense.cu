@@ -28,6 +28,7 @@ struct GemmArgs {
   float* Z;
   int64_t ldx, ldw, ldz, ldaux, n;
   int transW, K, N, epilogue, x_vec4, z_vec4;
+  TcLoss loss;
 };
 
 // 4 consecutive k of row gr (zeros outside the matrix)
@@ -129,7 +130,9 @@ __device__ __forceinline__ float row_lse(const float (&v)[COLS], const bool (&li
   return mx + logf(sum);
 }
 
-template <int LC, int NP, int TM, int WARPS, int BK>
+// NLL: log-softmax with its masked NLL and the gradient before the log-softmax, as the tensor-core kernel writes them (a kernel of
+// 2.4 us and its launch less per epoch of 16 K vertices).
+template <int LC, int NP, int TM, int WARPS, int BK, bool NLL>
 __global__ void __launch_bounds__(WARPS * 32) gemm_nn_kernel(GemmArgs a) {
   constexpr int BN = LC * 4 * NP, WR = 32 / LC * TM, BM = WARPS * WR, T = WARPS * 32;
   constexpr int XV = BM * BK / 4 / T;            // float4 of X per thread and tile
@@ -189,10 +192,11 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_nn_kernel(GemmArgs a) {
     __syncthreads();
   }
 
+  [[maybe_unused]] float picked = 0.f;
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
     const int64_t gr = row0 + r0 + i;            // no early exit: the shuffles need all lanes
-    if (a.epilogue == CAGNET_EPI_LOG_SOFTMAX || a.epilogue == CAGNET_EPI_LOG_SOFTMAX_256) {
+    if (NLL || a.epilogue == CAGNET_EPI_LOG_SOFTMAX || a.epilogue == CAGNET_EPI_LOG_SOFTMAX_256) {
       float v[NP * 4];
       bool live[NP * 4];
 #pragma unroll
@@ -212,6 +216,47 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_nn_kernel(GemmArgs a) {
 #pragma unroll
       for (int p = 0; p < NP; ++p)
         store_z4(a, gr, n0 + p * (LC * 4) + lc * 4, make_float4(acc[i][p][0], acc[i][p][1], acc[i][p][2], acc[i][p][3]));
+      if constexpr (NLL) {
+        int at = -1;
+        if (a.loss.mask[gr]) {
+          const int64_t label = a.loss.y[gr];
+          if (label >= a.loss.cls_lo && label < a.loss.cls_hi) at = static_cast<int>(label - a.loss.cls_lo);
+        }
+        const float w = a.loss.inv_count;
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          const int c = p * (LC * 4) + lc * 4;
+          float g[4] = {0.f, 0.f, 0.f, 0.f};
+          if (at >= 0) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              g[j] = (c + j == at ? -w : 0.f) + expf(acc[i][p][j]) * w;
+              if (c + j == at) picked += acc[i][p][j];
+            }
+          }
+          float* d = a.loss.dz + gr * a.loss.lddz + c;
+          if (c + 4 <= a.N && a.z_vec4) {
+            *reinterpret_cast<float4*>(d) = make_float4(g[0], g[1], g[2], g[3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (c + j < a.N) d[j] = g[j];
+          }
+        }
+      }
+    }
+  }
+  if constexpr (NLL) {
+    __shared__ float red[WARPS];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) picked += __shfl_xor_sync(0xffffffffu, picked, off);
+    if (lane == 0) red[warp] = picked;
+    __syncthreads();
+    if (tid == 0) {
+      float t = red[0];
+#pragma unroll
+      for (int w = 1; w < WARPS; ++w) t += red[w];
+      a.loss.parts[blockIdx.x] = t;
     }
   }
 }
@@ -414,17 +459,29 @@ __device__ __forceinline__ void cp_async16(float* smem_dst, const float* gmem_sr
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(gmem_src), "r"(src_bytes) : "memory");
 }
 
-__global__ void __launch_bounds__(256, 2) gemm_tn_small_kernel(const float* __restrict__ H, int64_t ldh,
-                                                               const float* __restrict__ G, int64_t ldg, int64_t n,
-                                                               int K, int N, int64_t rows_per_chunk,
-                                                               float* __restrict__ ws) {
+struct TnSmallArgs {
+  const float *H, *G;
+  float* ws;
+  int64_t ldh, ldg, rows_per_chunk;
+  int K, N, chunks, ktiles;            // chunks * ktiles blocks
+};
+// One product, or both weight gradients of a small epoch at a time (the blocks of the second behind those of the first: each fills a
+// fraction of the chip, and a launch costs as much as either, 5 us at 16 K vertices).
+__global__ void __launch_bounds__(256, 2) gemm_tn_small_kernel(TnSmallArgs first, TnSmallArgs second, int64_t n) {
   extern __shared__ __align__(16) float tn_smem[];
   pdl_trigger();
   pdl_wait();
+  const bool other = blockIdx.x >= first.chunks * first.ktiles;
+  const TnSmallArgs& a = other ? second : first;
+  const int blk = blockIdx.x - (other ? first.chunks * first.ktiles : 0);
+  const float *__restrict__ H = a.H, *__restrict__ G = a.G;
+  float* __restrict__ ws = a.ws;
+  const int64_t ldh = a.ldh, ldg = a.ldg, rows_per_chunk = a.rows_per_chunk;
+  const int K = a.K, N = a.N, chunk = blk % a.chunks;
   const int tid = threadIdx.x;
   const int kq = tid & 15, rs = tid >> 4;
-  const int k0 = blockIdx.y * kTnKT;
-  const int64_t r_begin = static_cast<int64_t>(blockIdx.x) * rows_per_chunk;
+  const int k0 = blk / a.chunks * kTnKT;
+  const int64_t r_begin = static_cast<int64_t>(chunk) * rows_per_chunk;
   const int64_t r_end = min(n, r_begin + rows_per_chunk);
   const int steps = static_cast<int>((r_end - r_begin + kTnSmallRB - 1) / kTnSmallRB);
 
@@ -502,7 +559,7 @@ __global__ void __launch_bounds__(256, 2) gemm_tn_small_kernel(const float* __re
             make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
   }
   __syncthreads();
-  float* wp = ws + static_cast<int64_t>(blockIdx.x) * K * N;
+  float* wp = ws + static_cast<int64_t>(chunk) * K * N;
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const int e = tid + 256 * u;                  // element of the 64 x 16 tile: k = e / 16, column j = e % 16
@@ -956,6 +1013,45 @@ static int elementwise_blocks(int64_t total) {
 
 using namespace cagnet;
 
+// Row tiles are as tall as W is narrow (8 rows per thread); below about two tiles per SM, with a K worth splitting, the warps of
+// a block share its rows and split K instead.
+static bool gemm_splits_k(int64_t n, int K, int N, int epilogue) {
+  return N <= 64 && K >= 64 && n < 40000 && epilogue != CAGNET_EPI_LOG_SOFTMAX_256;
+}
+static int gemm_fma_rows(int64_t n, int N) {
+  if (N <= 16) return n < 20000 ? 64 : n < 160000 ? 128 : 256;
+  if (N <= 32) return n < 80000 ? 32 : 128;
+  return N <= 64 ? 128 : 64;
+}
+template <bool NLL>
+static cudaError_t launch_gemm_fma(const GemmArgs& a, cudaStream_t s) {
+  const int64_t n = a.n;
+  const int N = a.N;
+  auto rows = [&](int bm) { return dim3(static_cast<unsigned>((n + bm - 1) / bm), 1); };
+  if constexpr (!NLL) {
+    if (gemm_splits_k(n, a.K, N, a.epilogue)) {
+      if (N <= 16) return launch_pdl(gemm_nn_splitk_kernel<4, 2>, rows(16), dim3(256), 0, s, a);
+      if (N <= 32) return launch_pdl(gemm_nn_splitk_kernel<8, 4>, rows(16), dim3(256), 0, s, a);
+      return launch_pdl(gemm_nn_splitk_kernel<16, 8>, rows(16), dim3(256), 0, s, a);
+    }
+  }
+  const int bm = gemm_fma_rows(n, N);
+  if (N <= 16) {
+    if (bm == 64) return launch_pdl(gemm_nn_kernel<4, 1, 2, 4, 32, NLL>, rows(bm), dim3(128), 0, s, a);
+    if (bm == 128) return launch_pdl(gemm_nn_kernel<4, 1, 4, 4, 32, NLL>, rows(bm), dim3(128), 0, s, a);
+    return launch_pdl(gemm_nn_kernel<4, 1, 8, 4, 16, NLL>, rows(bm), dim3(128), 0, s, a);
+  }
+  if (N <= 32) {
+    if (bm == 32) return launch_pdl(gemm_nn_kernel<8, 1, 2, 4, 32, NLL>, rows(bm), dim3(128), 0, s, a);
+    return launch_pdl(gemm_nn_kernel<8, 1, 8, 4, 32, NLL>, rows(bm), dim3(128), 0, s, a);
+  }
+  if (N <= 64) return launch_pdl(gemm_nn_kernel<16, 1, 8, 8, 32, NLL>, rows(bm), dim3(256), 0, s, a);
+  if (N <= 128) return launch_pdl(gemm_nn_kernel<32, 1, 8, 8, 16, NLL>, rows(bm), dim3(256), 0, s, a);
+  dim3 grid = rows(bm);
+  grid.y = (N + 255) / 256;
+  return launch_pdl(gemm_nn_kernel<32, 2, 8, 8, 16, NLL>, grid, dim3(256), 0, s, a);
+}
+
 extern "C" int cagnet_gemm_nn_f32(const float* X, int64_t ldx, const float* W, int64_t ldw, int32_t transW, float* Z,
                                   int64_t ldz, int64_t n, int32_t K, int32_t N, int32_t epilogue, const float* aux,
                                   int64_t ldaux, void* stream) {
@@ -980,34 +1076,7 @@ extern "C" int cagnet_gemm_nn_f32(const float* X, int64_t ldx, const float* W, i
   a.transW = transW; a.K = K; a.N = N; a.epilogue = epilogue;
   a.x_vec4 = (ldx % 4 == 0 && aligned(X, 16)) ? 1 : 0;
   a.z_vec4 = (ldz % 4 == 0 && aligned(Z, 16)) ? 1 : 0;
-  // Row tiles are as tall as W is narrow (8 rows per thread); below about two tiles per SM, with a K worth splitting, the
-  // warps of a block share its rows and split K instead.
-  const bool splitk = N <= 64 && K >= 64 && n < 40000 && epilogue != CAGNET_EPI_LOG_SOFTMAX_256;
-  auto rows = [&](int bm) { return dim3(static_cast<unsigned>((n + bm - 1) / bm), 1); };
-  cudaError_t e;
-  if (splitk) {
-    if (N <= 16) e = launch_pdl(gemm_nn_splitk_kernel<4, 2>, rows(16), dim3(256), 0, s, a);
-    else if (N <= 32) e = launch_pdl(gemm_nn_splitk_kernel<8, 4>, rows(16), dim3(256), 0, s, a);
-    else e = launch_pdl(gemm_nn_splitk_kernel<16, 8>, rows(16), dim3(256), 0, s, a);
-  } else if (N <= 16 && n < 20000) {
-    e = launch_pdl(gemm_nn_kernel<4, 1, 2, 4, 32>, rows(64), dim3(128), 0, s, a);
-  } else if (N <= 16 && n < 160000) {
-    e = launch_pdl(gemm_nn_kernel<4, 1, 4, 4, 32>, rows(128), dim3(128), 0, s, a);
-  } else if (N <= 16) {
-    e = launch_pdl(gemm_nn_kernel<4, 1, 8, 4, 16>, rows(256), dim3(128), 0, s, a);
-  } else if (N <= 32 && n < 80000) {
-    e = launch_pdl(gemm_nn_kernel<8, 1, 2, 4, 32>, rows(32), dim3(128), 0, s, a);
-  } else if (N <= 32) {
-    e = launch_pdl(gemm_nn_kernel<8, 1, 8, 4, 32>, rows(128), dim3(128), 0, s, a);
-  } else if (N <= 64) {
-    e = launch_pdl(gemm_nn_kernel<16, 1, 8, 8, 32>, rows(128), dim3(256), 0, s, a);
-  } else if (N <= 128) {
-    e = launch_pdl(gemm_nn_kernel<32, 1, 8, 8, 16>, rows(64), dim3(256), 0, s, a);
-  } else {
-    dim3 grid = rows(64);
-    grid.y = (N + 255) / 256;
-    e = launch_pdl(gemm_nn_kernel<32, 2, 8, 8, 16>, grid, dim3(256), 0, s, a);
-  }
+  const cudaError_t e = launch_gemm_fma<false>(a, s);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(CAGNET_E_LAUNCH, "cagnet_gemm_nn_f32: CUDA launch failed: %s", cudaGetErrorString(e));
@@ -1035,9 +1104,20 @@ static int tn_small_opt_in() {
   return CAGNET_OK;
 }
 
-// The partial products of H^T * G in ws, and what it takes to add them up.
+static int launch_tn_small(const TnSmallArgs& a, const TnSmallArgs& b, int64_t n, cudaStream_t s) {
+  if (int rc = tn_small_opt_in()) return rc;
+  const cudaError_t e = launch_pdl(gemm_tn_small_kernel, dim3(a.chunks * a.ktiles + b.chunks * b.ktiles), dim3(256), kTnSmallSmemBytes, s, a, b, n);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(CAGNET_E_LAUNCH, "cagnet_gemm_tn_f32: CUDA launch failed: %s", cudaGetErrorString(e));
+  }
+  return CAGNET_OK;
+}
+
+// The partial products of H^T * G in ws, and what it takes to add them up.  With `later` the narrow kernel is not launched but
+// its arguments are left there (later->chunks stays 0 where another kernel ran).
 static int tn_partials(const float* H, int64_t ldh, const float* G, int64_t ldg, int64_t n, int32_t K, int32_t N, void* ws,
-                       size_t ws_bytes, cagnet_tn_sum* sum, cudaStream_t s) {
+                       size_t ws_bytes, cagnet_tn_sum* sum, cudaStream_t s, TnSmallArgs* later = nullptr) {
   if (!ws || (n > 0 && (!H || !G))) return fail(CAGNET_E_ARG, "cagnet_gemm_tn_f32: null pointer");
   if (ldh < K || ldg < N) return fail(CAGNET_E_ALIGN, "cagnet_gemm_tn_f32: leading dimension too small");
   if (static_cast<int64_t>(K) * N > INT_MAX) return fail(CAGNET_E_OVERFLOW, "cagnet_gemm_tn_f32: K*N exceeds int32");
@@ -1066,13 +1146,15 @@ static int tn_partials(const float* H, int64_t ldh, const float* G, int64_t ldg,
   sum->transposed = swap ? 1 : 0;
   cudaError_t e;
   if (small) {
-    if (int rc = tn_small_opt_in()) return rc;
-    e = launch_pdl(gemm_tn_small_kernel, dim3(sh.chunks, sh.ktiles), dim3(256), kTnSmallSmemBytes, s, H, ldh, G, ldg, n, K, N,
-                   sh.rows_per_chunk, partials);
-  } else {
-    e = launch_pdl(gemm_tn_partial_kernel, dim3(sh.chunks, sh.ktiles, sh.ntiles), dim3(256), 0, s, H, ldh, G, ldg, n, K, N,
-                   sh.rows_per_chunk, partials);
+    const TnSmallArgs a{H, G, partials, ldh, ldg, sh.rows_per_chunk, K, N, sh.chunks, sh.ktiles};
+    if (later) {
+      *later = a;
+      return CAGNET_OK;
+    }
+    return launch_tn_small(a, TnSmallArgs{}, n, s);
   }
+  e = launch_pdl(gemm_tn_partial_kernel, dim3(sh.chunks, sh.ktiles, sh.ntiles), dim3(256), 0, s, H, ldh, G, ldg, n, K, N,
+                 sh.rows_per_chunk, partials);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(CAGNET_E_LAUNCH, "cagnet_gemm_tn_f32: CUDA launch failed: %s", cudaGetErrorString(e));
@@ -1099,6 +1181,21 @@ extern "C" int cagnet_gemm_tn_partials_f32(const float* H, int64_t ldh, const fl
                                            void* ws, size_t ws_bytes, cagnet_tn_sum* sum, void* stream) {
   if (n < 0 || K <= 0 || N <= 0 || !sum) return fail(CAGNET_E_ARG, "cagnet_gemm_tn_partials_f32: bad argument");
   return tn_partials(H, ldh, G, ldg, n, K, N, ws, ws_bytes, sum, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int cagnet_gemm_tn_partials2_f32(const cagnet_tn_product* p, cagnet_tn_sum* sum, int64_t n, int32_t* launches, void* stream) {
+  if (n < 0 || !p || !sum || !launches || p[0].K <= 0 || p[0].N <= 0 || p[1].K <= 0 || p[1].N <= 0)
+    return fail(CAGNET_E_ARG, "cagnet_gemm_tn_partials2_f32: bad argument");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  TnSmallArgs later[2] = {};
+  *launches = 0;
+  for (int i = 0; i < 2; ++i) {
+    if (int rc = tn_partials(p[i].H, p[i].ldh, p[i].G, p[i].ldg, n, p[i].K, p[i].N, p[i].ws, p[i].ws_bytes, sum + i, s, later + i)) return rc;
+    *launches += later[i].chunks == 0;
+  }
+  if (later[0].chunks == 0 && later[1].chunks == 0) return CAGNET_OK;
+  ++*launches;
+  return later[0].chunks ? launch_tn_small(later[0], later[1], n, s) : launch_tn_small(later[1], TnSmallArgs{}, n, s);
 }
 
 extern "C" int cagnet_relu_fwd_f32(const float* z, int64_t ldz, float* h, int64_t ldh, int64_t n, int32_t N,
@@ -1247,7 +1344,7 @@ extern "C" int cagnet_log_softmax_nll_f32(const float* z, int64_t ldz, int64_t n
   const int vecs = (N + 3) / 4;
   auto run = [&](auto kernel, int lanes) {
     const int64_t blocks = max(static_cast<int64_t>(1), (n + 256 / lanes - 1) / (256 / lanes));
-    *parts = static_cast<int32_t>(min(blocks, static_cast<int64_t>(kNllBlocks)));
+    *parts = static_cast<int32_t>(min(blocks, static_cast<int64_t>(kTcLossParts)));
     launch_pdl(kernel, dim3(*parts), dim3(256), 0, s, z, ldz, logp, ldl, y, mask, n, N, cls_lo, cls_hi, 1.f / count, dz, lddz,
                static_cast<float*>(ws), vec4);
   };
@@ -1259,8 +1356,8 @@ extern "C" int cagnet_log_softmax_nll_f32(const float* z, int64_t ldz, int64_t n
   return check_launch("cagnet_log_softmax_nll_f32");
 }
 
-// One launch where the product runs on the tensor cores (its epilogue has every row's log-probabilities at hand: 700K x 256 classes
-// 596 us for the two, of which 110 us to read them back), two elsewhere.
+// One launch where one block has whole rows (on the tensor cores the epilogue has every row's log-probabilities at hand: 700K x 256 classes
+// 596 us for the two, of which 110 us to read them back), two where K is split.
 extern "C" int cagnet_gemm_nll_f32(const float* X, int64_t ldx, const float* W, int64_t ldw, int64_t n, int32_t K, int32_t N,
                                    const int64_t* y, const uint8_t* mask, int32_t cls_lo, int32_t cls_hi, float count, float* logp,
                                    int64_t ldl, float* dz, int64_t lddz, int32_t* parts, int32_t* launches, void* ws, size_t ws_bytes,
@@ -1275,6 +1372,20 @@ extern "C" int cagnet_gemm_nll_f32(const float* X, int64_t ldx, const float* W, 
     *launches = 1;
     const TcLoss loss{y, mask, dz, static_cast<float*>(ws), lddz, cls_lo, cls_hi, 1.f / count};
     return gemm_nn_tc_nll(X, ldx, W, ldw, logp, ldl, n, K, N, loss, parts, static_cast<cudaStream_t>(stream));
+  }
+  const int64_t blocks = (n + gemm_fma_rows(n, N) - 1) / gemm_fma_rows(n, N);
+  if (n > 0 && blocks <= kTcLossParts && !gemm_splits_k(n, K, N, epilogue)) {
+    GemmArgs a = {};
+    a.X = X; a.W = W; a.Z = logp;
+    a.ldx = ldx; a.ldw = ldw; a.ldz = ldl; a.n = n;
+    a.K = K; a.N = N; a.epilogue = epilogue;
+    a.x_vec4 = (ldx % 4 == 0 && aligned(X, 16)) ? 1 : 0;
+    a.z_vec4 = (ldl % 4 == 0 && lddz % 4 == 0 && aligned(logp, 16) && aligned(dz, 16)) ? 1 : 0;
+    a.loss = TcLoss{y, mask, dz, static_cast<float*>(ws), lddz, cls_lo, cls_hi, 1.f / count};
+    *launches = 1;
+    *parts = static_cast<int32_t>(blocks);
+    if (launch_gemm_fma<true>(a, static_cast<cudaStream_t>(stream)) != cudaSuccess) return check_launch("cagnet_gemm_nll_f32");
+    return CAGNET_OK;
   }
   *launches = 2;
   if (int rc = cagnet_gemm_nn_f32(X, ldx, W, ldw, 0, logp, ldl, n, K, N, epilogue, nullptr, 0, stream)) return rc;

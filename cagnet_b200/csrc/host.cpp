@@ -203,7 +203,8 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
   int64_t launches = 0;
   // One allocation for what a small epoch needs: its matrices (eight at most) and about as much again for workspaces.
   const int64_t floats = n * (pad_ld(f) + 4 * pad_ld(h) + 3 * pad_ld(c));
-  Scratch scratch(o, floats <= (2 << 20) ? static_cast<size_t>(floats) * 8 + (4 << 20) : 0);
+  const bool small = floats <= (8 << 20);
+  Scratch scratch(o, small ? static_cast<size_t>(floats) * 8 + (4 << 20) : 0);
   auto product = [&](const cagnet_block* b, const float* B, int64_t ldb, const Buffer& C, int32_t width) {
     if (!hook.is_none()) hook(true, b == At && b != A, width);
     launches += multiply(b, B, ldb, C.p(), C.ld, width, 0.f, scratch, s);
@@ -223,9 +224,17 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
     check(cagnet_log_softmax_fwd_f32(Z.p(), Z.ld, Z.p(), Z.ld, n, N, s), "log_softmax");
     ++launches;
   };
-  auto tn = [&](const float* H, int64_t ldh, const Buffer& G, int32_t K, int32_t N, cagnet_tn_sum& sum) {
+  // weight gradients as partial sums; a small epoch's wait for each other and go in one launch
+  std::array<cagnet_tn_sum, 2> sums;
+  std::array<cagnet_tn_product, 2> waiting = {};
+  auto tn = [&](int layer, const float* H, int64_t ldh, const Buffer& G, int32_t K, int32_t N) {
     const size_t bytes = cagnet_gemm_tn_workspace_bytes(n, K, N);
-    check(cagnet_gemm_tn_partials_f32(H, ldh, G.p(), G.ld, n, K, N, scratch.bytes(bytes), bytes, &sum, s), "gemm_tn");
+    void* ws = scratch.bytes(bytes);
+    if (small) {
+      waiting[layer] = {H, G.p(), ldh, G.ld, K, N, ws, bytes};
+      return;
+    }
+    check(cagnet_gemm_tn_partials_f32(H, ldh, G.p(), G.ld, n, K, N, ws, bytes, &sums[layer], s), "gemm_tn");
     ++launches;
   };
   const float* X = x.data_ptr<float>();
@@ -300,8 +309,7 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
   }
 
   // ---- backward: second layer
-  Buffer dh(scratch, n, h);         // gradient before the first activation
-  cagnet_tn_sum sum1, sum2;
+  Buffer dh(scratch, n, h), ag1, ag2;         // dh: gradient before the first activation
   const int mask_epi = activations ? CAGNET_EPI_RELU_MASK : CAGNET_EPI_NONE;
   if (widen2) {
     Buffer dzw(scratch, n, h);
@@ -311,20 +319,26 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
       check(cagnet_relu_bwd_f32(H.p(), H.ld, dh.p(), dh.ld, dh.p(), dh.ld, n, h, s), "relu_bwd");
       ++launches;
     }
-    tn(agg2.p(), agg2.ld, dz, h, c, sum2);
+    tn(1, agg2.p(), agg2.ld, dz, h, c);
   } else {
-    Buffer ag(scratch, n, c);
-    product(At, dz.p(), dz.ld, ag, c);
-    gemm(ag.p(), ag.ld, w2, true, dh, c, h, mask_epi, H.p(), H.ld);
-    tn(H.p(), H.ld, ag, h, c, sum2);
+    ag2 = Buffer(scratch, n, c);
+    product(At, dz.p(), dz.ld, ag2, c);
+    gemm(ag2.p(), ag2.ld, w2, true, dh, c, h, mask_epi, H.p(), H.ld);
+    tn(1, H.p(), H.ld, ag2, h, c);
+    if (!small) ag2 = Buffer();
   }
   // ---- backward: first layer
   if (widen1) {
-    tn(agg1.p(), agg1.ld, dh, f, h, sum1);
+    tn(0, agg1.p(), agg1.ld, dh, f, h);
   } else {
-    Buffer ag(scratch, n, h);
-    product(At, dh.p(), dh.ld, ag, h);
-    tn(X, ldx, ag, f, h, sum1);
+    ag1 = Buffer(scratch, n, h);
+    product(At, dh.p(), dh.ld, ag1, h);
+    tn(0, X, ldx, ag1, f, h);
+  }
+  if (small) {
+    int32_t kernels = 0;
+    check(cagnet_gemm_tn_partials2_f32(waiting.data(), sums.data(), n, &kernels, s), "gemm_tn");
+    launches += kernels;
   }
   // ---- gradients from their partial sums, Adam, loss
   at::Tensor g1 = at::empty({f, h}, o), g2 = at::empty({h, c}, o);
@@ -340,7 +354,7 @@ py::tuple epoch(uintptr_t fwd, uintptr_t bwd, const at::Tensor& x, const at::Ten
     adam->step1.unsafeGetTensorImpl()->bump_version();
     adam->step2.unsafeGetTensorImpl()->bump_version();
   }
-  check(cagnet_epoch_tail_f32(&sum1, g1.data_ptr<float>(), a[0], a[1], a[2], &sum2, g2.data_ptr<float>(), a[3], a[4], a[5],
+  check(cagnet_epoch_tail_f32(&sums[0], g1.data_ptr<float>(), a[0], a[1], a[2], &sums[1], g2.data_ptr<float>(), a[3], a[4], a[5],
                               adam ? adam->lr : 0., adam ? adam->beta1 : 0., adam ? adam->beta2 : 0., adam ? adam->eps : 0., step,
                               loss_ws, parts, static_cast<float>(count), activations ? loss.data_ptr<float>() : nullptr, s), "epoch_tail");
   ++launches;

@@ -347,7 +347,7 @@ struct SplitShape {
 // in L2) and four-vector ones out of small ones, which they cannot spread over the chip (0.6 M nonzeros, width 128:
 // 33.9 us with 2, 38.8 with 4), unless their rows are even (0.75 M nonzeros in rows of 125, width 200: 45.4 us with 2, 38.9
 // with 4).  The smallest take one vector per lane for the same reason (0.1 M nonzeros, width 64:
-// 11.8 us with 1, 13.7 with 2).  COO operands, whose row indices take registers and a second stage, stay with two (4 M
+// 11.8 us with 1, 13.7 with 2; 0.03 M, width 400: 12.5 and 14.2; but 0.09 M, width 1,093: 51.7 and, with 3, 39.4).  COO operands, whose row indices take registers and a second stage, stay with two (4 M
 // nonzeros, width 128: 158 us with 2, 230 with 4).
 //
 // Chunk length: the launch is a whole number of full waves, a wave being what the SMs hold.  All chunks take about as long,
@@ -363,7 +363,7 @@ static SplitShape split_shape(int64_t nnz, int m, int f, bool coo, bool even) {
   const int longest = v <= 8 ? 1024 : 704, shortest = 32;
   s.lpn = v <= 4 ? 4 : 8;
   s.nv = 1;
-  if (v > 8 && nnz >= (v <= 16 ? 500000 : 150000)) {
+  if (v > 8 && (v <= 16 ? nnz >= 500000 : nnz * v >= 5000000)) {
     const bool wide = even || nnz >= 2000000;
     const int few = coo || v <= 16 || !wide ? 2 : 3, many = coo ? 2 : wide ? 4 : 3;
     constexpr int weight[5] = {0, 0, 108, 100, 106};

@@ -296,6 +296,16 @@ typedef struct {
 } cagnet_tn_sum;
 int cagnet_gemm_tn_partials_f32(const float* H, int64_t ldh, const float* G, int64_t ldg, int64_t n, int32_t K, int32_t N,
                                 void* ws, size_t ws_bytes, cagnet_tn_sum* sum, void* stream);
+/* Two such products over the same rows, p[0] and p[1] into sum[0] and sum[1]: in one launch where both are narrow.  *launches (host):
+ * kernels launched. */
+typedef struct {
+  const float *H, *G;
+  int64_t ldh, ldg;
+  int32_t K, N;
+  void* ws;
+  size_t ws_bytes;
+} cagnet_tn_product;
+int cagnet_gemm_tn_partials2_f32(const cagnet_tn_product* p, cagnet_tn_sum* sum, int64_t n, int32_t* launches, void* stream);
 
 /* ---- Elementwise / row-wise pieces, for callers that do not use the fused epilogues. */
 int cagnet_relu_fwd_f32(const float* z, int64_t ldz, float* h, int64_t ldh, int64_t n, int32_t N, void* stream);
