@@ -66,6 +66,7 @@ PROTOTYPES = {
                                      _sz, _vp]),
     "cagnet_nll_softmax_bwd_f32": (_i32, [_vp, _i64, _vp, _vp, _i64, _i32, _i32, _i32, _f32, _vp, _i64,
                                           ctypes.POINTER(_i32), _vp, _sz, _vp]),
+    "cagnet_gemm_tn_partials2_f32": (_i32, [_vp, _vp, _i64, ctypes.POINTER(_i32), _vp]),
     "cagnet_gemm_tn_partials_f32": (_i32, [_vp, _i64, _vp, _i64, _i64, _i32, _i32, _vp, _sz, _vp, _vp]),
     "cagnet_log_softmax_nll_f32": (_i32, [_vp, _i64, _i64, _i32, _vp, _vp, _i32, _i32, _f32, _vp, _i64, _vp, _i64,
                                           ctypes.POINTER(_i32), _vp, _sz, _vp]),

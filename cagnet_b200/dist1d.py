@@ -493,11 +493,11 @@ class Model:
             plan = self.am_pbyp
             back = getattr(plan, "backward_plan", None) or plan
             self._local = len(plan.groups) == 1 and len(back.groups) == 1 and local_epoch.plan(
-                self.rt.backend, plan.groups[0].block, back.groups[0].block, 0, self.classes, self.rt.activations,
-                self.rt.order == "min_width") or False
+                self.rt.backend, plan.groups[0].block, back.groups[0].block, 0, self.classes) or False
         if not self._local:
             return None
-        return local_epoch.train(self._local, self, self.inputs_loc, self.datay_rank, self.rank_train_mask, self.train_count)
+        return local_epoch.train(self._local, self, self.inputs_loc, self.datay_rank, self.rank_train_mask, self.train_count,
+                                 self.rt.order == "min_width")
 
     def capture(self):
         """Record one whole epoch (both layers, loss, backward, collectives, Adam) into a CUDA graph; `train()`

@@ -423,7 +423,7 @@ def train_local(model):
         return None
     if model._local is None:
         back = model.adj_t.adj_block if model.adj_t is not None else model.adj_block
-        model._local = local_epoch.plan(be, model.adj_block, back, model.cls_lo, model.cls_hi, rt.activations, False) or False
+        model._local = local_epoch.plan(be, model.adj_block, back, model.cls_lo, model.cls_hi) or False
     if not model._local or model.local_train_rows <= 0:
         return None
     outputs = local_epoch.train(model._local, model, model.inputs_loc, model.y_eff, model.mask_eff, model.train_count_global)

@@ -13,9 +13,9 @@ from .backend import CudaBackend
 
 
 class _Plan:
-    def __init__(self, fwd, bwd, cls_lo, cls_hi, activations, min_width, backend):
+    def __init__(self, fwd, bwd, cls_lo, cls_hi, backend):
         self.fwd, self.bwd, self.backend = fwd, bwd, backend
-        self.cls_lo, self.cls_hi, self.activations, self.min_width = cls_lo, cls_hi, activations, min_width
+        self.cls_lo, self.cls_hi = cls_lo, cls_hi
 
 
 def _weight_ok(w, device):
@@ -51,19 +51,19 @@ def _adam_state(optimizer, w1, w2):
     return states, g
 
 
-def plan(backend, fwd, bwd, cls_lo, cls_hi, activations, min_width):
+def plan(backend, fwd, bwd, cls_lo, cls_hi):
     """The constant part of a model's epochs, or None where the general path has to run."""
     if type(backend) is not CudaBackend:
         return None
     for b in (fwd, bwd):
         if not isinstance(b, ops.CsrBlock) or b.n != b.m or (b.tiles is None and b._rect[0] is not None):
             return None
-    return _Plan(fwd, bwd, int(cls_lo), int(cls_hi), bool(activations), bool(min_width), backend)
+    return _Plan(fwd, bwd, int(cls_lo), int(cls_hi), backend)
 
 
-def train(p, model, x, y, mask, count):
+def train(p, model, x, y, mask, count, min_width=False):
     """Run one epoch of `model` (weights, optimizer, last_loss) on features x, labels y and train mask by plan p, the loss a
-    mean over `count` rows; the outputs, or None to decline."""
+    mean over `count` rows, sparse products at the narrower width of a layer if `min_width`; the outputs, or None to decline."""
     w1, w2 = model.weight1, model.weight2
     if count <= 0 or not (_weight_ok(w1, x.device) and _weight_ok(w2, x.device)):
         return None
@@ -77,7 +77,7 @@ def train(p, model, x, y, mask, count):
     if p.backend.spmm_events is not None:
         hook = _event_hook(p)
     out, loss, g1, g2, launches = host.epoch(p.fwd.address(), p.bwd.address(), x, w1.detach(), w2.detach(), y.contiguous(),
-                                             mask.contiguous(), count, p.cls_lo, p.cls_hi, p.activations, p.min_width, adam, hook)
+                                             mask.contiguous(), count, p.cls_lo, p.cls_hi, bool(model.rt.activations), min_width, adam, hook)
     ops.LAUNCHES[0] += launches
     w1.grad, w2.grad = g1, g2
     if state is not None:
